@@ -4,35 +4,41 @@
 // precision pattern: the error of a float solve (with or without FP64-residual refinement)
 // is measured against it, on lattices where a CPU FP64 solve would take hours.
 //
-// The convolution runs as five passes of zero-padded 2n-point transforms over a work buffer
-// [3][ni][2nj][2nl] (only the i < ni planes of the padded grid exist, as in the float
-// passes), with the Green tensor's FP64 octant [6][ni+1][nj+1][nl+1] (green.cu) unfolded by
-// its parities:
-//   Z  forward along l of every lattice row (c, i, j < nj), rows zero-padded to 2nl
-//   Y  forward along j of tiles of spectral columns (c, i, kz), zero-padded to 2nj
+// The convolution runs as five passes over a work buffer [3][ni][2nj][2nl] (only the i < ni
+// planes of the padded grid exist, as in the float passes), with the Green tensor's FP64
+// octant [6][ni+1][nj+1][nl+1] (green.cu) unfolded by its parities:
+//   Z  forward along l of every lattice row (c, i, j < nj)
+//   Y  forward along j of tiles of spectral columns (c, i, kz)
 //   X  forward along i, the symmetric 3x3 product, inverse along i (i < ni kept), per
 //      tile of (ky, kz) columns with all 3 components
 //   YI inverse along j (j < nj kept)
 //   ZI inverse along l (l < nl kept) with the solver epilogue out = sv v - alpha_m conv
-// Each line lives in shared memory and is transformed by an iterative radix-2 FFT with an
-// FP64 twiddle table built on the host.  Throughput is not the aim of this path; exactness
-// is: a 128^3 FP64 matvec takes a few milliseconds.
+// Every transform is an n-point FFT: the even and odd bins of a zero-padded 2n-point line
+// are DFT_n(x) and DFT_n(x W_2n^j), and of the inverse only the first n outputs are kept,
+// IDFT_n(even) + W_2n^-j IDFT_n(odd).  An n-point line is two register DFTs (n = R1 R2)
+// with one exchange through shared memory, its sizes compile-time constants.
+//
+// What bounds it: the passes move 1248 n^3 bytes at least (48 + 96, 96 + 192, 192 + 192,
+// 192 + 96, 96 + 48), from L2 while the work buffer fits there, and do about 450 n^3
+// double multiply-adds; the first form (iterative radix-2 stages over padded 2n-point lines
+// in shared memory) moved every line through shared memory 2 log2(2n) times.
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
+#include "common.cuh"
 #include "fp64.h"
 
 namespace ddagpu {
 
 namespace {
 
-constexpr int kT = 256;      // threads per block of every pass
-constexpr int kTZ = 8;       // spectral columns per block of the Y, X and YI passes
-constexpr int kLJ = 8;       // lattice rows per block of the Z and ZI passes
+constexpr int kT = 256;      // threads per block of the field passes
+constexpr int kF = 128;      // threads per block of the transform passes
 
 __device__ __forceinline__ double2 dadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 dsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
@@ -43,48 +49,74 @@ __device__ __forceinline__ double2 dmul(double2 a, double2 b)
 __device__ __forceinline__ double2 dconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double2 dzero() { return make_double2(0.0, 0.0); }
 
-// In-place radix-2 FFT of `nlines` lines of M points (M a power of two, 2..256) in shared
-// memory, element k of line t at buf[t * LS + k]: bit reversal, then log2 M butterfly
-// stages.  tw[k] = exp(-2 pi i k / M) for k < M / 2; inv conjugates them (the reference's
-// inverse is conj(DFT(conj x)) with no 1/M, fft_func.cpp:556-653).  Every thread of the
-// block calls it; it synchronises before and after.
-__device__ void fft_lines_d(double2 *buf, int M, int LS, int nlines, const double2 *__restrict__ tw,
-                            bool inv)
+// exp(-2 pi i m / 16), m = 0..7
+__device__ __forceinline__ double2 w16d(int m)
 {
-    __syncthreads();
-    const int logM = __ffs(M) - 1;
-    for (int e = threadIdx.x; e < nlines * M; e += blockDim.x) {
-        const int t = e / M, k = e - t * M;
-        const int r = (int)(__brev((unsigned)k) >> (32 - logM));
-        if (r > k) {
-            double2 *b = buf + (size_t)t * LS;
-            const double2 x = b[k];
-            b[k] = b[r];
-            b[r] = x;
-        }
-    }
-    __syncthreads();
-    const int half = M >> 1;
-    for (int hs = 1; hs < M; hs <<= 1) {
-        const int step = half / hs;
-        for (int e = threadIdx.x; e < nlines * half; e += blockDim.x) {
-            const int t = e / half, b = e - t * half;
-            const int j = b % hs, i0 = (b / hs) * 2 * hs + j, i1 = i0 + hs;
-            double2 w = tw[j * step];
-            if (inv) w.y = -w.y;
-            double2 *L = buf + (size_t)t * LS;
-            const double2 u = L[i0], v = dmul(L[i1], w);
-            L[i0] = dadd(u, v);
-            L[i1] = dsub(u, v);
-        }
-        __syncthreads();
+    const double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173, h = 0.70710678118654752440;
+    switch (m) {
+    case 0: return make_double2(1.0, 0.0);
+    case 1: return make_double2(c1, -s1);
+    case 2: return make_double2(h, -h);
+    case 3: return make_double2(s1, -c1);
+    case 4: return make_double2(0.0, -1.0);
+    case 5: return make_double2(-s1, -c1);
+    case 6: return make_double2(-h, -h);
+    default: return make_double2(-c1, -s1);
     }
 }
+
+// In-register DFT of R points (a power of two, <= 16), natural order in and out; INV
+// conjugates the twiddles (the reference's inverse is conj(DFT(conj x)) with no 1/n,
+// fft_func.cpp:556-653).
+template <int R, bool INV>
+__device__ __forceinline__ void dft_d(double2 (&v)[R])
+{
+    if (R == 1) return;
+#pragma unroll
+    for (int len = R; len >= 2; len >>= 1) {
+#pragma unroll
+        for (int s = 0; s < R; s += len) {
+#pragma unroll
+            for (int j = 0; j < len / 2; j++) {
+                const double2 a = v[s + j], b = v[s + j + len / 2], d = dsub(a, b);
+                v[s + j] = dadd(a, b);
+                if (j == 0) {
+                    v[s + j + len / 2] = d;
+                } else if (4 * j == len) {
+                    v[s + j + len / 2] = INV ? make_double2(-d.y, d.x) : make_double2(d.y, -d.x);
+                } else {
+                    double2 w = w16d(j * (16 / len));
+                    if (INV) w.y = -w.y;
+                    v[s + j + len / 2] = dmul(d, w);
+                }
+            }
+        }
+    }
+    double2 t[R];
+#pragma unroll
+    for (int k = 0; k < R; k++) t[k] = v[bitrev_c(k, ilog2c<R>::v)];
+#pragma unroll
+    for (int k = 0; k < R; k++) v[k] = t[k];
+}
+
+// A line of N = R1 R2 points: step A is R2 register DFTs of R1 points (elements t2 + R2 r,
+// then times W_N^(t2 k1)), step B is R1 DFTs of R2 points (over t2, outputs k1 + R1 k2).
+// Between them element (k1, t2) sits at k1 (R2 + 1) + t2: the pad keeps the eight lanes of
+// a 128-byte shared-memory phase on distinct banks when they differ in k1 (row passes).
+template <int N>
+struct Line {
+    static constexpr int R1 = fft_split<N>::R1, R2 = fft_split<N>::R2, LEN = R1 * (R2 + 1);
+    // rows per block of the Z passes, columns per block of the Y and X passes: the 2 R1 step-B
+    // items of a line (both parity halves) over kF threads; a Y column tile is a 128-byte run
+    static constexpr int ROWS = kF / (2 * R1), YC = 8, XC = kF / (2 * R1);
+    static constexpr size_t XSMEM = (size_t)3 * 2 * N * XC * sizeof(double2);
+    __device__ static int at(int k1, int t2) { return k1 * (R2 + 1) + t2; }
+};
 
 struct Mv64 {
     int ni, nj, nl;
     size_t N;
-    const double2 *twi, *twj, *twl;   // exp(-2 pi i k / 2n), k < n, per axis
+    const double2 *twi, *twj, *twl;   // exp(-2 pi i k / 2n), k < 2n, per axis
     const double2 *g;                 // [6][ni+1][nj+1][nl+1]
     double2 *work;                    // [3][ni][2nj][2nl]
     int conj;
@@ -105,113 +137,328 @@ __device__ __forceinline__ size_t wrow(const Mv64 &a, int c, int i, int js)
     return (((size_t)c * a.ni + i) * (2 * a.nj) + js) * (2 * a.nl);
 }
 
-// Z: rows (c, i, j0 .. j0 + kLJ) of the field, zero-padded, forward along l
-__global__ void __launch_bounds__(kT) z_fwd(Mv64 a, const double2 *__restrict__ src)
+// Step A of one half h of a line whose R1 inputs of lane t2 are in v (overwritten).
+template <int N, bool INV>
+__device__ __forceinline__ void step_a(double2 (&v)[Line<N>::R1], int t2, const double2 *__restrict__ tw)
 {
-    extern __shared__ double2 smd[];
-    const int M = 2 * a.nl, LS = M + 1, j0 = blockIdx.x * kLJ, i = blockIdx.y, c = blockIdx.z;
-    const int nr = a.nj - j0 < kLJ ? a.nj - j0 : kLJ;
-    const double2 *s = src + (size_t)c * a.N + ((size_t)i * a.nj + j0) * a.nl;
-    for (int e = threadIdx.x; e < nr * M; e += blockDim.x) {
-        const int t = e / M, l = e - t * M;
-        smd[t * LS + l] = l < a.nl ? s[(size_t)t * a.nl + l] : dzero();
-    }
-    fft_lines_d(smd, M, LS, nr, a.twl, false);
-    for (int e = threadIdx.x; e < nr * M; e += blockDim.x) {
-        const int t = e / M, k = e - t * M;
-        a.work[wrow(a, c, i, j0 + t) + k] = smd[t * LS + k];
-    }
-}
-
-// Y / YI: spectral columns kz0 .. kz0 + tz of plane (c, i), along j
-__global__ void __launch_bounds__(kT) y_pass(Mv64 a, int inv, int tz)
-{
-    extern __shared__ double2 smd[];
-    const int M = 2 * a.nj, LS = M + 1, kz0 = blockIdx.x * tz, i = blockIdx.y, c = blockIdx.z;
-    const int nload = inv ? M : a.nj, nstore = inv ? a.nj : M;
-    for (int e = threadIdx.x; e < M * tz; e += blockDim.x) {
-        const int j = e / tz, t = e - j * tz;
-        smd[t * LS + j] = j < nload ? a.work[wrow(a, c, i, j) + kz0 + t] : dzero();
-    }
-    fft_lines_d(smd, M, LS, tz, a.twj, inv != 0);
-    for (int e = threadIdx.x; e < nstore * tz; e += blockDim.x) {
-        const int j = e / tz, t = e - j * tz;
-        a.work[wrow(a, c, i, j) + kz0 + t] = smd[t * LS + j];
-    }
-}
-
-// X: columns (ky, kz0 .. kz0 + tz), 3 components: forward along i, G product, inverse
-__global__ void __launch_bounds__(kT) x_pass(Mv64 a, int tz)
-{
-    extern __shared__ double2 smd[];
-    const int M = 2 * a.ni, LS = M + 1, kz0 = blockIdx.x * tz, ky = blockIdx.y;
-    // line (c, t) at (c * tz + t) * LS
-    for (int e = threadIdx.x; e < 3 * M * tz; e += blockDim.x) {
-        const int t = e % tz, i = (e / tz) % M, c = e / (tz * M);
-        smd[(c * tz + t) * LS + i] = i < a.ni ? a.work[wrow(a, c, i, ky) + kz0 + t] : dzero();
-    }
-    fft_lines_d(smd, M, LS, 3 * tz, a.twi, false);
-    const int nj = a.nj, nl = a.nl, ni = a.ni;
-    const bool my = ky > nj;
-    const int oy = my ? 2 * nj - ky : ky;
-    const size_t per = (size_t)(ni + 1) * (nj + 1) * (nl + 1);
-    for (int e = threadIdx.x; e < M * tz; e += blockDim.x) {
-        const int t = e % tz, kx = e / tz, kz = kz0 + t;
-        const bool mx = kx > ni, mz = kz > nl;
-        const int ox = mx ? 2 * ni - kx : kx, oz = mz ? 2 * nl - kz : kz;
-        const size_t q = ((size_t)ox * (nj + 1) + oy) * (nl + 1) + oz;
-        double2 g[6];
+    dft_d<Line<N>::R1, INV>(v);
 #pragma unroll
-        for (int k = 0; k < 6; k++) g[k] = a.g[k * per + q];
-        if (mx ^ my) g[1] = make_double2(-g[1].x, -g[1].y);
-        if (mx ^ mz) g[2] = make_double2(-g[2].x, -g[2].y);
-        if (my ^ mz) g[4] = make_double2(-g[4].x, -g[4].y);
-        if (a.conj)
-#pragma unroll
-            for (int k = 0; k < 6; k++) g[k] = dconj(g[k]);
-        double2 *bx = smd + (size_t)(0 * tz + t) * LS + kx, *by = smd + (size_t)(1 * tz + t) * LS + kx,
-                *bz = smd + (size_t)(2 * tz + t) * LS + kx;
-        const double2 vx = *bx, vy = *by, vz = *bz;
-        *bx = dadd(dadd(dmul(g[0], vx), dmul(g[1], vy)), dmul(g[2], vz));
-        *by = dadd(dadd(dmul(g[1], vx), dmul(g[3], vy)), dmul(g[4], vz));
-        *bz = dadd(dadd(dmul(g[2], vx), dmul(g[4], vy)), dmul(g[5], vz));
-    }
-    fft_lines_d(smd, M, LS, 3 * tz, a.twi, true);
-    for (int e = threadIdx.x; e < 3 * a.ni * tz; e += blockDim.x) {
-        const int t = e % tz, i = (e / tz) % a.ni, c = e / (tz * a.ni);
-        a.work[wrow(a, c, i, ky) + kz0 + t] = smd[(c * tz + t) * LS + i];
+    for (int k1 = 1; k1 < Line<N>::R1; k1++) {
+        double2 w = __ldg(&tw[2 * t2 * k1]);
+        if (INV) w.y = -w.y;
+        v[k1] = dmul(v[k1], w);
     }
 }
 
-// ZI: rows (c, i, j0 .. j0 + kLJ), inverse along l, l < nl kept, epilogue
-__global__ void __launch_bounds__(kT) z_inv(Mv64 a, Ep64 ep, double2 *__restrict__ out)
+// Z: rows (c, i, j0 ..) of the field, forward along l.  Items of a block are spread over its
+// threads with the parity half fastest, so a warp's loads and stores are runs of the row.
+template <int N>
+__global__ void __launch_bounds__(kF) z_fwd(Mv64 a, const double2 *__restrict__ src)
 {
-    extern __shared__ double2 smd[];
-    const int M = 2 * a.nl, LS = M + 1, j0 = blockIdx.x * kLJ, i = blockIdx.y, c = blockIdx.z;
-    const int nr = a.nj - j0 < kLJ ? a.nj - j0 : kLJ;
-    for (int e = threadIdx.x; e < nr * M; e += blockDim.x) {
-        const int t = e / M, k = e - t * M;
-        smd[t * LS + k] = a.work[wrow(a, c, i, j0 + t) + k];
-    }
-    fft_lines_d(smd, M, LS, nr, a.twl, true);
-    for (int e = threadIdx.x; e < nr * a.nl; e += blockDim.x) {
-        const int t = e / a.nl, l = e - t * a.nl;
-        const size_t q = ((size_t)i * a.nj + j0 + t) * a.nl + l, o = (size_t)c * a.N + q;
-        const double2 conv = smd[t * LS + l];
-        double2 res = conv;
-        if (ep.mode == 1) {
-            const int m = ep.occ[q];
-            if (!ep.mv[m]) {
-                res = dzero();
-            } else {
-                double2 al = ep.alpha[m];
-                if (ep.conj) al = dconj(al);
-                const double2 sv = ep.sv != 0.0 ? make_double2(ep.v[o].x * ep.sv, ep.v[o].y * ep.sv) : dzero();
-                res = dsub(sv, dmul(al, conv));
-            }
+    using S = Line<N>;
+    constexpr int R1 = S::R1, R2 = S::R2, G = S::ROWS;
+    __shared__ double2 sm[G * 2 * S::LEN];
+    const int j0 = blockIdx.x * G, i = blockIdx.y, c = blockIdx.z;
+    const int nr = a.nj - j0 < G ? a.nj - j0 : G;
+    const double2 *s = src + (size_t)c * a.N + ((size_t)i * a.nj + j0) * N;
+    for (int e = threadIdx.x; e < nr * 2 * R2; e += kF) {
+        const int t2 = e % R2, h = (e / R2) % 2, t = e / (2 * R2);
+        double2 v[R1];
+#pragma unroll
+        for (int r = 0; r < R1; r++) {
+            v[r] = s[t * N + t2 + R2 * r];
+            if (h) v[r] = dmul(v[r], __ldg(&a.twl[t2 + R2 * r]));
         }
-        out[o] = res;
+        step_a<N, false>(v, t2, a.twl);
+#pragma unroll
+        for (int k1 = 0; k1 < R1; k1++) sm[(t * 2 + h) * S::LEN + S::at(k1, t2)] = v[k1];
     }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nr * 2 * R1; e += kF) {
+        const int h = e % 2, k1 = (e / 2) % R1, t = e / (2 * R1);
+        double2 u[R2];
+#pragma unroll
+        for (int q = 0; q < R2; q++) u[q] = sm[(t * 2 + h) * S::LEN + S::at(k1, q)];
+        dft_d<R2, false>(u);
+        double2 *d = a.work + wrow(a, c, i, j0 + t);
+#pragma unroll
+        for (int k2 = 0; k2 < R2; k2++) d[2 * (k1 + R1 * k2) + h] = u[k2];
+    }
+}
+
+// Y: spectral columns kz0 .. of plane (c, i), forward along j
+template <int N>
+__global__ void __launch_bounds__(kF) y_fwd(Mv64 a)
+{
+    using S = Line<N>;
+    constexpr int R1 = S::R1, R2 = S::R2, TC = S::YC;
+    __shared__ double2 sm[2][R1][R2][TC];
+    const int t = threadIdx.x % TC, kz = blockIdx.x * TC + t, i = blockIdx.y, c = blockIdx.z;
+    const bool ok = kz < 2 * a.nl;
+    double2 *col = a.work + wrow(a, c, i, 0) + kz;
+    const size_t rs = (size_t)2 * a.nl;
+    // the inputs are read before any output row is written (the pass is in place)
+    for (int e = threadIdx.x / TC; e < 2 * R2; e += kF / TC) {
+        if (!ok) break;
+        const int h = e % 2, t2 = e / 2;
+        double2 v[R1];
+#pragma unroll
+        for (int r = 0; r < R1; r++) {
+            v[r] = col[(t2 + R2 * r) * rs];
+            if (h) v[r] = dmul(v[r], __ldg(&a.twj[t2 + R2 * r]));
+        }
+        step_a<N, false>(v, t2, a.twj);
+#pragma unroll
+        for (int k1 = 0; k1 < R1; k1++) sm[h][k1][t2][t] = v[k1];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x / TC; e < 2 * R1; e += kF / TC) {
+        if (!ok) break;
+        const int h = e % 2, k1 = e / 2;
+        double2 u[R2];
+#pragma unroll
+        for (int q = 0; q < R2; q++) u[q] = sm[h][k1][q][t];
+        dft_d<R2, false>(u);
+#pragma unroll
+        for (int k2 = 0; k2 < R2; k2++) col[(2 * (k1 + R1 * k2) + h) * rs] = u[k2];
+    }
+}
+
+// YI: the same columns, inverse along j, j < N kept
+template <int N>
+__global__ void __launch_bounds__(kF) y_inv(Mv64 a)
+{
+    using S = Line<N>;
+    constexpr int R1 = S::R1, R2 = S::R2, TC = S::YC;
+    __shared__ double2 sm[2][R1][R2][TC];
+    const int t = threadIdx.x % TC, kz = blockIdx.x * TC + t, i = blockIdx.y, c = blockIdx.z;
+    const bool ok = kz < 2 * a.nl;
+    double2 *col = a.work + wrow(a, c, i, 0) + kz;
+    const size_t rs = (size_t)2 * a.nl;
+    for (int e = threadIdx.x / TC; e < 2 * R2; e += kF / TC) {
+        if (!ok) break;
+        const int h = e % 2, t2 = e / 2;
+        double2 v[R1];
+#pragma unroll
+        for (int r = 0; r < R1; r++) v[r] = col[(2 * (t2 + R2 * r) + h) * rs];
+        step_a<N, true>(v, t2, a.twj);
+#pragma unroll
+        for (int k1 = 0; k1 < R1; k1++) sm[h][k1][t2][t] = v[k1];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x / TC; e < R1; e += kF / TC) {
+        if (!ok) break;
+        double2 u[R2], o[R2];
+#pragma unroll
+        for (int q = 0; q < R2; q++) {
+            u[q] = sm[0][e][q][t];
+            o[q] = sm[1][e][q][t];
+        }
+        dft_d<R2, true>(u);
+        dft_d<R2, true>(o);
+#pragma unroll
+        for (int k2 = 0; k2 < R2; k2++) {
+            const int j = e + R1 * k2;
+            col[j * rs] = dadd(u[k2], dmul(o[k2], dconj(__ldg(&a.twj[j]))));
+        }
+    }
+}
+
+// X: columns (ky, kz0 ..), 3 components: forward along i, G product, inverse.  A thread of
+// step B holds 3 x R2 frequencies, so the product and the first inverse step need no exchange.
+template <int N>
+__global__ void __launch_bounds__(kF) x_pass(Mv64 a)
+{
+    using S = Line<N>;
+    constexpr int R1 = S::R1, R2 = S::R2, TC = S::XC;
+    extern __shared__ double2 smd[];   // [3][2][R1][R2][TC]
+    auto B = [&](int c, int h, int k1, int t2, int t) -> double2 & {
+        return smd[((((c * 2 + h) * R1) + k1) * R2 + t2) * TC + t];
+    };
+    const int t = threadIdx.x % TC, g0 = threadIdx.x / TC, kz = blockIdx.x * TC + t, ky = blockIdx.y;
+    const bool ok = kz < 2 * a.nl;
+    double2 *col = a.work + wrow(a, 0, 0, ky) + kz;
+    const size_t rs = (size_t)(2 * a.nj) * (2 * a.nl), cs = rs * N;
+    for (int e = g0; e < 6 * R2; e += kF / TC) {
+        if (!ok) break;
+        const int h = e % 2, t2 = (e / 2) % R2, c = e / (2 * R2);
+        double2 v[R1];
+#pragma unroll
+        for (int r = 0; r < R1; r++) {
+            v[r] = col[c * cs + (t2 + R2 * r) * rs];
+            if (h) v[r] = dmul(v[r], __ldg(&a.twi[t2 + R2 * r]));
+        }
+        step_a<N, false>(v, t2, a.twi);
+#pragma unroll
+        for (int k1 = 0; k1 < R1; k1++) B(c, h, k1, t2, t) = v[k1];
+    }
+    __syncthreads();
+    if (ok) {
+        const int h = g0 % 2, k1 = g0 / 2, nj = a.nj, nl = a.nl;
+        const bool my = ky > nj, mz = kz > nl;
+        const int oy = my ? 2 * nj - ky : ky, oz = mz ? 2 * nl - kz : kz;
+        const size_t yz = (size_t)oy * (nl + 1) + oz, xs = (size_t)(nj + 1) * (nl + 1), per = (N + 1) * xs;
+        double2 X[3][R2];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+#pragma unroll
+            for (int q = 0; q < R2; q++) X[c][q] = B(c, h, k1, q, t);
+            dft_d<R2, false>(X[c]);
+        }
+#pragma unroll
+        for (int q = 0; q < R2; q++) {
+            const int kx = 2 * (k1 + R1 * q) + h;
+            const bool mx = kx > N;
+            const double2 *G = a.g + (size_t)(mx ? 2 * N - kx : kx) * xs + yz;
+            double2 g[6];
+#pragma unroll
+            for (int k = 0; k < 6; k++) g[k] = __ldg(&G[k * per]);
+            if (mx ^ my) g[1] = make_double2(-g[1].x, -g[1].y);
+            if (mx ^ mz) g[2] = make_double2(-g[2].x, -g[2].y);
+            if (my ^ mz) g[4] = make_double2(-g[4].x, -g[4].y);
+            if (a.conj)
+#pragma unroll
+                for (int k = 0; k < 6; k++) g[k] = dconj(g[k]);
+            const double2 vx = X[0][q], vy = X[1][q], vz = X[2][q];
+            X[0][q] = dadd(dadd(dmul(g[0], vx), dmul(g[1], vy)), dmul(g[2], vz));
+            X[1][q] = dadd(dadd(dmul(g[1], vx), dmul(g[3], vy)), dmul(g[4], vz));
+            X[2][q] = dadd(dadd(dmul(g[2], vx), dmul(g[4], vy)), dmul(g[5], vz));
+        }
+        // inverse, transposed split: R2 points over q, times W^-(k1 u); kept at (k1, u)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            dft_d<R2, true>(X[c]);
+#pragma unroll
+            for (int u = 0; u < R2; u++)
+                B(c, h, k1, u, t) = u ? dmul(X[c][u], dconj(__ldg(&a.twi[2 * k1 * u]))) : X[c][u];
+        }
+    }
+    __syncthreads();
+    // R1 points over k1 of both halves: outputs u + R2 k2
+    for (int e = g0; e < 3 * R2; e += kF / TC) {
+        if (!ok) break;
+        const int u = e % R2, c = e / R2;
+        double2 v[R1], w[R1];
+#pragma unroll
+        for (int k1 = 0; k1 < R1; k1++) {
+            v[k1] = B(c, 0, k1, u, t);
+            w[k1] = B(c, 1, k1, u, t);
+        }
+        dft_d<R1, true>(v);
+        dft_d<R1, true>(w);
+#pragma unroll
+        for (int k2 = 0; k2 < R1; k2++) {
+            const int i = u + R2 * k2;
+            col[c * cs + i * rs] = dadd(v[k2], dmul(w[k2], dconj(__ldg(&a.twi[i]))));
+        }
+    }
+}
+
+// ZI: rows (c, i, j0 ..), inverse along l, l < N kept, epilogue
+template <int N>
+__global__ void __launch_bounds__(kF) z_inv(Mv64 a, Ep64 ep, double2 *__restrict__ out)
+{
+    using S = Line<N>;
+    constexpr int R1 = S::R1, R2 = S::R2, G = S::ROWS;
+    __shared__ double2 sm[G * 2 * S::LEN];
+    const int j0 = blockIdx.x * G, i = blockIdx.y, c = blockIdx.z;
+    const int nr = a.nj - j0 < G ? a.nj - j0 : G;
+    for (int e = threadIdx.x; e < nr * 2 * R2; e += kF) {
+        const int h = e % 2, t2 = (e / 2) % R2, t = e / (2 * R2);
+        const double2 *s = a.work + wrow(a, c, i, j0 + t);
+        double2 v[R1];
+#pragma unroll
+        for (int r = 0; r < R1; r++) v[r] = s[2 * (t2 + R2 * r) + h];
+        step_a<N, true>(v, t2, a.twl);
+#pragma unroll
+        for (int k1 = 0; k1 < R1; k1++) sm[(t * 2 + h) * S::LEN + S::at(k1, t2)] = v[k1];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nr * R1; e += kF) {
+        const int k1 = e % R1, t = e / R1;
+        double2 u[R2], o[R2];
+#pragma unroll
+        for (int q = 0; q < R2; q++) {
+            u[q] = sm[(t * 2) * S::LEN + S::at(k1, q)];
+            o[q] = sm[(t * 2 + 1) * S::LEN + S::at(k1, q)];
+        }
+        dft_d<R2, true>(u);
+        dft_d<R2, true>(o);
+#pragma unroll
+        for (int k2 = 0; k2 < R2; k2++) {
+            const int l = k1 + R1 * k2;
+            const size_t q = ((size_t)i * a.nj + j0 + t) * N + l, oq = (size_t)c * a.N + q;
+            const double2 conv = dadd(u[k2], dmul(o[k2], dconj(__ldg(&a.twl[l]))));
+            double2 res = conv;
+            if (ep.mode == 1) {
+                const int m = ep.occ[q];
+                if (!ep.mv[m]) {
+                    res = dzero();
+                } else {
+                    double2 al = ep.alpha[m];
+                    if (ep.conj) al = dconj(al);
+                    const double2 sv = ep.sv != 0.0 ? make_double2(ep.v[oq].x * ep.sv, ep.v[oq].y * ep.sv) : dzero();
+                    res = dsub(sv, dmul(al, conv));
+                }
+            }
+            out[oq] = res;
+        }
+    }
+}
+
+inline unsigned nb(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
+
+// f(std::integral_constant<int, n>) for a lattice edge n (a power of two, 2..128)
+template <class F>
+cudaError_t with_edge(int n, F &&f)
+{
+    switch (n) {
+    case 2: return f(std::integral_constant<int, 2>{});
+    case 4: return f(std::integral_constant<int, 4>{});
+    case 8: return f(std::integral_constant<int, 8>{});
+    case 16: return f(std::integral_constant<int, 16>{});
+    case 32: return f(std::integral_constant<int, 32>{});
+    case 64: return f(std::integral_constant<int, 64>{});
+    case 128: return f(std::integral_constant<int, 128>{});
+    }
+    return cudaErrorInvalidValue;
+}
+
+// out = epilogue of G * src: the five passes
+cudaError_t matvec64(const Mv64 &a, const Ep64 &ep, const double2 *src, double2 *out, cudaStream_t st)
+{
+    const int ni = a.ni, nj = a.nj, nl = a.nl;
+    cudaError_t e = with_edge(nl, [&](auto n) {
+        constexpr int N = decltype(n)::value;
+        z_fwd<N><<<dim3(nb(nj, Line<N>::ROWS), ni, 3), kF, 0, st>>>(a, src);
+        return cudaGetLastError();
+    });
+    if (e == cudaSuccess)
+        e = with_edge(nj, [&](auto n) {
+            constexpr int N = decltype(n)::value;
+            y_fwd<N><<<dim3(nb(2 * nl, Line<N>::YC), ni, 3), kF, 0, st>>>(a);
+            return cudaGetLastError();
+        });
+    if (e == cudaSuccess)
+        e = with_edge(ni, [&](auto n) {
+            constexpr int N = decltype(n)::value;
+            if (cudaError_t r = raise_smem_limit((const void *)x_pass<N>, (int)Line<N>::XSMEM)) return r;
+            x_pass<N><<<dim3(nb(2 * nl, Line<N>::XC), 2 * nj), kF, Line<N>::XSMEM, st>>>(a);
+            return cudaGetLastError();
+        });
+    if (e == cudaSuccess)
+        e = with_edge(nj, [&](auto n) {
+            constexpr int N = decltype(n)::value;
+            y_inv<N><<<dim3(nb(2 * nl, Line<N>::YC), ni, 3), kF, 0, st>>>(a);
+            return cudaGetLastError();
+        });
+    if (e == cudaSuccess)
+        e = with_edge(nl, [&](auto n) {
+            constexpr int N = decltype(n)::value;
+            z_inv<N><<<dim3(nb(nj, Line<N>::ROWS), ni, 3), kF, 0, st>>>(a, ep, out);
+            return cudaGetLastError();
+        });
+    return e;
 }
 
 // ---------------------------------------------------------------- field operations
@@ -545,8 +792,6 @@ __global__ void cg_dir(F64 f, double2 b, const double2 *r, double2 *s, float2 *s
     }
 }
 
-inline unsigned nb(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
-
 }  // namespace
 
 // ------------------------------------------------------------------ host side
@@ -575,7 +820,7 @@ cudaError_t Fp64Buffers::ensure(int ni_, int nj_, int nl_, double kd_, cudaStrea
         if (e == cudaSuccess) e = cudaMalloc((void **)q, n * sizeof(double2));
     };
     A(&g, oct);
-    A(&tw, (size_t)ni_ + nj_ + nl_);
+    A(&tw, (size_t)2 * (ni_ + nj_ + nl_));
     A(&work, wst);
     A(&p, n3);
     A(&pmin, n3);
@@ -595,13 +840,13 @@ cudaError_t Fp64Buffers::ensure(int ni_, int nj_, int nl_, double kd_, cudaStrea
     nj = nj_;
     nl = nl_;
     kd = kd_;
-    // twiddles exp(-2 pi i k / 2n), k < n, per axis, in FP64
-    std::vector<double2> t((size_t)ni + nj + nl);
+    // twiddles exp(-2 pi i k / 2n), k < 2n, per axis, in FP64
+    std::vector<double2> t((size_t)2 * (ni + nj + nl));
     const double pi = 3.14159265358979323846264338327950288;
     const int ns[3] = {ni, nj, nl};
     size_t o = 0;
     for (int ax = 0; ax < 3; ax++)
-        for (int k = 0; k < ns[ax]; k++, o++)
+        for (int k = 0; k < 2 * ns[ax]; k++, o++)
             t[o] = make_double2(std::cos(-pi * k / ns[ax]), std::sin(-pi * k / ns[ax]));
     if ((e = cudaMemcpyAsync(tw, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice, st)) ||
         (e = green_build_octant64(ni, nj, nl, kd, g, st)) || (e = cudaStreamSynchronize(st))) {
@@ -622,8 +867,6 @@ struct Fp64Run {
     long long *launches;
     int matvecs = 0;
 
-    static size_t smem(int M, int lines) { return (size_t)lines * (M + 1) * sizeof(double2); }
-
     // out = sv v - alpha_m conv(src) on active cells (0 elsewhere); conj: the conjugate
     // operator with conj(alpha) (Convolution_conj)
     cudaError_t matvec(const double2 *src, double2 *out, double sv, const double2 *v, int conj)
@@ -631,15 +874,9 @@ struct Fp64Run {
         Mv64 a = m;
         a.conj = conj;
         Ep64 ep{1, sv, v, f.occ, f.mv, f.alpha, conj};
-        const int ni = a.ni, nj = a.nj, nl = a.nl, tz = 2 * nl < kTZ ? 2 * nl : kTZ;
-        z_fwd<<<dim3(nb(nj, kLJ), ni, 3), kT, smem(2 * nl, kLJ), st>>>(a, src);
-        y_pass<<<dim3(2 * nl / tz, ni, 3), kT, smem(2 * nj, tz), st>>>(a, 0, tz);
-        x_pass<<<dim3(2 * nl / tz, 2 * nj), kT, smem(2 * ni, 3 * tz), st>>>(a, tz);
-        y_pass<<<dim3(2 * nl / tz, ni, 3), kT, smem(2 * nj, tz), st>>>(a, 1, tz);
-        z_inv<<<dim3(nb(nj, kLJ), ni, 3), kT, smem(2 * nl, kLJ), st>>>(a, ep, out);
         *launches += 5;
         matvecs++;
-        return cudaGetLastError();
+        return matvec64(a, ep, src, out, st);
     }
 
     cudaError_t reduce(int kind, const double2 *a, const double2 *b, double out[2])
@@ -700,15 +937,9 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
     typedef std::complex<double> cd;
     const int ni = B.ni, nj = B.nj, nl = B.nl;
     const size_t N = (size_t)ni * nj * nl;
-    // the passes hold up to 3 kTZ lines of 2n + 1 points in shared memory
-    const int big = (int)Fp64Run::smem(2 * ni, 3 * kTZ);
-    CKE(raise_smem_limit((const void *)x_pass, big));
-    CKE(raise_smem_limit((const void *)y_pass, (int)Fp64Run::smem(2 * nj, kTZ)));
-    CKE(raise_smem_limit((const void *)z_fwd, (int)Fp64Run::smem(2 * nl, kLJ)));
-    CKE(raise_smem_limit((const void *)z_inv, (int)Fp64Run::smem(2 * nl, kLJ)));
     CKE(cudaMemcpyAsync(B.alpha, P.alpha, P.nmat1 * sizeof(double2), cudaMemcpyHostToDevice, st));
     F64 f{N, ni, nj, nl, P.occ, P.mv, B.alpha};
-    Mv64 m{ni, nj, nl, N, B.tw, B.tw + ni, B.tw + ni + nj, B.g, B.work, 0};
+    Mv64 m{ni, nj, nl, N, B.tw, B.tw + 2 * ni, B.tw + 2 * (ni + nj), B.g, B.work, 0};
     Fp64Run X{B, st, f, m, P.nact, launches};
     double2 *p = B.p, *pmin = B.pmin, *r = B.r, *s = B.s, *g = B.gg, *h = B.h, *w = B.w, *b = B.b;
     const size_t bytes = 3 * N * sizeof(double2);
