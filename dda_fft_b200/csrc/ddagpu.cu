@@ -1177,30 +1177,37 @@ int ddagpu_autotune(ddagpu_ctx *c, int nrhs)
     return DDAGPU_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// A host field of cvectors [N][3] into [3][N] on the device: copied as it is (through c->w,
+// idle between solves) and transposed there, not on the host.
+int upload_field(ddagpu_ctx *c, const float *p, float2 *dst)
+{
+    CK(cudaMemcpyAsync(c->w, p, 3 * c->N * sizeof(float2), cudaMemcpyHostToDevice, c->st));
+    CK(field_to_soa(c->w, dst, c->N, c->st));
+    c->launches += 1;
+    return DDAGPU_OK;
+}
+}  // namespace
+
+extern "C" {
+
 int ddagpu_convolution(ddagpu_ctx *c, const float *p, float *out, int conj)
 {
     if (!c || !p || !out) return fail(DDAGPU_EINVAL, "null argument");
     std::lock_guard<std::mutex> lk(c->mu);
     DevGuard dg(c->dev);
     const size_t N = c->N;
-    // AoS cvector -> SoA complex planes on the host side of the copy
-    std::vector<float2> soa(3 * N);
-    for (size_t q = 0; q < N; q++)
-        for (int k = 0; k < 3; k++) soa[k * N + q] = make_float2(p[6 * q + 2 * k], p[6 * q + 2 * k + 1]);
-    CK(cudaMemcpyAsync(c->p, soa.data(), 3 * N * sizeof(float2), cudaMemcpyHostToDevice, c->st));
+    RET(upload_field(c, p, c->p));
     MatvecArgs a = mv_args(c, 1, c->p, c->r, 0, 0.f, nullptr, conj ? 1 : 0, 1, false);
     CK(launch_matvec(a, c->st));
-    CK(cudaMemcpyAsync(soa.data(), c->r, 3 * N * sizeof(float2), cudaMemcpyDeviceToHost, c->st));
+    CK(field_to_aos(c->r, c->w, N, c->st));
+    CK(cudaMemcpyAsync(out, c->w, 3 * N * sizeof(float2), cudaMemcpyDeviceToHost, c->st));
     int werr = 0;
     CK(cudaMemcpyAsync(&werr, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    RET(device_wait_error(c, werr));
-    for (size_t q = 0; q < N; q++)
-        for (int k = 0; k < 3; k++) {
-            out[6 * q + 2 * k] = soa[k * N + q].x;
-            out[6 * q + 2 * k + 1] = soa[k * N + q].y;
-        }
-    return DDAGPU_OK;
+    return device_wait_error(c, werr);
 }
 
 }  // extern "C"
@@ -1720,21 +1727,6 @@ int mixed_refine(ddagpu_ctx *c, const float *cListMaterials, int nmat1, int nact
     return DDAGPU_OK;
 }
 
-void aos_to_soa(const float *in, float2 *out, size_t N)
-{
-    for (size_t q = 0; q < N; q++)
-        for (int k = 0; k < 3; k++) out[k * N + q] = make_float2(in[6 * q + 2 * k], in[6 * q + 2 * k + 1]);
-}
-
-void soa_to_aos(const float2 *in, float *out, size_t N)
-{
-    for (size_t q = 0; q < N; q++)
-        for (int k = 0; k < 3; k++) {
-            out[6 * q + 2 * k] = in[k * N + q].x;
-            out[6 * q + 2 * k + 1] = in[k * N + q].y;
-        }
-}
-
 }  // namespace
 
 extern "C" {
@@ -1765,9 +1757,7 @@ int ddagpu_solve_linear(ddagpu_ctx *c, int solver, float rTau, const float *cLis
     CK(cudaMemcpyAsync(c->alpha, al.data(), nmat1 * sizeof(float2), cudaMemcpyHostToDevice, c->st));
     // nact: counted by upload_materials
     if (nact == 0) return fail(DDAGPU_EINVAL, "no active dipoles");
-    std::vector<float2> soa(n3);
-    aos_to_soa(rhs, soa.data(), c->N);
-    CK(cudaMemcpyAsync(c->b32, soa.data(), n3 * sizeof(float2), cudaMemcpyHostToDevice, c->st));
+    RET(upload_field(c, rhs, c->b32));
     ddagpu_refine_info ri;
     std::memset(&ri, 0, sizeof ri);
     if (refine && solver == 0) {
@@ -1793,9 +1783,10 @@ int ddagpu_solve_linear(ddagpu_ctx *c, int solver, float rTau, const float *cLis
         ri.err = S.restored ? S.err_min : S.err;
         ri.err_history[0] = ri.err;
     }
-    CK(cudaMemcpyAsync(soa.data(), c->p, n3 * sizeof(float2), cudaMemcpyDeviceToHost, c->st));
+    CK(field_to_aos(c->p, c->w, c->N, c->st));
+    c->launches += 1;
+    CK(cudaMemcpyAsync(x_out, c->w, n3 * sizeof(float2), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    soa_to_aos(soa.data(), x_out, c->N);
     if (info) *info = ri;
     return DDAGPU_OK;
 }
@@ -1903,18 +1894,8 @@ int ddagpu_solve_fp64(ddagpu_ctx *c, int solver, double tau, const double *alpha
     if (nact == 0) return fail(DDAGPU_EINVAL, "no active dipoles");
     if (!c->f64) c->f64 = new Fp64Buffers();
     CK(c->f64->ensure(c->ni, c->nj, c->nl, c->kd, c->st));
-    const size_t N = c->N;
-    // the reference's cvector layout [N][3] <-> structure of arrays [3][N]
-    auto to_soa = [&](const double *in, std::vector<double2> &out) {
-        out.resize(3 * N);
-        for (size_t q = 0; q < N; q++)
-            for (int k = 0; k < 3; k++) out[k * N + q] = make_double2(in[6 * q + 2 * k], in[6 * q + 2 * k + 1]);
-    };
-    std::vector<double2> al((size_t)nmat1), rs, xs, ps;
+    std::vector<double2> al((size_t)nmat1);
     for (int m = 0; m < nmat1; m++) al[(size_t)m] = make_double2(alpha[2 * m], alpha[2 * m + 1]);
-    if (rhs) to_soa(rhs, rs);
-    if (x0) to_soa(x0, xs);
-    if (p_out) ps.resize(3 * N);
     Fp64Problem P{};
     P.solver = solver;
     P.tau = tau;
@@ -1926,27 +1907,21 @@ int ddagpu_solve_fp64(ddagpu_ctx *c, int solver, double tau, const double *alpha
     P.d0 = d0;
     for (int k = 0; k < 3; k++) P.kinc[k] = kinc[k];
     for (int k = 0; k < 6; k++) P.einc[k] = Einc[k];
-    P.rhs = rhs ? rs.data() : nullptr;
-    P.x0 = x0 ? xs.data() : nullptr;
+    P.rhs = reinterpret_cast<const double2 *>(rhs);
+    P.x0 = reinterpret_cast<const double2 *>(x0);
     P.max_step = Max_Step;
     P.err_max = Error_max;
     P.ndir = ndir;
     P.ksc = ksc;
     Fp64Result R;
     R.esc = Esc;
-    R.p = p_out ? ps.data() : nullptr;
+    R.p = reinterpret_cast<double2 *>(p_out);
     R.trace = trace;
     R.trace_len = trace ? Max_Step + 1 : 0;
     if (trace) std::fill(trace, trace + Max_Step + 1, 0.0);
     CK(solve_fp64(*c->f64, P, c->st, R, &c->launches));
     *Cabs = R.cabs;
     *Cext = R.cext;
-    if (p_out)
-        for (size_t q = 0; q < N; q++)
-            for (int k = 0; k < 3; k++) {
-                p_out[6 * q + 2 * k] = ps[k * N + q].x;
-                p_out[6 * q + 2 * k + 1] = ps[k * N + q].y;
-            }
     if (info) {
         info->steps = R.steps;
         info->step_min = R.step_min;
@@ -1980,11 +1955,7 @@ int ddagpu_farfield(ddagpu_ctx *c, const int *iListMV, int n_mat, const signed c
     int nact = 0;
     RET(upload_materials(c, iListMV, nmat1, cAlpha, &nact));
     RET(ensure_post(c, std::max(ndir, 1), 1, 1));
-    const size_t N = c->N;
-    std::vector<float2> soa(3 * N);
-    for (size_t q = 0; q < N; q++)
-        for (int k = 0; k < 3; k++) soa[k * N + q] = make_float2(p[6 * q + 2 * k], p[6 * q + 2 * k + 1]);
-    CK(cudaMemcpyAsync(c->p, soa.data(), 3 * N * sizeof(float2), cudaMemcpyHostToDevice, c->st));
+    RET(upload_field(c, p, c->p));
     std::vector<double> kd((size_t)ndir * 3);
     for (size_t k = 0; k < kd.size(); k++) kd[k] = ksc[k];
     std::vector<float2> zero_alpha((size_t)nmat1, make_float2(0.f, 0.f));
@@ -2016,11 +1987,7 @@ int ddagpu_cabscext(ddagpu_ctx *c, float d0, const float *kinc, const float *Ein
     std::vector<int> mv((size_t)nmat1, 1);
     RET(upload_materials(c, mv.data(), nmat1, cAlpha));
     RET(ensure_post(c, 1, 1, 1));
-    const size_t N = c->N;
-    std::vector<float2> soa(3 * N);
-    for (size_t q = 0; q < N; q++)
-        for (int k = 0; k < 3; k++) soa[k * N + q] = make_float2(p[6 * q + 2 * k], p[6 * q + 2 * k + 1]);
-    CK(cudaMemcpyAsync(c->p, soa.data(), 3 * N * sizeof(float2), cudaMemcpyHostToDevice, c->st));
+    RET(upload_field(c, p, c->p));
     std::vector<float2> al((size_t)nmat1);
     for (int m = 0; m < nmat1; m++) al[(size_t)m] = make_float2(cListMaterials[2 * m], cListMaterials[2 * m + 1]);
     double kd3[3] = {kinc[0], kinc[1], kinc[2]}, ed6[6];

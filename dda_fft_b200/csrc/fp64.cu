@@ -735,29 +735,70 @@ __global__ void __launch_bounds__(kT) mixed_apply(F64 f, const double2 *v, const
     if (acc) block_add<1>(e, acc);
 }
 
-// acc[0..1] += sum s w (bilinear), acc[2..3] += sum r s, over active cells
-__global__ void __launch_bounds__(kT) cg_dots(F64 f, const double2 *s, const double2 *w, const double2 *r,
-                                              double *acc)
+// The Krylov scalars stay on the device: every reduction adds into a set of kSet doubles, the
+// update kernels form their coefficients from the set, and the host reads one residual per
+// iteration while the next iteration's matvec already runs.
+constexpr int kSet = 12;
+// CG set: <s,w> (0,1), <r,s> (2,3), <r,w> of the new r (4,5), sum |r| (6)
+// BiCGStab set: rho (0,1), <g,h> (2,3), <w,r> (4,5), <w,w> (6,7), sum |r| (8)
+
+__device__ __forceinline__ double2 set_at(const double *a, int k) { return make_double2(a[k], a[k + 1]); }
+__device__ __forceinline__ double2 ddiv(double2 a, double2 b)
+{
+    const double d = b.x * b.x + b.y * b.y;
+    return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
+}
+__device__ __forceinline__ void bil_add(double &re, double &im, double2 a, double2 b)
+{
+    re += a.x * b.x - a.y * b.y;
+    im += a.x * b.y + a.y * b.x;
+}
+
+// acc[0..1] += sum a b (bilinear), acc[2..3] += sum c d, over active cells; CG: (s, w), (r, s)
+__global__ void __launch_bounds__(kT) two_dots(F64 f, const double2 *a, const double2 *b, const double2 *c,
+                                               const double2 *d, double *acc)
 {
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < f.N; q += (size_t)gridDim.x * blockDim.x) {
         if (!active(f, q)) continue;
-        for (int c = 0; c < 3; c++) {
-            const size_t k = c * f.N + q;
-            const double2 a = s[k], b = w[k], d = r[k];
-            v[0] += a.x * b.x - a.y * b.y;
-            v[1] += a.x * b.y + a.y * b.x;
-            v[2] += d.x * a.x - d.y * a.y;
-            v[3] += d.x * a.y + d.y * a.x;
+        for (int k = 0; k < 3; k++) {
+            const size_t o = k * f.N + q;
+            bil_add(v[0], v[1], a[o], b[o]);
+            if (c) bil_add(v[2], v[3], c[o], d[o]);
         }
     }
     block_add<4>(v, acc);
 }
 
-// x -= a s; r -= a w on active cells; acc[0..1] += sum r w, acc[2] += sum |r| (the new r)
-__global__ void __launch_bounds__(kT) cg_update(F64 f, double2 a, double2 *x, double2 *r, const double2 *s,
-                                                const double2 *w, double *acc)
+// w = s - alpha_m conv on active cells (0 elsewhere) and the dots of CG in the same pass
+__global__ void __launch_bounds__(kT) mixed_apply_dots(F64 f, const double2 *s, const float2 *conv, const double2 *r,
+                                                       double2 *w, double *acc)
 {
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < f.N; q += (size_t)gridDim.x * blockDim.x) {
+        const int m = f.occ[q];
+        if (!f.mv[m]) {
+            for (int k = 0; k < 3; k++) w[k * f.N + q] = dzero();
+            continue;
+        }
+        const double2 al = f.alpha[m];
+        for (int k = 0; k < 3; k++) {
+            const size_t o = k * f.N + q;
+            const float2 g = conv[o];
+            const double2 sv = s[o], wv = dsub(sv, dmul(al, make_double2(g.x, g.y)));
+            w[o] = wv;
+            bil_add(v[0], v[1], sv, wv);
+            bil_add(v[2], v[3], r[o], sv);
+        }
+    }
+    block_add<4>(v, acc);
+}
+
+// a = <r,s> / <s,w>: x -= a s; r -= a w on active cells; set[4..5] += sum r w, set[6] += sum |r|
+__global__ void __launch_bounds__(kT) cg_update(F64 f, double2 *x, double2 *r, const double2 *s, const double2 *w,
+                                                double *set)
+{
+    const double2 a = ddiv(set_at(set, 2), set_at(set, 0));
     double v[3] = {0.0, 0.0, 0.0};
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < f.N; q += (size_t)gridDim.x * blockDim.x) {
         if (!active(f, q)) continue;
@@ -768,27 +809,92 @@ __global__ void __launch_bounds__(kT) cg_update(F64 f, double2 a, double2 *x, do
             x[k] = dsub(x[k], dmul(a, sv));
             const double2 rv = dsub(r[k], dmul(a, wv));
             r[k] = rv;
-            v[0] += rv.x * wv.x - rv.y * wv.y;
-            v[1] += rv.x * wv.y + rv.y * wv.x;
+            bil_add(v[0], v[1], rv, wv);
             t += rv.x * rv.x + rv.y * rv.y;
         }
         v[2] += sqrt(t);
     }
-    block_add<3>(v, acc);
+    block_add<3>(v, set + 4);
 }
 
-// s = r - b s on active cells (inactive cells keep their zeros); s32 = float(s)
-__global__ void cg_dir(F64 f, double2 b, const double2 *r, double2 *s, float2 *s32)
+// b = <r,w> / <s,w>: s = r - b s on active cells (inactive cells keep their zeros); s32 (may
+// be null) = float(s)
+__global__ void cg_dir(F64 f, const double *set, const double2 *r, double2 *s, float2 *s32)
 {
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (q >= f.N) return;
+    const double2 b = ddiv(set_at(set, 4), set_at(set, 0));
     const bool act = active(f, q);
     for (int c = 0; c < 3; c++) {
         const size_t k = c * f.N + q;
         double2 v = s[k];
         if (act) v = dsub(r[k], dmul(b, v));
         s[k] = v;
-        s32[k] = make_float2((float)v.x, (float)v.y);
+        if (s32) s32[k] = make_float2((float)v.x, (float)v.y);
+    }
+}
+
+// BiCGStab (dda_func.cpp:1423-1469): la = rho / <g,h>, lw = <w,r> / <w,w> of a set
+// s = r + lb s - lb lw h, lb = (rho la1) / (rho1 lw1), from the new rho and the last set
+__global__ void bi_dir(F64 f, const double *last, const double *cur, const double2 *r, const double2 *h, double2 *s)
+{
+    const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (q >= f.N) return;
+    const double2 rho1 = set_at(last, 0), la = ddiv(rho1, set_at(last, 2)), lw = ddiv(set_at(last, 4), set_at(last, 6));
+    const double2 lb = ddiv(dmul(set_at(cur, 0), la), dmul(rho1, lw)), c2 = dmul(lb, lw);
+    const bool act = active(f, q);
+    for (int c = 0; c < 3; c++) {
+        const size_t k = c * f.N + q;
+        s[k] = act ? dsub(dadd(r[k], dmul(lb, s[k])), dmul(c2, h[k])) : dzero();
+    }
+}
+
+// r -= la h on active cells
+__global__ void bi_r(F64 f, const double *set, const double2 *h, double2 *r)
+{
+    const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (q >= f.N || !active(f, q)) return;
+    const double2 la = ddiv(set_at(set, 0), set_at(set, 2));
+    for (int c = 0; c < 3; c++) {
+        const size_t k = c * f.N + q;
+        r[k] = dsub(r[k], dmul(la, h[k]));
+    }
+}
+
+// p = p - la s - lw r (0 on inactive cells); r -= lw w; set[8] += sum |r|, next[0..1] += <r,g>
+__global__ void __launch_bounds__(kT) bi_update(F64 f, double *set, double *next, double2 *p, double2 *r,
+                                                const double2 *s, const double2 *w, const double2 *g)
+{
+    const double2 la = ddiv(set_at(set, 0), set_at(set, 2)), lw = ddiv(set_at(set, 4), set_at(set, 6));
+    double e[1] = {0.0}, v[2] = {0.0, 0.0};
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < f.N; q += (size_t)gridDim.x * blockDim.x) {
+        if (!active(f, q)) {
+            for (int c = 0; c < 3; c++) p[c * f.N + q] = dzero();
+            continue;
+        }
+        double t = 0.0;
+        for (int c = 0; c < 3; c++) {
+            const size_t k = c * f.N + q;
+            const double2 rv = r[k], rn = dsub(rv, dmul(lw, w[k]));
+            p[k] = dsub(dsub(p[k], dmul(la, s[k])), dmul(lw, rv));
+            r[k] = rn;
+            bil_add(v[0], v[1], rn, g[k]);
+            t += rn.x * rn.x + rn.y * rn.y;
+        }
+        e[0] += sqrt(t);
+    }
+    block_add<1>(e, set + 8);
+    block_add<2>(v, next);
+}
+
+// the reference's cvector layout [N][3] <-> structure of arrays [3][N]
+template <class T>
+__global__ void aos_soa(const T *in, T *out, size_t N, int to_soa)
+{
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < 3 * N; e += (size_t)gridDim.x * blockDim.x) {
+        const size_t q = e / 3, c = e - 3 * q;
+        if (to_soa) out[c * N + q] = in[e];
+        else out[e] = in[c * N + q];
     }
 }
 
@@ -796,15 +902,63 @@ __global__ void cg_dir(F64 f, double2 b, const double2 *r, double2 *s, float2 *s
 
 // ------------------------------------------------------------------ host side
 
+template <class T>
+static cudaError_t layout(const T *in, T *out, size_t N, int to_soa, cudaStream_t st)
+{
+    aos_soa<T><<<4 * 148, kT, 0, st>>>(in, out, N, to_soa);
+    return cudaGetLastError();
+}
+cudaError_t field_to_soa(const float2 *aos, float2 *soa, size_t N, cudaStream_t st) { return layout(aos, soa, N, 1, st); }
+cudaError_t field_to_aos(const float2 *soa, float2 *aos, size_t N, cudaStream_t st) { return layout(soa, aos, N, 0, st); }
+
+// Pinned slot and event of a residual on its way to the host, and the sets of scalars.
+cudaError_t KrylovScalars::ensure()
+{
+    cudaError_t e = cudaSuccess;
+    if (!acc) e = cudaMalloc((void **)&acc, 3 * kSet * sizeof(double));
+    if (e == cudaSuccess && !pin) e = cudaHostAlloc((void **)&pin, kSet * sizeof(double), cudaHostAllocDefault);
+    if (e == cudaSuccess && !ready) e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+    return e;
+}
+
+void KrylovScalars::release()
+{
+    if (acc) cudaFree(acc);
+    if (pin) cudaFreeHost(pin);
+    if (ready) cudaEventDestroy(ready);
+    acc = pin = nullptr;
+    ready = nullptr;
+}
+
+double *KrylovScalars::set(int k) const { return acc + k * kSet; }
+
+cudaError_t KrylovScalars::zero(int k, cudaStream_t st) const
+{
+    return cudaMemsetAsync(set(k), 0, kSet * sizeof(double), st);
+}
+
+cudaError_t KrylovScalars::send(const double *from, cudaStream_t st) const
+{
+    const cudaError_t e = cudaMemcpyAsync(pin, from, sizeof(double), cudaMemcpyDeviceToHost, st);
+    return e == cudaSuccess ? cudaEventRecord(ready, st) : e;
+}
+
+cudaError_t KrylovScalars::wait(double &v) const
+{
+    const cudaError_t e = cudaEventSynchronize(ready);
+    v = *pin;
+    return e;
+}
+
 Fp64Buffers::~Fp64Buffers() { release(); }
 
 void Fp64Buffers::release()
 {
-    void *ptrs[] = {g, tw, work, p, pmin, r, s, gg, h, w, b, alpha, acc};
+    void *ptrs[] = {g, tw, work, p, pmin, r, s, gg, h, w, b, alpha};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     g = tw = work = p = pmin = r = s = gg = h = w = b = alpha = nullptr;
-    acc = nullptr;
+    scal.release();
     ni = nj = nl = 0;
 }
 
@@ -831,7 +985,7 @@ cudaError_t Fp64Buffers::ensure(int ni_, int nj_, int nl_, double kd_, cudaStrea
     A(&w, n3);
     A(&b, n3);
     A(&alpha, 256);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&acc, 8 * sizeof(double));
+    if (e == cudaSuccess) e = scal.ensure();
     if (e != cudaSuccess) {
         release();
         return e;
@@ -881,19 +1035,12 @@ struct Fp64Run {
 
     cudaError_t reduce(int kind, const double2 *a, const double2 *b, double out[2])
     {
-        cudaError_t e = cudaMemsetAsync(B.acc, 0, 2 * sizeof(double), st);
+        cudaError_t e = cudaMemsetAsync(B.scal.acc, 0, 2 * sizeof(double), st);
         if (e) return e;
-        reduce64<<<4 * 148, kT, 0, st>>>(f, kind, a, b, B.acc);
+        reduce64<<<4 * 148, kT, 0, st>>>(f, kind, a, b, B.scal.acc);
         *launches += 1;
-        if ((e = cudaMemcpyAsync(out, B.acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, st))) return e;
+        if ((e = cudaMemcpyAsync(out, B.scal.acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, st))) return e;
         return cudaStreamSynchronize(st);
-    }
-    cudaError_t bil(const double2 *a, const double2 *b, std::complex<double> &z)
-    {
-        double o[2];
-        cudaError_t e = reduce(0, a, b, o);
-        z = {o[0], o[1]};
-        return e;
     }
     cudaError_t herm(const double2 *a, const double2 *b, double &x)
     {
@@ -917,6 +1064,28 @@ struct Fp64Run {
         *launches += 1;
         return cudaGetLastError();
     }
+    cudaError_t dots(const double2 *a, const double2 *b, const double2 *c, const double2 *d, double *acc)
+    {
+        two_dots<<<4 * 148, kT, 0, st>>>(f, a, b, c, d, acc);
+        *launches += 1;
+        return cudaGetLastError();
+    }
+    // the rest of a BiCGStab step after h = A s: set cur holds its rho, next (zeroed here) the
+    // next step's; p, r updated and the residual sum sent to the host
+    cudaError_t bicg_step(double2 *p, double2 *r, const double2 *s, const double2 *g, const double2 *h, double2 *w,
+                          int cur, int next)
+    {
+        const KrylovScalars &K = B.scal;
+        cudaError_t e = dots(g, h, nullptr, nullptr, K.set(cur) + 2);
+        if (e) return e;
+        bi_r<<<nb(f.N, kT), kT, 0, st>>>(f, K.set(cur), h, r);
+        if ((e = matvec(r, w, 1.0, r, 0))) return e;
+        if ((e = dots(w, r, w, w, K.set(cur) + 4))) return e;
+        if ((e = K.zero(next, st))) return e;
+        bi_update<<<4 * 148, kT, 0, st>>>(f, K.set(cur), K.set(next), p, r, s, w, g);
+        *launches += 2;
+        return K.send(K.set(cur) + 8, st);
+    }
     cudaError_t copy(double2 *dst, const double2 *src)
     {
         return cudaMemcpyAsync(dst, src, 3 * f.N * sizeof(double2), cudaMemcpyDeviceToDevice, st);
@@ -934,7 +1103,6 @@ struct Fp64Run {
 cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp64Result &R,
                        long long *launches)
 {
-    typedef std::complex<double> cd;
     const int ni = B.ni, nj = B.nj, nl = B.nl;
     const size_t N = (size_t)ni * nj * nl;
     CKE(cudaMemcpyAsync(B.alpha, P.alpha, P.nmat1 * sizeof(double2), cudaMemcpyHostToDevice, st));
@@ -946,14 +1114,19 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
     const int solver = P.solver;
 
     // right-hand side b (p_inc or the caller's), start p = x0 or b (dda_func.cpp:1102-1104)
-    if (P.rhs) CKE(cudaMemcpyAsync(w, P.rhs, bytes, cudaMemcpyHostToDevice, st));
+    // (the caller's fields are [N][3]; the FFT work space is the staging buffer)
+    if (P.rhs) {
+        CKE(cudaMemcpyAsync(B.work, P.rhs, bytes, cudaMemcpyHostToDevice, st));
+        CKE(layout(B.work, w, N, 1, st));
+    }
     first_approx64<<<nb(N, kT), kT, 0, st>>>(f, P.d0, P.kinc[0], P.kinc[1], P.kinc[2],
                                              make_double2(P.einc[0], P.einc[1]),
                                              make_double2(P.einc[2], P.einc[3]),
                                              make_double2(P.einc[4], P.einc[5]), P.rhs ? w : nullptr, b);
     *launches += 1;
     if (P.x0) {
-        CKE(cudaMemcpyAsync(w, P.x0, bytes, cudaMemcpyHostToDevice, st));
+        CKE(cudaMemcpyAsync(B.work, P.x0, bytes, cudaMemcpyHostToDevice, st));
+        CKE(layout(B.work, w, N, 1, st));
         CKE(X.lin3(w, 0.0, nullptr, 0.0, nullptr, p, 1));          // p = x0 on active cells
         CKE(X.matvec(p, w, 1.0, p, 0));                              // w = A p
         CKE(X.lin3(w, -1.0, b, 0.0, nullptr, r, 1));                // r = A p - b
@@ -962,7 +1135,6 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
         CKE(X.matvec(p, r, 0.0, nullptr, 0));                        // r = -alpha conv(p)
     }
 
-    cd ldA = 0, ldW = 0, rho1 = 0, z;
     double RR1 = 0;
     if (solver == 0) CKE(X.copy(s, r));
     if (solver == 1) {
@@ -972,30 +1144,29 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
     if (solver == 2) {
         CKE(X.copy(g, r));
         CKE(X.copy(s, r));
-        CKE(X.bil(r, g, rho1));
+        CKE(B.scal.zero(0, st));
+        CKE(X.dots(r, g, nullptr, nullptr, B.scal.set(0)));
         CKE(X.matvec(s, h, 1.0, s, 0));
-        CKE(X.bil(g, h, z));
-        ldA = rho1 / z;
-        CKE(X.lin3(r, -ldA, h, 0.0, nullptr, r, 0));
-        CKE(X.matvec(r, w, 1.0, r, 0));
-        cd wr, ww;
-        CKE(X.bil(w, r, wr));
-        CKE(X.bil(w, w, ww));
-        ldW = wr / ww;
-        CKE(X.lin3(p, -ldA, s, -ldW, r, p, 1));
-        CKE(X.lin3(r, -ldW, w, 0.0, nullptr, r, 0));
+        CKE(X.bicg_step(p, r, s, g, h, w, 0, 1));
     }
     if (solver == 3) {
         CKE(X.copy(s, p));
         CKE(X.lin3(s, -1.0, r, 0.0, nullptr, p, 0));   // p = s - r (r vanishes off the target)
     }
     double err = 0;
-    CKE(X.err(r, err));
+    if (solver == 2) {
+        CKE(B.scal.wait(err));
+        err /= P.nact;
+    } else {
+        CKE(X.err(r, err));
+    }
     double err_min = err;
     int step_min = 0, nt = 0;
     if (R.trace && nt < R.trace_len) R.trace[nt] = err;
     nt++;
     CKE(X.copy(pmin, p));
+    const KrylovScalars &K = B.scal;
+    bool ahead = false;   // the next step's first matvec is already in the stream
     for (int o = 1; o <= P.max_step; o++) {   // dda_func.cpp:1301-1535
         if (err <= P.err_max) break;
         if (err < err_min) {
@@ -1004,33 +1175,30 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
             CKE(X.copy(pmin, p));
         }
         if (solver == 2) {
-            cd rho;
-            CKE(X.bil(r, g, rho));
-            const cd ldB = (rho * ldA) / (rho1 * ldW);
-            CKE(X.lin3(r, ldB, s, -(ldB * ldW), h, s, 1));
-            rho1 = rho;
-            CKE(X.matvec(s, h, 1.0, s, 0));
-            CKE(X.bil(g, h, z));
-            ldA = rho / z;
-            CKE(X.lin3(r, -ldA, h, 0.0, nullptr, r, 0));
-            CKE(X.matvec(r, w, 1.0, r, 0));
-            cd wr, ww;
-            CKE(X.bil(w, r, wr));
-            CKE(X.bil(w, w, ww));
-            ldW = wr / ww;
-            CKE(X.lin3(p, -ldA, s, -ldW, r, p, 1));
-            CKE(X.lin3(r, -ldW, w, 0.0, nullptr, r, 0));
+            if (!ahead) {
+                bi_dir<<<nb(N, kT), kT, 0, st>>>(f, K.set((o - 1) & 1), K.set(o & 1), r, h, s);
+                *launches += 1;
+                CKE(X.matvec(s, h, 1.0, s, 0));
+            }
+            CKE(X.bicg_step(p, r, s, g, h, w, o & 1, (o + 1) & 1));
+            // the next step's direction and first product run while the residual travels;
+            // neither p nor r changes, so a step that turns out not to be needed costs nothing else
+            if ((ahead = o < P.max_step)) {
+                bi_dir<<<nb(N, kT), kT, 0, st>>>(f, K.set(o & 1), K.set((o + 1) & 1), r, h, s);
+                *launches += 1;
+                CKE(X.matvec(s, h, 1.0, s, 0));
+            }
+            CKE(K.wait(err));
         } else if (solver == 0) {
-            CKE(X.matvec(s, w, 1.0, s, 0));
-            cd den, rs, rw;
-            CKE(X.bil(s, w, den));
-            CKE(X.bil(r, s, rs));
-            const cd a = rs / den;
-            CKE(X.lin3(p, -a, s, 0.0, nullptr, p, 0));
-            CKE(X.lin3(r, -a, w, 0.0, nullptr, r, 0));
-            CKE(X.bil(r, w, rw));
-            const cd bb = rw / den;
-            CKE(X.lin3(r, -bb, s, 0.0, nullptr, s, 0));
+            if (!ahead) CKE(X.matvec(s, w, 1.0, s, 0));
+            CKE(K.zero(0, st));
+            CKE(X.dots(s, w, r, s, K.set(0)));
+            cg_update<<<4 * 148, kT, 0, st>>>(f, p, r, s, w, K.set(0));
+            CKE(K.send(K.set(0) + 6, st));
+            cg_dir<<<nb(N, kT), kT, 0, st>>>(f, K.set(0), r, s, nullptr);
+            *launches += 2;
+            if ((ahead = o < P.max_step)) CKE(X.matvec(s, w, 1.0, s, 0));
+            CKE(K.wait(err));
         } else if (solver == 1) {
             CKE(X.matvec(s, w, 1.0, s, 0));
             double SS, RR;
@@ -1048,10 +1216,12 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
             simple64<<<nb(N, kT), kT, 0, st>>>(f, w, s, r, p, P.tau);
             *launches += 1;
         }
-        CKE(X.err(r, err));
+        if (solver == 0 || solver == 2) err /= P.nact;
+        else CKE(X.err(r, err));
         if (R.trace && nt < R.trace_len) R.trace[nt] = err;
         nt++;
     }
+    if (ahead) X.matvecs -= 1;   // of the step that was not taken
     R.steps = nt - 1;
     R.err = err;
     R.err_min = err < err_min ? err : err_min;
@@ -1063,13 +1233,13 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
     R.rolled_back = R.step_min >= 0;
     R.matvecs = X.matvecs;
     // CabsCext and the far field of the final dipoles
-    CKE(cudaMemsetAsync(B.acc, 0, 2 * sizeof(double), st));
+    CKE(cudaMemsetAsync(B.scal.acc, 0, 2 * sizeof(double), st));
     cabscext64<<<4 * 148, kT, 0, st>>>(f, P.nmat1, P.d0, P.kinc[0], P.kinc[1], P.kinc[2],
                                        make_double2(P.einc[0], P.einc[1]), make_double2(P.einc[2], P.einc[3]),
-                                       make_double2(P.einc[4], P.einc[5]), p, B.acc);
+                                       make_double2(P.einc[4], P.einc[5]), p, B.scal.acc);
     *launches += 1;
     double cc[2];
-    CKE(cudaMemcpyAsync(cc, B.acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CKE(cudaMemcpyAsync(cc, B.scal.acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
     if (P.ndir > 0) {
         double *kd = nullptr, *ed = nullptr;
         CKE(cudaMallocAsync((void **)&kd, (size_t)P.ndir * 3 * sizeof(double), st));
@@ -1088,7 +1258,10 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
     const double pi = 3.14159265358979323846264338327950288;
     R.cext = 4.0 * pi / e2 * cc[0];
     R.cabs = 4.0 * pi / e2 * cc[1];
-    if (R.p) CKE(cudaMemcpyAsync(R.p, p, bytes, cudaMemcpyDeviceToHost, st));
+    if (R.p) {
+        CKE(layout(p, B.work, N, 0, st));
+        CKE(cudaMemcpyAsync(R.p, B.work, bytes, cudaMemcpyDeviceToHost, st));
+    }
     return cudaStreamSynchronize(st);
 }
 
@@ -1098,11 +1271,11 @@ MixedCgBuffers::~MixedCgBuffers() { release(); }
 
 void MixedCgBuffers::release()
 {
-    void *ptrs[] = {x, r, s, w, b, best, alpha, acc};
+    void *ptrs[] = {x, r, s, w, b, best, alpha};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     x = r = s = w = b = best = alpha = nullptr;
-    acc = nullptr;
+    scal.release();
     n3 = 0;
 }
 
@@ -1121,7 +1294,7 @@ cudaError_t MixedCgBuffers::ensure(size_t n)
     A(&b, n);
     A(&best, n);
     A(&alpha, 256);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&acc, 8 * sizeof(double));
+    if (e == cudaSuccess) e = scal.ensure();
     if (e != cudaSuccess) {
         release();
         return e;
@@ -1150,25 +1323,20 @@ cudaError_t mixed_cg(MixedCgBuffers &B, const Field64View &f, const double2 *alp
                      const ConvFn &conv, float2 *s32, float2 *conv32, float2 *x32, float2 *p32,
                      cudaStream_t st, MixedCgResult &R, long long *launches)
 {
-    typedef std::complex<double> cd;
     const size_t N = f.N, n3 = 3 * N, bytes = n3 * sizeof(double2);
     const unsigned red = 4 * 148;
-    double h[4];
-    auto sums = [&](int k) -> cudaError_t {
-        CKE(cudaMemcpyAsync(h, B.acc, k * sizeof(double), cudaMemcpyDeviceToHost, st));
-        return cudaStreamSynchronize(st);
-    };
-    auto zero = [&]() { return cudaMemsetAsync(B.acc, 0, 4 * sizeof(double), st); };
+    const KrylovScalars &K = B.scal;
     // true residual r = x - alpha G*x - b and its discrepancy (ldError of it)
     auto true_residual = [&](double &err) -> cudaError_t {
         to_f32<<<red, kT, 0, st>>>(B.x, x32, n3);
         CKE(conv(x32, conv32));
-        CKE(zero());
-        mixed_apply<<<red, kT, 0, st>>>(f, B.x, conv32, B.b, B.r, B.acc);
+        CKE(K.zero(1, st));
+        mixed_apply<<<red, kT, 0, st>>>(f, B.x, conv32, B.b, B.r, K.set(1));
         *launches += 2;
         R.matvecs++;
-        CKE(sums(1));
-        err = h[0] / nact;
+        CKE(K.send(K.set(1), st));
+        CKE(K.wait(err));
+        err /= nact;
         return cudaSuccess;
     };
     CKE(cudaMemcpyAsync(B.alpha, alpha_host, nmat1 * sizeof(double2), cudaMemcpyHostToDevice, st));
@@ -1185,27 +1353,26 @@ cudaError_t mixed_cg(MixedCgBuffers &B, const Field64View &f, const double2 *alp
         *launches += 1;
         int since = 0;
         const long long cap = (long long)(max_outer + 1) * inner_max_step;
+        bool ahead = false;   // the next direction's convolution is already in the stream
         for (long long it = 0; it < cap; it++) {
-            // w = A s (dda_func.cpp:1325-1357)
-            CKE(conv(s32, conv32));
-            mixed_apply<<<red, kT, 0, st>>>(f, B.s, conv32, nullptr, B.w, nullptr);
-            CKE(zero());
-            cg_dots<<<red, kT, 0, st>>>(f, B.s, B.w, B.r, B.acc);
-            *launches += 2;
+            // w = A s (dda_func.cpp:1325-1357) and the dots of the step (1359-1371, without the
+            // float casts); the residual travels to the host while the next convolution runs
+            if (!ahead) CKE(conv(s32, conv32));
+            CKE(K.zero(0, st));
+            mixed_apply_dots<<<red, kT, 0, st>>>(f, B.s, conv32, B.r, B.w, K.set(0));
             R.matvecs++;
-            CKE(sums(4));
-            const cd den(h[0], h[1]), rs(h[2], h[3]);
-            const cd a = rs / den;   // dda_func.cpp:1359-1371, without the float casts
-            CKE(zero());
-            cg_update<<<red, kT, 0, st>>>(f, make_double2(a.real(), a.imag()), B.x, B.r, B.s, B.w, B.acc);
-            CKE(sums(3));
-            const cd bb = cd(h[0], h[1]) / den;
-            const double err_rec = h[2] / nact;
-            cg_dir<<<nb(N, kT), kT, 0, st>>>(f, make_double2(bb.real(), bb.imag()), B.r, B.s, s32);
-            *launches += 2;
+            cg_update<<<red, kT, 0, st>>>(f, B.x, B.r, B.s, B.w, K.set(0));
+            CKE(K.send(K.set(0) + 6, st));
+            cg_dir<<<nb(N, kT), kT, 0, st>>>(f, K.set(0), B.r, B.s, s32);
+            *launches += 3;
+            if ((ahead = it + 1 < cap)) CKE(conv(s32, conv32));
+            double err_rec;
+            CKE(K.wait(err_rec));
+            err_rec /= nact;
             R.iterations++;
             since++;
             if (err_rec <= err_max || err_rec <= inner_rel * anchor || since >= inner_max_step) {
+                ahead = false;
                 CKE(true_residual(err));
                 R.outer++;
                 if (R.outer < 64) R.history[R.outer] = err;

@@ -10,6 +10,23 @@ namespace ddagpu {
 // FP64 octant of the Green tensor FFT, [comp][kx][ky][kz] for k in [0, n]^3 (green.cu)
 cudaError_t green_build_octant64(int ni, int nj, int nl, double kd, double2 *out, cudaStream_t st);
 
+// Device scalars of an FP64 Krylov iteration (three sets of sums) and the pinned slot and
+// event that bring one residual to the host while the stream goes on.
+struct KrylovScalars {
+    double *acc = nullptr, *pin = nullptr;
+    cudaEvent_t ready = nullptr;
+    cudaError_t ensure();
+    void release();
+    double *set(int k) const;
+    cudaError_t zero(int k, cudaStream_t st) const;
+    cudaError_t send(const double *from, cudaStream_t st) const;
+    cudaError_t wait(double &v) const;
+};
+
+// float fields between the reference's cvector layout [N][3] and [3][N], on the device
+cudaError_t field_to_soa(const float2 *aos, float2 *soa, size_t N, cudaStream_t st);
+cudaError_t field_to_aos(const float2 *soa, float2 *aos, size_t N, cudaStream_t st);
+
 // Device buffers of the FP64 solve for one lattice, built on first use and kept.
 struct Fp64Buffers {
     int ni = 0, nj = 0, nl = 0;
@@ -17,7 +34,7 @@ struct Fp64Buffers {
     double2 *g = nullptr, *tw = nullptr, *work = nullptr;
     double2 *p = nullptr, *pmin = nullptr, *r = nullptr, *s = nullptr, *gg = nullptr, *h = nullptr,
             *w = nullptr, *b = nullptr, *alpha = nullptr;
-    double *acc = nullptr;
+    KrylovScalars scal;
     ~Fp64Buffers();
     void release();
     cudaError_t ensure(int ni, int nj, int nl, double kd, cudaStream_t st);
@@ -33,8 +50,8 @@ struct Fp64Problem {
     int nact;
     double d0;
     double kinc[3], einc[6];
-    const double2 *rhs;       // host [3][N] or null (b = p_inc)
-    const double2 *x0;        // host [3][N] or null (start from b)
+    const double2 *rhs;       // host [N][3] or null (b = p_inc)
+    const double2 *x0;        // host [N][3] or null (start from b)
     int max_step;
     double err_max;
     int ndir;
@@ -46,7 +63,7 @@ struct Fp64Result {
     double err = 0, err_min = 0;
     double cabs = 0, cext = 0;
     double *esc = nullptr;    // host [ndir][6]
-    double2 *p = nullptr;     // host [3][N] or null
+    double2 *p = nullptr;     // host [N][3] or null
     double *trace = nullptr;  // host, trace_len entries, or null
     int trace_len = 0;
 };
@@ -86,7 +103,7 @@ struct MixedCgBuffers {
     size_t n3 = 0;
     double2 *x = nullptr, *r = nullptr, *s = nullptr, *w = nullptr, *b = nullptr, *best = nullptr,
             *alpha = nullptr;
-    double *acc = nullptr;
+    KrylovScalars scal;
     ~MixedCgBuffers();
     void release();
     cudaError_t ensure(size_t n3);
