@@ -93,7 +93,7 @@ __device__ inline int zmapd(int oz, int nl) { return (oz & 1) ? (nl / 2 + 1 + (o
 
 __global__ void to_octant(const double2 *in, float2 *ahat, int ni, int nj, int nl)
 {
-    // in[comp][kx][ky][kz] -> ahat[kx][ky][zmap(kz)][comp]
+    // in[comp][kx][ky][kz] -> ahat[kx][ky][comp / 2][zmap(kz)][comp % 2]
     const size_t per = (size_t)(ni + 1) * (nj + 1) * (nl + 1);
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (q >= 6 * per) return;
@@ -101,7 +101,7 @@ __global__ void to_octant(const double2 *in, float2 *ahat, int ni, int nj, int n
     const size_t xy = (q / (nl + 1)) % ((size_t)(ni + 1) * (nj + 1));
     const int comp = (int)(q / per);
     const double2 v = in[q];
-    ahat[((xy * (nl + 1)) + zmapd(oz, nl)) * 6 + comp] = make_float2((float)v.x, (float)v.y);
+    ahat[((xy * 3 + comp / 2) * (nl + 1) + zmapd(oz, nl)) * 2 + comp % 2] = make_float2((float)v.x, (float)v.y);
 }
 
 // Octant from a dense float Ahat [2ni][2nj][2nl][6] (the reference's cmA layout): the
@@ -130,7 +130,7 @@ __global__ void project_dense(const float2 *dense, float2 *ahat, int ni, int nj,
         sr += s * v.x;
         si += s * v.y;
     }
-    ahat[((((size_t)ox * (nj + 1) + oy) * (nl + 1)) + zmapd(oz, nl)) * 6 + c] =
+    ahat[((((size_t)ox * (nj + 1) + oy) * 3 + c / 2) * (nl + 1) + zmapd(oz, nl)) * 2 + c % 2] =
         make_float2((float)(sr / 8.0), (float)(si / 8.0));
 }
 

@@ -629,9 +629,11 @@ k2f(MatvecArgs a, const __grid_constant__ CUtensorMap tmap)
     const int my = jp > nj, oy = my ? 2 * nj - jp : jp;
     const int ls = l0 + t, hl = ls >= nl, kl = ls - hl * nl, lp = 2 * kl + hl;
     const int mz = lp > nl, oz = mz ? 2 * nl - lp : lp;
-    // Ahat[ox][oy][zmap(oz)][6]: the 6 components of one frequency are one 48-byte entry
-    const size_t sz = 6, sy = (size_t)(nl + 1) * 6, sxo = (size_t)(nj + 1) * sy;
-    const float2 *Ayz = a.ahat + (size_t)oy * sy + (size_t)zmapf(oz, nl) * sz;
+    // Ahat[ox][oy][3][zmap(oz)], two components per float4: consecutive lanes read consecutive
+    // float4s (as 48-byte entries per frequency the three loads took 12 wavefronts each
+    // instead of 4)
+    const size_t sp = (size_t)(nl + 1), sy = 3 * sp, sxo = (size_t)(nj + 1) * sy;
+    const float4 *Ayz = reinterpret_cast<const float4 *>(a.ahat) + (size_t)oy * sy + zmapf(oz, nl);
 #pragma unroll 1
     for (int h = 0; h < 2; h++) {
         float2 X[3][R2];
@@ -656,8 +658,8 @@ k2f(MatvecArgs a, const __grid_constant__ CUtensorMap tmap)
 #pragma unroll 1
                 for (int k = 0; k < R1; k++) {
                     const int kx = 2 * k + h, mx = kx > NI, ox = mx ? 2 * NI - kx : kx;
-                    const float4 *A = reinterpret_cast<const float4 *>(Ayz + (size_t)ox * sxo);
-                    const float4 a01 = __ldg(A), a23 = __ldg(A + 1), a45 = __ldg(A + 2);
+                    const float4 *A = Ayz + (size_t)ox * sxo;
+                    const float4 a01 = __ldg(A), a23 = __ldg(A + sp), a45 = __ldg(A + 2 * sp);
                     float2 g0 = make_float2(a01.x, a01.y), g1 = make_float2(a01.z, a01.w),
                            g2 = make_float2(a23.x, a23.y), g3 = make_float2(a23.z, a23.w),
                            g4 = make_float2(a45.x, a45.y), g5 = make_float2(a45.z, a45.w);
@@ -677,8 +679,8 @@ k2f(MatvecArgs a, const __grid_constant__ CUtensorMap tmap)
 #pragma unroll
                 for (int q = 0; q < R2; q++) {
                     const int kx = 2 * (k1 + R1 * q) + h, mx = kx > NI, ox = mx ? 2 * NI - kx : kx;
-                    const float4 *A = reinterpret_cast<const float4 *>(Ayz + (size_t)ox * sxo);
-                    const float4 a01 = __ldg(A), a23 = __ldg(A + 1), a45 = __ldg(A + 2);
+                    const float4 *A = Ayz + (size_t)ox * sxo;
+                    const float4 a01 = __ldg(A), a23 = __ldg(A + sp), a45 = __ldg(A + 2 * sp);
                     float2 g0 = make_float2(a01.x, a01.y), g1 = make_float2(a01.z, a01.w),
                            g2 = make_float2(a23.x, a23.y), g3 = make_float2(a23.z, a23.w),
                            g4 = make_float2(a45.x, a45.y), g5 = make_float2(a45.z, a45.w);
@@ -838,8 +840,8 @@ __global__ void __launch_bounds__(Sp<NI>::RM * TL, k2_min_blocks(NI, Sp<NI>::RM 
     const int my = jp > nj, oy = my ? 2 * nj - jp : jp;
     const int ls = l0 + t, hl = ls >= nl, kl = ls - hl * nl, lp = 2 * kl + hl;
     const int mz = lp > nl, oz = mz ? 2 * nl - lp : lp;
-    const size_t sz = 6, sy = (size_t)(nl + 1) * 6, sxo = (size_t)(nj + 1) * sy;
-    const float2 *Ayz = a.ahat + (size_t)oy * sy + (size_t)zmapf(oz, nl) * sz;
+    const size_t sp = (size_t)(nl + 1), sy = 3 * sp, sxo = (size_t)(nj + 1) * sy;
+    const float4 *Ayz = reinterpret_cast<const float4 *>(a.ahat) + (size_t)oy * sy + zmapf(oz, nl);
 #pragma unroll 1
     for (int pol = 0; pol < 2; pol++) {
         const double *E = a.einc + 6 * (rhs0 + pol);
@@ -860,8 +862,8 @@ __global__ void __launch_bounds__(Sp<NI>::RM * TL, k2_min_blocks(NI, Sp<NI>::RM 
 #pragma unroll
                 for (int q = 0; q < R2; q++) {
                     const int kx = 2 * (k1 + R1 * q) + h, mx = kx > NI, ox = mx ? 2 * NI - kx : kx;
-                    const float4 *A = reinterpret_cast<const float4 *>(Ayz + (size_t)ox * sxo);
-                    const float4 a01 = __ldg(A), a23 = __ldg(A + 1), a45 = __ldg(A + 2);
+                    const float4 *A = Ayz + (size_t)ox * sxo;
+                    const float4 a01 = __ldg(A), a23 = __ldg(A + sp), a45 = __ldg(A + 2 * sp);
                     float2 g0 = make_float2(a01.x, a01.y), g1 = make_float2(a01.z, a01.w),
                            g2 = make_float2(a23.x, a23.y), g3 = make_float2(a23.z, a23.w),
                            g4 = make_float2(a45.x, a45.y), g5 = make_float2(a45.z, a45.w);
