@@ -81,6 +81,7 @@ struct ddagpu_ctx {
     int fast = 0;                // compile-time-sized passes in use
     int fx = 0, fyz = 0;         // their launch variants (x pass, y/z passes)
     float2 *ahat = nullptr, *tw = nullptr;
+    float4 *aq = nullptr;        // Green octant in the z order of the compile-time-sized passes
     float2 *work = nullptr, *p = nullptr, *pmin = nullptr, *r = nullptr, *s = nullptr,
            *g = nullptr, *h = nullptr, *w = nullptr;
     RhsState *state = nullptr;
@@ -197,8 +198,8 @@ bool encode_work_maps(ddagpu_ctx *c)
                                dim[0] * dim[1] * dim[2] * 3 * e};
     const cuuint32_t one[5] = {1, 1, 1, 1, 1};
     for (int v = 0; v < 3; v++) {
-        const int tl = matvec_fast_x_tile(c->ni, v);
-        if (tl < 2 || (tl * e) % 16 != 0) return false;
+        const int tl = matvec_fast_x_tile(c->ni, c->nl, v);
+        if (tl == 0) continue;   // rows shorter than the tile: the variant runs the next one
         const cuuint32_t box[5] = {(cuuint32_t)tl, 1, (cuuint32_t)c->ni, 1, 1};
         if (encode(&c->tmaps[v], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, c->work, dim, str, box, one,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -282,6 +283,7 @@ MatvecArgs mv_args(ddagpu_ctx *c, int nrhs, const float2 *src, float2 *out, int 
     a.work = c->work;
     a.wstride = (size_t)3 * c->ni * (2 * c->nj) * (2 * c->nl);
     a.ahat = c->ahat;
+    a.aq = c->aq;
     a.conj = conj;
     a.out = out;
     a.ep.mode = epmode;
@@ -958,7 +960,9 @@ int ddagpu_create(ddagpu_ctx **out, int device, int i_max, int j_max, int l_max,
         if (x != cudaSuccess && e == cudaSuccess) e = x;
     };
     A(dalloc(&c->ahat, ahat_elems(i_max, j_max, l_max)));
-    A(dalloc(&c->tw, (size_t)2 * (i_max + j_max + l_max)));
+    const int zs = matvec_z_split(j_max, l_max);
+    const size_t ntw = (size_t)2 * (i_max + j_max + l_max) + j_max + l_max / zs + (size_t)2 * zs * l_max;
+    A(dalloc(&c->tw, ntw));
     A(dalloc(&c->work, wst * max_rhs));
     A(dalloc(&c->p, n3 * max_rhs));
     A(dalloc(&c->pmin, n3 * max_rhs));
@@ -984,26 +988,51 @@ int ddagpu_create(ddagpu_ctx **out, int device, int i_max, int j_max, int l_max,
     if (e != cudaSuccess)
         return bail(fail(e == cudaErrorMemoryAllocation ? DDAGPU_ENOMEM : DDAGPU_ECUDA,
                          std::string("allocation: ") + cudaGetErrorString(e)));
-    std::vector<float2> tw((size_t)2 * (i_max + j_max + l_max));
-    twiddles(i_max, tw.data());
-    twiddles(j_max, tw.data() + 2 * i_max);
-    twiddles(l_max, tw.data() + 2 * (i_max + j_max));
     c->L.ni = i_max;
     c->L.nj = j_max;
     c->L.nl = l_max;
     c->L.N = c->N;
+    const bool fast = matvec_fast_supported(c->L);
+    if (fast && (e = dalloc(&c->aq, green_order_elems(c->L))) != cudaSuccess)
+        return bail(fail(e == cudaErrorMemoryAllocation ? DDAGPU_ENOMEM : DDAGPU_ECUDA,
+                         std::string("allocation: ") + cudaGetErrorString(e)));
+    std::vector<float2> tw(ntw);
+    twiddles(i_max, tw.data());
+    twiddles(j_max, tw.data() + 2 * i_max);
+    twiddles(l_max, tw.data() + 2 * (i_max + j_max));
+    // the sized y/z passes' tables (Lat::ty, tz, fz)
+    float2 *ty = tw.data() + 2 * (i_max + j_max + l_max), *tz = ty + j_max, *fz = tz + l_max / zs;
+    if (fast) {
+        const double pi = 3.14159265358979323846264338327950288;
+        auto w = [&](long long num, long long den) {   // exp(-2 pi i num / den)
+            const double ph = -2.0 * pi * (double)(num % den) / (double)den;
+            return make_float2((float)std::cos(ph), (float)std::sin(ph));
+        };
+        auto line = [&](int n, float2 *t) {
+            const int r2 = line_r2(n);
+            for (int k = 0; k < n; k++) t[k] = w((long long)(k / r2) * (k % r2), n);
+        };
+        line(j_max, ty);
+        line(l_max / zs, tz);
+        for (int q = 0; q < 2 * zs; q++)
+            for (int l = 0; l < l_max; l++) fz[(size_t)q * l_max + l] = w((long long)q * l, 2 * l_max);
+    }
     c->L.tw_i = c->tw;
     c->L.tw_j = c->tw + 2 * i_max;
     c->L.tw_l = c->tw + 2 * (i_max + j_max);
+    c->L.ty = c->tw + 2 * (i_max + j_max + l_max);
+    c->L.tz = c->L.ty + j_max;
+    c->L.fz = c->L.tz + l_max / zs;
     if ((e = cudaMemcpyAsync(c->tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice,
                              c->st)) != cudaSuccess ||
         (e = matvec_prepare(c->L, c->tile_x, c->rows_g)) != cudaSuccess ||
-        (matvec_fast_supported(c->L) && (e = matvec_fast_prepare(c->L)) != cudaSuccess) ||
+        (fast && (e = matvec_fast_prepare(c->L)) != cudaSuccess) ||
         (e = post_prepare(j_max, l_max)) != cudaSuccess ||
         (e = green_build_octant(i_max, j_max, l_max, kd, c->ahat, c->st)) != cudaSuccess ||
+        (fast && (e = green_order(c->L, c->ahat, c->aq, c->st)) != cudaSuccess) ||
         (e = cudaStreamSynchronize(c->st)) != cudaSuccess)
         return bail(fail(DDAGPU_ECUDA, std::string("setup: ") + cudaGetErrorString(e)));
-    c->fast = matvec_fast_supported(c->L) ? 1 : 0;
+    c->fast = fast ? 1 : 0;
     if (c->fast) c->has_tmap = encode_work_maps(c);
     if (cudaMemset(c->err_dev, 0, sizeof(int)) != cudaSuccess)
         return bail(fail(DDAGPU_ECUDA, "setup: error flag"));
@@ -1023,7 +1052,7 @@ int ddagpu_destroy(ddagpu_ctx *c)
     if (c->graph) cudaGraphDestroy(c->graph);
     if (c->wexec) cudaGraphExecDestroy(c->wexec);
     if (c->wgraph) cudaGraphDestroy(c->wgraph);
-    void *ptrs[] = {c->ahat, c->tw,     c->work,   c->p,       c->pmin,   c->r,     c->s,
+    void *ptrs[] = {c->ahat, c->aq, c->tw,     c->work,   c->p,       c->pmin,   c->r,     c->s,
                     c->w,    c->g,      c->h,      c->state,   c->active, c->trace, c->occ,
                     c->mv,   c->alpha,  c->kinc,   c->einc,    c->ksc,    c->esc_acc,
                     c->cc_acc, c->normals, c->mueller, c->esc, c->cabs,   c->cext,
@@ -1049,6 +1078,7 @@ int ddagpu_set_green(ddagpu_ctx *c, const float *cmA)
     CK(dalloc(&dense, n));
     cudaError_t e = cudaMemcpyAsync(dense, cmA, n * sizeof(float2), cudaMemcpyHostToDevice, c->st);
     if (e == cudaSuccess) e = green_project_dense(c->ni, c->nj, c->nl, dense, c->ahat, c->st);
+    if (e == cudaSuccess && c->aq) e = green_order(c->L, c->ahat, c->aq, c->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
     cudaFree(dense);
     CK(e);

@@ -37,6 +37,9 @@ struct Lat {
     int ni, nj, nl;
     size_t N;               // ni * nj * nl
     const float2 *tw_i, *tw_j, *tw_l;   // [W_n^k, k<n ; W_2n^j, j<n] per axis
+    // sized y/z passes, in their lanes' order (n = R1 R2, matvec_yz.cu): ty[k1 R2 + t2] = W_nj^(t2 k1),
+    // tz the same for the nl / zs points of a z line, fz[s nl + l] = W_2nl^(s l), s < 2 zs
+    const float2 *ty, *tz, *fz;
 };
 
 // Epilogue of the inverse pass: out = sv * v - a_m * conv on active cells, 0 elsewhere;
@@ -61,14 +64,16 @@ struct MatvecArgs {
     float2 *work;           // [nrhs][3][ni][2nj][2nl]
     size_t wstride;
     const float2 *ahat;     // octant Green tensor [ni+1][nj+1][3][nl+1] float4 (two components, z in parity order)
+    const float4 *aq;       // the same in the z order of the sized passes
+    int zs;                 // z split of the sized passes (set by launch_matvec_fast)
     int conj;               // use conj(Ahat)
     float2 *out;            // [nrhs][3][N]
     Epilogue ep;
     const int *rhs_active;  // [nrhs] or null
     int tile_x;             // columns per CTA of the x pass (generic kernels)
     int rows_g;             // rows per staging group of the y/z passes (generic kernels)
-    int fast;               // 1: compile-time-sized kernels of matvec_fast.cu
-    int fx, fyz;            // launch variants of the fast x pass (0..5) and y/z passes (0..2)
+    int fast;               // 1: compile-time-sized kernels (matvec_yz.cu, matvec_x.cu)
+    int fx, fyz;            // launch variants of the fast x pass (0..11) and y/z passes (0..2)
     int *err;               // device flag set by a kernel whose bounded wait gave up (or null)
     const void *tmaps;      // host CUtensorMap[3] of the work buffer (TMA x variants), or null
     int wait_selftest;      // 1: the bulk-copy wait waits (briefly) for a phase that never completes
@@ -99,13 +104,33 @@ size_t matvec_smem_yz(const Lat &L, int rows_g);
 size_t matvec_smem_x(const Lat &L, int tile_x);
 cudaError_t matvec_prepare(const Lat &L, int tile_x, int rows_g);
 
-// compile-time-sized passes for edges in {16, 32, 64} (matvec_fast.cu)
+// compile-time-sized passes for edges 4..128 (matvec_fast.cu: dispatch; matvec_x.cu, matvec_yz.cu)
 bool matvec_fast_supported(const Lat &L);
 constexpr int kXVariants = 12;     // launch variants of the fast x pass (9..11: TMA tensor tiles)
 constexpr int kYZVariants = 3;     // launch variants of the fast y/z passes
 cudaError_t matvec_fast_prepare(const Lat &L);
-int matvec_fast_x_tile(int ni, int x_variant);   // spectral columns per CTA of an x variant
+int matvec_fast_x_tile(int ni, int nl, int x_variant);   // spectral columns per CTA, 0: row too short
 cudaError_t launch_matvec_fast(const MatvecArgs &a, cudaStream_t st);
+size_t green_order_elems(const Lat &L);   // float4 elements of MatvecArgs::aq
+cudaError_t green_order(const Lat &L, const float2 *ahat, float4 *out, cudaStream_t st);
+// CTAs per plane of the y/z passes: at most 4096 pairs (64 KB of shared memory) each
+__host__ __device__ constexpr int matvec_z_split(int nj, int nl) { return nj * nl <= 4096 ? 1 : nj * nl <= 8192 ? 2 : 4; }
+// per edge, one object each (Makefile)
+template <int NJ> cudaError_t yz_prepare(int nl);
+template <int NJ> cudaError_t yz_launch(const MatvecArgs &a, int fwd, cudaStream_t st);
+template <int NI> cudaError_t x_prepare();
+template <int NI> cudaError_t x_launch(const MatvecArgs &a, cudaStream_t st);
+#define DDA_EDGES(F) F(4) F(8) F(16) F(32) F(64) F(128)
+#define DDA_DECLARE(N)                                                                        \
+    template <> cudaError_t yz_prepare<N>(int nl);                                            \
+    template <> cudaError_t yz_launch<N>(const MatvecArgs &a, int fwd, cudaStream_t st);      \
+    template <> cudaError_t x_prepare<N>();                                                   \
+    template <> cudaError_t x_launch<N>(const MatvecArgs &a, cudaStream_t st);
+DDA_EDGES(DDA_DECLARE)
+#undef DDA_DECLARE
+
+// smaller factor R2 of an edge's line split (pair.cuh line_split)
+constexpr int line_r2(int n) { return n <= 8 ? 2 : n <= 32 ? 4 : 8; }
 
 // Green tensor (green.cu)
 cudaError_t green_build_octant(int ni, int nj, int nl, double kd, float2 *ahat, cudaStream_t st);
