@@ -149,8 +149,8 @@ struct ddagpu_ctx {
     double *kz_val = nullptr;
     float2 *kz_sum = nullptr;
     size_t kz_tab_cap = 0, kz_val_cap = 0, kz_sum_cap = 0;
-    // TMA tensor maps of the work buffer, one per x-pass column tile (x variants 9..11)
-    alignas(64) CUtensorMap tmaps[3];
+    // TMA tensor map of the work buffer, one column tile of the x pass (x variants 9..11)
+    alignas(64) CUtensorMap tmap;
     bool has_tmap = false;
     Fp64Buffers *f64 = nullptr;  // FP64 solve buffers (ddagpu_solve_fp64), built on first use
     MixedCgBuffers *mcg = nullptr;   // FP64 fields of the mixed-precision CG refinement
@@ -176,9 +176,9 @@ struct DevGuard {
     }
 };
 
-// The work buffer [cap][3][ni][2nj][2nl] complex float as a 5-D tensor map per x-pass
-// column tile (box TL x 1 x ni x 1 x 1, 8-byte elements, no swizzle, no multicast), for the
-// TMA variants of the x pass.  false if the driver does not offer the encoder.
+// The work buffer [cap][3][ni][2nj][2nl] complex float as a 5-D tensor map (box 16 columns x
+// 1 x ni x 1 x 1, 8-byte elements, no swizzle, no multicast), for the TMA variants of the x
+// pass.  false if the driver does not offer the encoder or the rows are shorter.
 bool encode_work_maps(ddagpu_ctx *c)
 {
     typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -197,15 +197,13 @@ bool encode_work_maps(ddagpu_ctx *c)
     const cuuint64_t str[4] = {dim[0] * e, dim[0] * dim[1] * e, dim[0] * dim[1] * dim[2] * e,
                                dim[0] * dim[1] * dim[2] * 3 * e};
     const cuuint32_t one[5] = {1, 1, 1, 1, 1};
-    for (int v = 0; v < 3; v++) {
-        const int tl = matvec_fast_x_tile(c->ni, c->nl, v);
-        if (tl == 0) continue;   // rows shorter than the tile: the variant runs the next one
-        const cuuint32_t box[5] = {(cuuint32_t)tl, 1, (cuuint32_t)c->ni, 1, 1};
-        if (encode(&c->tmaps[v], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, c->work, dim, str, box, one,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return false;
-    }
+    const int tl = matvec_fast_x_tile(c->nl);
+    if (!tl) return false;
+    const cuuint32_t box[5] = {(cuuint32_t)tl, 1, (cuuint32_t)c->ni, 1, 1};
+    if (encode(&c->tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, c->work, dim, str, box, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
     return true;
 }
 
@@ -303,7 +301,7 @@ MatvecArgs mv_args(ddagpu_ctx *c, int nrhs, const float2 *src, float2 *out, int 
     a.fyz = c->fyz;
     a.err = c->err_dev;
     a.wait_selftest = c->wait_selftest;
-    a.tmaps = c->has_tmap ? (const void *)c->tmaps : nullptr;
+    a.tmaps = c->has_tmap ? (const void *)&c->tmap : nullptr;
     return a;
 }
 
@@ -1033,7 +1031,10 @@ int ddagpu_create(ddagpu_ctx **out, int device, int i_max, int j_max, int l_max,
         (e = cudaStreamSynchronize(c->st)) != cudaSuccess)
         return bail(fail(DDAGPU_ECUDA, std::string("setup: ") + cudaGetErrorString(e)));
     c->fast = fast ? 1 : 0;
-    if (c->fast) c->has_tmap = encode_work_maps(c);
+    if (c->fast) {
+        c->has_tmap = encode_work_maps(c);
+        matvec_fast_defaults(c->L, c->has_tmap, &c->fx, &c->fyz);
+    }
     if (cudaMemset(c->err_dev, 0, sizeof(int)) != cudaSuccess)
         return bail(fail(DDAGPU_ECUDA, "setup: error flag"));
     *out = c;
@@ -1111,7 +1112,7 @@ int ddagpu_set_kernels(ddagpu_ctx *c, int fast)
 {
     if (!c) return fail(DDAGPU_EINVAL, "null context");
     if (fast && !matvec_fast_supported(c->L))
-        return fail(DDAGPU_EINVAL, "compile-time-sized passes need edges in {16, 32, 64, 128}");
+        return fail(DDAGPU_EINVAL, "compile-time-sized passes need edges of 4 at least");
     c->fast = fast ? 1 : 0;
     return DDAGPU_OK;
 }
@@ -1182,8 +1183,13 @@ int ddagpu_autotune(ddagpu_ctx *c, int nrhs)
     if (matvec_fast_supported(c->L)) {
         // the compile-time-sized passes in each launch variant
         c->fast = 1;
-        for (int vx = 0; vx < (c->has_tmap ? kXVariants : 9); vx++)
-            for (int vyz = 0; vyz < kYZVariants; vyz++) {
+        // (the x variants that differ: three tiles of the unpacked form at edge 64, then the
+        // packed form's three ways of loading)
+        std::vector<int> vxs = {3, 6};
+        if (c->ni == 64) vxs.insert(vxs.begin(), {0, 1, 2});
+        if (c->has_tmap) vxs.push_back(9);
+        for (int vx : vxs)
+            for (int vyz = 0; vyz < 2; vyz++) {   // (2 is 0)
                 c->fx = vx;
                 c->fyz = vyz;
                 float ms = 0;
@@ -1211,12 +1217,12 @@ int ddagpu_autotune(ddagpu_ctx *c, int nrhs)
 
 namespace {
 // A host field of cvectors [N][3] into [3][N] on the device: copied as it is (through c->w,
-// idle between solves) and transposed there, not on the host.
+// idle between solves) and transposed there, not on the host (part of the copy: not counted
+// among the context's kernels).
 int upload_field(ddagpu_ctx *c, const float *p, float2 *dst)
 {
     CK(cudaMemcpyAsync(c->w, p, 3 * c->N * sizeof(float2), cudaMemcpyHostToDevice, c->st));
     CK(field_to_soa(c->w, dst, c->N, c->st));
-    c->launches += 1;
     return DDAGPU_OK;
 }
 }  // namespace
@@ -1814,7 +1820,6 @@ int ddagpu_solve_linear(ddagpu_ctx *c, int solver, float rTau, const float *cLis
         ri.err_history[0] = ri.err;
     }
     CK(field_to_aos(c->p, c->w, c->N, c->st));
-    c->launches += 1;
     CK(cudaMemcpyAsync(x_out, c->w, n3 * sizeof(float2), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     if (info) *info = ri;

@@ -75,7 +75,7 @@ struct MatvecArgs {
     int fast;               // 1: compile-time-sized kernels (matvec_yz.cu, matvec_x.cu)
     int fx, fyz;            // launch variants of the fast x pass (0..11) and y/z passes (0..2)
     int *err;               // device flag set by a kernel whose bounded wait gave up (or null)
-    const void *tmaps;      // host CUtensorMap[3] of the work buffer (TMA x variants), or null
+    const void *tmaps;      // host CUtensorMap of the work buffer (TMA x variants), or null
     int wait_selftest;      // 1: the bulk-copy wait waits (briefly) for a phase that never completes
     // step 0 from the incident field (compile-time-sized passes only): the forward y/z pass
     // computes its input p = alpha_m exp(i k.(r - c)) E_inc on active cells (0 elsewhere)
@@ -109,7 +109,8 @@ bool matvec_fast_supported(const Lat &L);
 constexpr int kXVariants = 12;     // launch variants of the fast x pass (9..11: TMA tensor tiles)
 constexpr int kYZVariants = 3;     // launch variants of the fast y/z passes
 cudaError_t matvec_fast_prepare(const Lat &L);
-int matvec_fast_x_tile(int ni, int nl, int x_variant);   // spectral columns per CTA, 0: row too short
+int matvec_fast_x_tile(int nl);           // spectral columns per TMA tile, 0: row too short
+void matvec_fast_defaults(const Lat &L, bool has_tmap, int *fx, int *fyz);   // untuned launch variants
 cudaError_t launch_matvec_fast(const MatvecArgs &a, cudaStream_t st);
 size_t green_order_elems(const Lat &L);   // float4 elements of MatvecArgs::aq
 cudaError_t green_order(const Lat &L, const float2 *ahat, float4 *out, cudaStream_t st);

@@ -11,25 +11,21 @@ bool fast_edge(int n) { return n >= 4 && n <= 128 && (n & (n - 1)) == 0; }
 
 // Green octant [ni+1][nj+1][3][nl+1] float4 (z in parity order) -> the z order of the rows
 __global__ void __launch_bounds__(256) order_green(const float4 *__restrict__ oct, float4 *__restrict__ out, int nl,
-                                                   int zs, size_t n)
+                                                   int zs, int split, size_t n)
 {
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (q >= n) return;
     const int oz = (int)(q % (nl + 1)), z = (oz & 1) ? (nl / 2 + 1 + (oz >> 1)) : (oz >> 1);
     const size_t row = q / (nl + 1);
-    out[row * z_entries(nl, zs) + z_order(oz, nl, zs)] = oct[row * (nl + 1) + z];
+    out[row * z_entries(nl, zs) + z_order(oz, nl, zs, split)] = oct[row * (nl + 1) + z];
 }
 
 }  // namespace
 
 bool matvec_fast_supported(const Lat &L) { return fast_edge(L.ni) && fast_edge(L.nj) && fast_edge(L.nl); }
 
-// spectral columns per CTA of an x variant; 0 where the rows are shorter
-int matvec_fast_x_tile(int ni, int nl, int v)
-{
-    const int t = (ni <= 64 ? 32 : 16) >> (v % 3);
-    return t <= 2 * nl ? t : 0;
-}
+// spectral columns per TMA tile of the x pass; 0 where the rows are shorter
+int matvec_fast_x_tile(int nl) { return nl >= 8 ? 16 : 0; }
 
 size_t green_order_elems(const Lat &L)
 {
@@ -40,8 +36,14 @@ cudaError_t green_order(const Lat &L, const float2 *ahat, float4 *out, cudaStrea
 {
     const size_t n = (size_t)(L.ni + 1) * (L.nj + 1) * 3 * (L.nl + 1);
     order_green<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4 *>(ahat), out, L.nl,
-                                                             matvec_z_split(L.nj, L.nl), n);
+                                                             matvec_z_split(L.nj, L.nl), z_parity_split(L.ni), n);
     return cudaGetLastError();
+}
+
+void matvec_fast_defaults(const Lat &L, bool has_tmap, int *fx, int *fyz)
+{
+    *fx = L.ni == 64 ? 1 : has_tmap ? 9 : 6;
+    *fyz = (long long)L.nj * L.nl <= 1024 ? 1 : 0;
 }
 
 cudaError_t matvec_fast_prepare(const Lat &L)
@@ -73,7 +75,7 @@ static cudaError_t yz(const MatvecArgs &a, int fwd, cudaStream_t st)
 
 cudaError_t launch_matvec_fast(const MatvecArgs &args, cudaStream_t st)
 {
-    if (args.fx >= 9 && !args.tmaps) return cudaErrorInvalidValue;   // no tensor maps for the TMA variants
+    if (args.fx >= 9 && args.L.nl >= 8 && !args.tmaps) return cudaErrorInvalidValue;   // no tensor maps for the TMA variants
     MatvecArgs a = args;
     a.zs = matvec_z_split(a.L.nj, a.L.nl);
     cudaError_t e = yz(a, 1, st);

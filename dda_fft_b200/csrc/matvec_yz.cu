@@ -69,10 +69,6 @@ struct Yz {
     }
 };
 
-// a pair as two columns of the work buffer
-DDA_DEV float4 columns_of(P2 p) { return make_float4(p.r.x, p.i.x, p.r.y, p.i.y); }
-DDA_DEV P2 of_columns(float4 q) { return {make_float2(q.x, q.z), make_float2(q.y, q.w)}; }
-
 // One row's inputs x[b][rr] (element t2 + R2 rr + ML b) -> the pair line of rank r, v[rr]
 // (element t2 + R2 rr of ML): bins s = 2 r, 2 r + 1 (mod 2 ZS), v_s = W^(s l') sum_b W^(s ML b) x_b.
 template <int NL, int ZS, int R1, int R2>
@@ -570,7 +566,7 @@ __global__ void __launch_bounds__(NT, Yz<NJ, NL, NT, MB>::MINB) k3p(MatvecArgs a
 
 // block sizes of the launch variants
 constexpr int yz_threads(int v) { return v == 1 ? 128 : 256; }
-constexpr int yz_blocks(int v) { return v == 1 ? 4 : v == 2 ? 3 : 2; }
+constexpr int yz_blocks(int v) { return v == 1 ? 4 : 2; }   // per SM where shared memory allows
 
 template <int NJ, int NL, int V>
 cudaError_t launch_yz_v(const MatvecArgs &a, int fwd, cudaStream_t st)
@@ -631,9 +627,8 @@ cudaError_t yz_prepare<YZ_NJ>(int nl)
 {
     return with_nl(nl, [](auto l) {
         constexpr int NL = decltype(l)::value;
-        cudaError_t e = prep_yz_v<YZ_NJ, NL, 0>();
-        if (e == cudaSuccess) e = prep_yz_v<YZ_NJ, NL, 1>();
-        return e == cudaSuccess ? prep_yz_v<YZ_NJ, NL, 2>() : e;
+        const cudaError_t e = prep_yz_v<YZ_NJ, NL, 0>();
+        return e == cudaSuccess ? prep_yz_v<YZ_NJ, NL, 1>() : e;
     });
 }
 
@@ -642,9 +637,7 @@ cudaError_t yz_launch<YZ_NJ>(const MatvecArgs &a, int fwd, cudaStream_t st)
 {
     return with_nl(a.L.nl, [&](auto l) {
         constexpr int NL = decltype(l)::value;
-        return a.fyz == 1 ? launch_yz_v<YZ_NJ, NL, 1>(a, fwd, st)
-             : a.fyz == 2 ? launch_yz_v<YZ_NJ, NL, 2>(a, fwd, st)
-                          : launch_yz_v<YZ_NJ, NL, 0>(a, fwd, st);
+        return a.fyz == 1 ? launch_yz_v<YZ_NJ, NL, 1>(a, fwd, st) : launch_yz_v<YZ_NJ, NL, 0>(a, fwd, st);
     });
 }
 

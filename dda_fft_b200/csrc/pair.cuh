@@ -42,6 +42,10 @@ DDA_DEV float2 psecond(P2 p) { return make_float2(p.r.y, p.i.y); }
 DDA_DEV P2 p_of(float4 q) { return {make_float2(q.x, q.y), make_float2(q.z, q.w)}; }
 DDA_DEV float4 f4_of(P2 p) { return make_float4(p.r.x, p.r.y, p.i.x, p.i.y); }
 
+// a pair as two columns of the work buffer
+DDA_DEV float4 columns_of(P2 p) { return make_float4(p.r.x, p.i.x, p.r.y, p.i.y); }
+DDA_DEV P2 of_columns(float4 q) { return {make_float2(q.x, q.z), make_float2(q.y, q.w)}; }
+
 // a -+ i b: the times -i (forward) or +i (inverse) of a butterfly as a choice of add and sub
 template <bool INV>
 DDA_DEV P2 padd_rot(P2 a, P2 b)   // a + (INV ? i : -i) b

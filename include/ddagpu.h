@@ -259,16 +259,14 @@ int ddagpu_anthrax_place(unsigned long long *rng_state, int i_max, float monomer
 int ddagpu_anthrax_rasterize(int device, int i_max, int j_max, int l_max, const float *monomers,
                              int count, signed char *occ, int *ndip);
 
-/* Launch variants of the compile-time-sized matvec passes (edges 16..128): x_variant
- * 0/1/2 = 32, 16 or 8 spectral columns per x-pass CTA (16, 8, 4 at edge 128), 3/4/5 = the
- * same with the input rows moved into shared memory by bulk asynchronous copies, 6/7/8 =
- * the same tiles with the x lines' second factorisation (16 = 8 x 2, 32 = 4 x 8,
- * 64 = 16 x 4, 128 = 8 x 16 instead of 4 x 4, 8 x 4, 8 x 8, 16 x 8: the radix schedule),
- * 9/10/11 = the tiles of 0/1/2 moved into shared memory as one TMA tensor tile per
- * component (cp.async.bulk.tensor over a tensor map of the work buffer; offered where the
- * driver provides the encoder);
- * yz_variant 0/1/2 = the default block size of the y/z passes, the other of 256 / 512, or
- * 128 threads.
+/* Launch variants of the compile-time-sized matvec passes (edges 4..128).  x_variant 0/1/2 =
+ * the unpacked x pass with 32, 16 or 8 spectral columns per CTA (edge 64; at other edges the
+ * packed pass with register loads), 3/4/5 = the packed x pass (pairs of z bins, packed FP32)
+ * with its input rows moved into shared memory by bulk asynchronous copies, 6/7/8 = with
+ * register loads, 9/10/11 = with one TMA tensor tile per component (cp.async.bulk.tensor over
+ * a tensor map of the work buffer; offered where the driver provides the encoder and l_max is
+ * at least 8); yz_variant 0 / 1 / 2 = 256, 128 or 256 threads per CTA of the y/z passes.
+ * A new context starts with the variants measured fastest at its edges.
  * ddagpu_autotune times every combination (and the generic passes) and keeps the
  * fastest.  No counterpart in the reference. */
 int ddagpu_set_fast_variant(ddagpu_ctx *ctx, int x_variant, int yz_variant);
@@ -293,8 +291,8 @@ int ddagpu_farfield_plan(const double *ksc, int nrhs, int ndir, int pairs, int n
                          double nact, int mode, int *groups, int *items);
 int ddagpu_get_fast_variant(ddagpu_ctx *ctx, int *x_variant, int *yz_variant);
 
-/* Self-test of the bounded device waits: on != 0 makes the bulk-copy x-pass variants
- * (ddagpu_set_fast_variant x 3..5) wait briefly for a barrier phase that nothing completes,
+/* Self-test of the bounded device waits: on != 0 makes the x-pass variants fed by
+ * asynchronous copies (ddagpu_set_fast_variant x 3..5, 9..11) wait briefly for a barrier phase that nothing completes,
  * so that the wait runs out; the call then fails with DDAGPU_ECUDA ("a device wait ran
  * out") and the context stays usable once the self-test is switched off.  Diagnostic
  * only; no counterpart in the reference. */
@@ -382,8 +380,8 @@ long long ddagpu_kernel_launches(ddagpu_ctx *ctx);
  * the fastest. */
 int ddagpu_set_tiling(ddagpu_ctx *ctx, int tile_x, int rows_g);
 int ddagpu_get_tiling(ddagpu_ctx *ctx, int *tile_x, int *rows_g);
-/* Kernel family of the matvec: 1 = passes specialised at compile time for lattice edges in
- * {16, 32, 64, 128} (the default where they apply), 0 = the generic passes (any edge 2..128). */
+/* Kernel family of the matvec: 1 = passes specialised at compile time for lattice edges
+ * 4..128 (the default where they apply), 0 = the generic passes (any edge 2..128). */
 int ddagpu_set_kernels(ddagpu_ctx *ctx, int fast);
 int ddagpu_get_kernels(ddagpu_ctx *ctx);
 int ddagpu_autotune(ddagpu_ctx *ctx, int nrhs);
