@@ -80,8 +80,8 @@ struct ddagpu_ctx {
     int tile_x = 32, rows_g = 16;
     int fast = 0;                // compile-time-sized passes in use
     int fx = 0, fyz = 0;         // their launch variants (x pass, y/z passes)
-    float2 *ahat = nullptr, *tw = nullptr;
-    float4 *aq = nullptr;        // Green octant in the z order of the compile-time-sized passes
+    float4 *ahat = nullptr;
+    float2 *tw = nullptr;
     float2 *work = nullptr, *p = nullptr, *pmin = nullptr, *r = nullptr, *s = nullptr,
            *g = nullptr, *h = nullptr, *w = nullptr;
     RhsState *state = nullptr;
@@ -281,7 +281,6 @@ MatvecArgs mv_args(ddagpu_ctx *c, int nrhs, const float2 *src, float2 *out, int 
     a.work = c->work;
     a.wstride = (size_t)3 * c->ni * (2 * c->nj) * (2 * c->nl);
     a.ahat = c->ahat;
-    a.aq = c->aq;
     a.conj = conj;
     a.out = out;
     a.ep.mode = epmode;
@@ -991,9 +990,6 @@ int ddagpu_create(ddagpu_ctx **out, int device, int i_max, int j_max, int l_max,
     c->L.nl = l_max;
     c->L.N = c->N;
     const bool fast = matvec_fast_supported(c->L);
-    if (fast && (e = dalloc(&c->aq, green_order_elems(c->L))) != cudaSuccess)
-        return bail(fail(e == cudaErrorMemoryAllocation ? DDAGPU_ENOMEM : DDAGPU_ECUDA,
-                         std::string("allocation: ") + cudaGetErrorString(e)));
     std::vector<float2> tw(ntw);
     twiddles(i_max, tw.data());
     twiddles(j_max, tw.data() + 2 * i_max);
@@ -1027,7 +1023,6 @@ int ddagpu_create(ddagpu_ctx **out, int device, int i_max, int j_max, int l_max,
         (fast && (e = matvec_fast_prepare(c->L)) != cudaSuccess) ||
         (e = post_prepare(j_max, l_max)) != cudaSuccess ||
         (e = green_build_octant(i_max, j_max, l_max, kd, c->ahat, c->st)) != cudaSuccess ||
-        (fast && (e = green_order(c->L, c->ahat, c->aq, c->st)) != cudaSuccess) ||
         (e = cudaStreamSynchronize(c->st)) != cudaSuccess)
         return bail(fail(DDAGPU_ECUDA, std::string("setup: ") + cudaGetErrorString(e)));
     c->fast = fast ? 1 : 0;
@@ -1053,7 +1048,7 @@ int ddagpu_destroy(ddagpu_ctx *c)
     if (c->graph) cudaGraphDestroy(c->graph);
     if (c->wexec) cudaGraphExecDestroy(c->wexec);
     if (c->wgraph) cudaGraphDestroy(c->wgraph);
-    void *ptrs[] = {c->ahat, c->aq, c->tw,     c->work,   c->p,       c->pmin,   c->r,     c->s,
+    void *ptrs[] = {c->ahat, c->tw,     c->work,   c->p,       c->pmin,   c->r,     c->s,
                     c->w,    c->g,      c->h,      c->state,   c->active, c->trace, c->occ,
                     c->mv,   c->alpha,  c->kinc,   c->einc,    c->ksc,    c->esc_acc,
                     c->cc_acc, c->normals, c->mueller, c->esc, c->cabs,   c->cext,
@@ -1079,7 +1074,6 @@ int ddagpu_set_green(ddagpu_ctx *c, const float *cmA)
     CK(dalloc(&dense, n));
     cudaError_t e = cudaMemcpyAsync(dense, cmA, n * sizeof(float2), cudaMemcpyHostToDevice, c->st);
     if (e == cudaSuccess) e = green_project_dense(c->ni, c->nj, c->nl, dense, c->ahat, c->st);
-    if (e == cudaSuccess && c->aq) e = green_order(c->L, c->ahat, c->aq, c->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
     cudaFree(dense);
     CK(e);

@@ -9,10 +9,11 @@
 //   even axis:  sum_x f(x) e^{-i pi k x / n} = f(0) + 2 sum_{0<x<n} f(x) cos(pi k x / n)
 //   odd axis:                                  -2i sum_{0<x<n} f(x) sin(pi k x / n)
 // The three axis sums run in FP64 here; the octant is stored in float as
-// Ahat[kx][ky][zmap(kz)][comp], z in parity order (even kz first, then odd kz), so the six
-// components of one frequency form one 48-byte entry.
+// Ahat[kx][ky][3][z_order(kz)], two components per float4, z in the order of the x pass's columns
+// (zorder.cuh), so that neighbouring lanes read runs of consecutive entries.
 #include "common.cuh"
 #include "internal.h"
+#include "zorder.cuh"
 
 namespace ddagpu {
 
@@ -89,11 +90,17 @@ __global__ void axis_sum(const double2 *in, double2 *out, int A6, int nt, int B,
     out[q] = odd ? make_double2(si, -sr) : make_double2(sr, si);
 }
 
-__device__ inline int zmapd(int oz, int nl) { return (oz & 1) ? (nl / 2 + 1 + (oz >> 1)) : (oz >> 1); }
-
-__global__ void to_octant(const double2 *in, float2 *ahat, int ni, int nj, int nl)
+// place of component c of bin (xy, oz) in the octant [ni+1][nj+1][3][z_entries] float4, as floats
+__device__ inline float2 *octant_at(float4 *ahat, size_t xy, int oz, int c, int ni, int nj, int nl)
 {
-    // in[comp][kx][ky][kz] -> ahat[kx][ky][comp / 2][zmap(kz)][comp % 2]
+    const int zs = matvec_z_split(nj, nl);
+    const size_t e = (xy * 3 + c / 2) * z_entries(nl, zs) + z_order(oz, nl, zs, z_parity_split(ni));
+    return reinterpret_cast<float2 *>(ahat + e) + c % 2;
+}
+
+__global__ void to_octant(const double2 *in, float4 *ahat, int ni, int nj, int nl)
+{
+    // in[comp][kx][ky][kz] -> the octant in the passes' z order
     const size_t per = (size_t)(ni + 1) * (nj + 1) * (nl + 1);
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (q >= 6 * per) return;
@@ -101,13 +108,13 @@ __global__ void to_octant(const double2 *in, float2 *ahat, int ni, int nj, int n
     const size_t xy = (q / (nl + 1)) % ((size_t)(ni + 1) * (nj + 1));
     const int comp = (int)(q / per);
     const double2 v = in[q];
-    ahat[((xy * 3 + comp / 2) * (nl + 1) + zmapd(oz, nl)) * 2 + comp % 2] = make_float2((float)v.x, (float)v.y);
+    *octant_at(ahat, xy, oz, comp, ni, nj, nl) = make_float2((float)v.x, (float)v.y);
 }
 
 // Octant from a dense float Ahat [2ni][2nj][2nl][6] (the reference's cmA layout): the
 // average of the 8 mirror images with the parity signs, which removes the index-n plane
 // contributions and keeps everything else.
-__global__ void project_dense(const float2 *dense, float2 *ahat, int ni, int nj, int nl)
+__global__ void project_dense(const float2 *dense, float4 *ahat, int ni, int nj, int nl)
 {
     const size_t per = (size_t)(ni + 1) * (nj + 1) * (nl + 1);
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -130,24 +137,29 @@ __global__ void project_dense(const float2 *dense, float2 *ahat, int ni, int nj,
         sr += s * v.x;
         si += s * v.y;
     }
-    ahat[((((size_t)ox * (nj + 1) + oy) * 3 + c / 2) * (nl + 1) + zmapd(oz, nl)) * 2 + c % 2] =
-        make_float2((float)(sr / 8.0), (float)(si / 8.0));
+    *octant_at(ahat, (size_t)ox * (nj + 1) + oy, oz, c, ni, nj, nl) = make_float2((float)(sr / 8.0), (float)(si / 8.0));
 }
+
+// components x bins of the octant
+inline size_t octant_elems(int ni, int nj, int nl) { return (size_t)6 * (ni + 1) * (nj + 1) * (nl + 1); }
 
 inline unsigned blocks(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
 
-size_t ahat_elems(int ni, int nj, int nl) { return (size_t)6 * (ni + 1) * (nj + 1) * (nl + 1); }
+size_t ahat_elems(int ni, int nj, int nl)
+{
+    return (size_t)3 * (ni + 1) * (nj + 1) * z_entries(nl, matvec_z_split(nj, nl));
+}
 
 namespace {
 
 // The octant in FP64 into b1 as [comp][kx][ky][kz] (natural kz order); b0 and tab are
-// scratch of ahat_elems and 6 (nmax + 1) nmax doubles.
+// scratch of octant_elems and 6 (nmax + 1) nmax doubles.
 void octant_fp64(int ni, int nj, int nl, double kd, double2 *b0, double2 *b1, double *tab,
                  size_t tabn, cudaStream_t st)
 {
-    const size_t big = ahat_elems(ni, nj, nl);
+    const size_t big = octant_elems(ni, nj, nl);
     double *ct[3], *stb[3];
     const int ns[3] = {ni, nj, nl};
     for (int a = 0; a < 3; a++) {
@@ -175,9 +187,9 @@ size_t trig_elems(int ni, int nj, int nl)
 
 }  // namespace
 
-cudaError_t green_build_octant(int ni, int nj, int nl, double kd, float2 *ahat, cudaStream_t st)
+cudaError_t green_build_octant(int ni, int nj, int nl, double kd, float4 *ahat, cudaStream_t st)
 {
-    const size_t big = ahat_elems(ni, nj, nl), tabn = trig_elems(ni, nj, nl);
+    const size_t big = octant_elems(ni, nj, nl), tabn = trig_elems(ni, nj, nl);
     double2 *b0 = nullptr, *b1 = nullptr;
     double *tab = nullptr;
     cudaError_t e;
@@ -194,7 +206,7 @@ cudaError_t green_build_octant(int ni, int nj, int nl, double kd, float2 *ahat, 
 
 cudaError_t green_build_octant64(int ni, int nj, int nl, double kd, double2 *out, cudaStream_t st)
 {
-    const size_t big = ahat_elems(ni, nj, nl), tabn = trig_elems(ni, nj, nl);
+    const size_t big = octant_elems(ni, nj, nl), tabn = trig_elems(ni, nj, nl);
     double2 *b0 = nullptr;
     double *tab = nullptr;
     cudaError_t e;
@@ -206,10 +218,10 @@ cudaError_t green_build_octant64(int ni, int nj, int nl, double kd, double2 *out
     return cudaGetLastError();
 }
 
-cudaError_t green_project_dense(int ni, int nj, int nl, const float2 *dense_dev, float2 *ahat,
+cudaError_t green_project_dense(int ni, int nj, int nl, const float2 *dense_dev, float4 *ahat,
                                 cudaStream_t st)
 {
-    const size_t big = ahat_elems(ni, nj, nl);
+    const size_t big = octant_elems(ni, nj, nl);
     project_dense<<<blocks(big, 256), 256, 0, st>>>(dense_dev, ahat, ni, nj, nl);
     return cudaGetLastError();
 }

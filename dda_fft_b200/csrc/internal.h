@@ -63,8 +63,7 @@ struct MatvecArgs {
     size_t fstride;         // 3 N
     float2 *work;           // [nrhs][3][ni][2nj][2nl]
     size_t wstride;
-    const float2 *ahat;     // octant Green tensor [ni+1][nj+1][3][nl+1] float4 (two components, z in parity order)
-    const float4 *aq;       // the same in the z order of the sized passes
+    const float4 *ahat;     // octant Green tensor [ni+1][nj+1][3][z_entries], two components each (zorder.cuh)
     int zs;                 // z split of the sized passes (set by launch_matvec_fast)
     int conj;               // use conj(Ahat)
     float2 *out;            // [nrhs][3][N]
@@ -112,10 +111,11 @@ cudaError_t matvec_fast_prepare(const Lat &L);
 int matvec_fast_x_tile(int nl);           // spectral columns per TMA tile, 0: row too short
 void matvec_fast_defaults(const Lat &L, bool has_tmap, int *fx, int *fyz);   // untuned launch variants
 cudaError_t launch_matvec_fast(const MatvecArgs &a, cudaStream_t st);
-size_t green_order_elems(const Lat &L);   // float4 elements of MatvecArgs::aq
-cudaError_t green_order(const Lat &L, const float2 *ahat, float4 *out, cudaStream_t st);
 // CTAs per plane of the y/z passes: at most 4096 pairs (64 KB of shared memory) each
 __host__ __device__ constexpr int matvec_z_split(int nj, int nl) { return nj * nl <= 4096 ? 1 : nj * nl <= 8192 ? 2 : 4; }
+// dynamic shared memory of a matvec kernel; the carveout stays the driver's choice (the largest
+// one cost 15%: what the passes leave, L1 uses for the Green tensor, twiddles and row sectors)
+cudaError_t matvec_kernel_smem(const void *kernel, int bytes);
 // per edge, one object each (Makefile)
 template <int NJ> cudaError_t yz_prepare(int nl);
 template <int NJ> cudaError_t yz_launch(const MatvecArgs &a, int fwd, cudaStream_t st);
@@ -134,9 +134,9 @@ DDA_EDGES(DDA_DECLARE)
 constexpr int line_r2(int n) { return n <= 8 ? 2 : n <= 32 ? 4 : 8; }
 
 // Green tensor (green.cu)
-cudaError_t green_build_octant(int ni, int nj, int nl, double kd, float2 *ahat, cudaStream_t st);
-cudaError_t green_project_dense(int ni, int nj, int nl, const float2 *dense_dev, float2 *ahat,
+cudaError_t green_build_octant(int ni, int nj, int nl, double kd, float4 *ahat, cudaStream_t st);
+cudaError_t green_project_dense(int ni, int nj, int nl, const float2 *dense_dev, float4 *ahat,
                                 cudaStream_t st);
-size_t ahat_elems(int ni, int nj, int nl);
+size_t ahat_elems(int ni, int nj, int nl);   // float4
 
 }  // namespace ddagpu

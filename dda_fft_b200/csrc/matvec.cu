@@ -21,14 +21,13 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "zorder.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace ddagpu {
 
 namespace {
-
-DDA_DEV int zmap(int oz, int nl) { return (oz & 1) ? (nl / 2 + 1 + (oz >> 1)) : (oz >> 1); }
 
 // ------------------------------------------------------------------------------ K1
 // src plane (nj x nl, component c, lattice plane i) -> work rows j_s = h nj + kj, each
@@ -101,14 +100,15 @@ __global__ void __launch_bounds__(512) k2_x_product(MatvecArgs a)
     // Symmetric 3x3 product with the Green tensor at frequency (kx, j', l').
     const int hj = js >= nj, kj = js - hj * nj, jp = 2 * kj + hj;
     const int my = jp > nj, oy = my ? 2 * nj - jp : jp;
-    // Ahat[ox][oy][3][zmap(oz)], two components per float4
-    const size_t sp = (size_t)(nl + 1), sy = 3 * sp, sxo = (size_t)(nj + 1) * sy;
+    // Ahat[ox][oy][3][z_order(oz)], two components per float4
+    const int zs = matvec_z_split(nj, nl);
+    const size_t sp = z_entries(nl, zs), sy = 3 * sp, sxo = (size_t)(nj + 1) * sy;
     for (int e = threadIdx.x; e < 2 * ni * TW; e += blockDim.x) {
         const int t = e % TW, kh = e / TW, k = kh >> 1, hx = kh & 1;
         const int kx = 2 * k + hx, mx = kx > ni, ox = mx ? 2 * ni - kx : kx;
         const int ls = l0 + t, hl = ls >= nl, kl = ls - hl * nl, lp = 2 * kl + hl;
         const int mz = lp > nl, oz = mz ? 2 * nl - lp : lp;
-        const float4 *A = reinterpret_cast<const float4 *>(a.ahat) + (size_t)ox * sxo + (size_t)oy * sy + zmap(oz, nl);
+        const float4 *A = a.ahat + (size_t)ox * sxo + (size_t)oy * sy + z_order(oz, nl, zs, z_parity_split(ni));
         const float4 a01 = __ldg(A), a23 = __ldg(A + sp), a45 = __ldg(A + 2 * sp);
         float2 g0 = make_float2(a01.x, a01.y), g1 = make_float2(a01.z, a01.w), g2 = make_float2(a23.x, a23.y),
                g3 = make_float2(a23.z, a23.w), g4 = make_float2(a45.x, a45.y), g5 = make_float2(a45.z, a45.w);

@@ -1,24 +1,11 @@
-// Dispatch of the compile-time-sized matvec passes (matvec_yz.cu, matvec_x.cu: one object per edge)
-// and the Green octant in their z order.
+// Dispatch of the compile-time-sized matvec passes (matvec_yz.cu, matvec_x.cu: one object per edge).
 #include "internal.h"
-#include "zorder.cuh"
 
 namespace ddagpu {
 
 namespace {
 
 bool fast_edge(int n) { return n >= 4 && n <= 128 && (n & (n - 1)) == 0; }
-
-// Green octant [ni+1][nj+1][3][nl+1] float4 (z in parity order) -> the z order of the rows
-__global__ void __launch_bounds__(256) order_green(const float4 *__restrict__ oct, float4 *__restrict__ out, int nl,
-                                                   int zs, int split, size_t n)
-{
-    const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (q >= n) return;
-    const int oz = (int)(q % (nl + 1)), z = (oz & 1) ? (nl / 2 + 1 + (oz >> 1)) : (oz >> 1);
-    const size_t row = q / (nl + 1);
-    out[row * z_entries(nl, zs) + z_order(oz, nl, zs, split)] = oct[row * (nl + 1) + z];
-}
 
 }  // namespace
 
@@ -27,17 +14,9 @@ bool matvec_fast_supported(const Lat &L) { return fast_edge(L.ni) && fast_edge(L
 // spectral columns per TMA tile of the x pass; 0 where the rows are shorter
 int matvec_fast_x_tile(int nl) { return nl >= 8 ? 16 : 0; }
 
-size_t green_order_elems(const Lat &L)
+cudaError_t matvec_kernel_smem(const void *kernel, int bytes)
 {
-    return (size_t)(L.ni + 1) * (L.nj + 1) * 3 * z_entries(L.nl, matvec_z_split(L.nj, L.nl));
-}
-
-cudaError_t green_order(const Lat &L, const float2 *ahat, float4 *out, cudaStream_t st)
-{
-    const size_t n = (size_t)(L.ni + 1) * (L.nj + 1) * 3 * (L.nl + 1);
-    order_green<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4 *>(ahat), out, L.nl,
-                                                             matvec_z_split(L.nj, L.nl), z_parity_split(L.ni), n);
-    return cudaGetLastError();
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 void matvec_fast_defaults(const Lat &L, bool has_tmap, int *fx, int *fyz)

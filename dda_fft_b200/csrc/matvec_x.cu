@@ -282,7 +282,7 @@ k2q(MatvecArgs a, const __grid_constant__ CUtensorMap tmap)
     const bool bz = lp >= nl;
     const unsigned sign = 0x80000000u, my = by ? sign : 0u, mz = bz ? sign : 0u;
     const size_t sp = z_entries(nl, a.zs), sy = 3 * sp, sxo = (size_t)(nj + 1) * sy;
-    const float4 *G0 = a.aq + (size_t)(by ? 2 * nj - jp : jp) * sy;
+    const float4 *G0 = a.ahat + (size_t)(by ? 2 * nj - jp : jp) * sy;
     const int e0 = z_order(bz ? 2 * nl - lp : lp, nl, a.zs, z_parity_split(NI)), e1 = z_order(bz ? 2 * nl - lp - 1 : lp + 1, nl, a.zs, z_parity_split(NI));
     const float2 sg = dup2(a.conj ? 1.f : -1.f), ng = dup2(a.conj ? -1.f : 1.f);
     const int k1 = sub;
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(Sx<NI>::RM * TL, 512 / (Sx<NI>::RM * TL)) k2f(
     const int lp = z_bin(l0 + t, nl, a.zs), mz = lp > nl, oz = mz ? 2 * nl - lp : lp;
     // [ox][oy][3][z_order(oz)], two components per float4
     const size_t sp = z_entries(nl, a.zs), sy = 3 * sp, sxo = (size_t)(nj + 1) * sy;
-    const float4 *Ayz = a.aq + (size_t)oy * sy + z_order(oz, nl, a.zs, z_parity_split(NI));
+    const float4 *Ayz = a.ahat + (size_t)oy * sy + z_order(oz, nl, a.zs, z_parity_split(NI));
 #pragma unroll 1
     for (int h = 0; h < 2; h++) {
         float2 X[3][R2];
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(Sx<NI>::RM * TL, pair_min_blocks<NI>() * XC / 
     const bool bz = lp > nl;
     const unsigned sign = 0x80000000u, my = by ? sign : 0u, mz = bz ? sign : 0u;
     const size_t sp = z_entries(nl, a.zs), sy = 3 * sp, sxo = (size_t)(nj + 1) * sy;
-    const float4 *G0 = a.aq + (size_t)(by ? 2 * nj - jp : jp) * sy + z_order(bz ? 2 * nl - lp : lp, nl, a.zs, z_parity_split(NI));
+    const float4 *G0 = a.ahat + (size_t)(by ? 2 * nj - jp : jp) * sy + z_order(bz ? 2 * nl - lp : lp, nl, a.zs, z_parity_split(NI));
     const double *E0 = a.einc + 6 * rhs0, *E1 = E0 + 6;
     P2 E[3];
 #pragma unroll
@@ -648,7 +648,7 @@ template <int NI>
 cudaError_t prep_x()
 {
     auto set = [](const void *k, size_t bytes) {
-        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        return matvec_kernel_smem(k, (int)bytes);
     };
     constexpr size_t P = (size_t)6 * NI * XC * sizeof(float4);
     cudaError_t e = set((const void *)k2q<NI, 0>, P);

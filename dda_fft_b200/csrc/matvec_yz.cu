@@ -602,7 +602,7 @@ cudaError_t prep_yz_v()
     const void *ks[4] = {(const void *)k1p<NJ, NL, NT, MB, 0>, (const void *)k1p<NJ, NL, NT, MB, 1>,
                          (const void *)k1p<NJ, NL, NT, MB, 2>, (const void *)k3p<NJ, NL, NT, MB>};
     for (const void *k : ks)
-        if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, B)) return e;
+        if (cudaError_t e = matvec_kernel_smem(k, B)) return e;
     return cudaSuccess;
 }
 
