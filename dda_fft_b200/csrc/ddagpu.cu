@@ -131,11 +131,22 @@ struct ddagpu_ctx {
     } gkey{};
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
-    GraphKey wkey{};                 // the whole-solve graph of batched calls
-    cudaGraph_t wgraph = nullptr;
-    cudaGraphExec_t wexec = nullptr;
-    long long w_fixed = 0, w_per_iter = 0;
-    int w_matvec0 = 0, w_matvec_it = 0;
+    struct WholeGraph {              // a recorded whole solve
+        GraphKey key{};
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        long long fixed = 0, per_iter = 0;
+        int matvec0 = 0, matvec_it = 0;
+        void drop()
+        {
+            if (exec) cudaGraphExecDestroy(exec);
+            if (graph) cudaGraphDestroy(graph);
+            exec = nullptr;
+            graph = nullptr;
+        }
+    } whole[2];                      // batched calls, single solves (ddagpu_dda_fft)
+    GraphKey single_key{};           // shape of the last single solves and how many there were:
+    int single_seen = 0;             // the third is recorded
     int *nact_dev = nullptr;         // [cap] active cells per right-hand side
     int *err_dev = nullptr;          // set by a kernel whose bounded wait gave up
     void *worm_buf = nullptr;        // monomers of the realisation being rasterised
@@ -145,6 +156,8 @@ struct ddagpu_ctx {
     // far field by kz groups: the plan of the directions last uploaded, its device tables
     ddagpu::KzPlan kz;
     int ff_mode = 0;                 // ddagpu_set_farfield_mode
+    std::vector<double> kz_dirs;     // the directions and the call shape that kz was planned for
+    double kz_shape[6] = {};
     int *kz_tab = nullptr;
     double *kz_val = nullptr;
     float2 *kz_sum = nullptr;
@@ -233,12 +246,9 @@ void drop_graphs(ddagpu_ctx *c)
     c->gen += 1;   // a group's graph holding this context is rebuilt too
     if (c->gexec) cudaGraphExecDestroy(c->gexec);
     if (c->graph) cudaGraphDestroy(c->graph);
-    if (c->wexec) cudaGraphExecDestroy(c->wexec);
-    if (c->wgraph) cudaGraphDestroy(c->wgraph);
+    for (auto &w : c->whole) w.drop();
     c->gexec = nullptr;
     c->graph = nullptr;
-    c->wexec = nullptr;
-    c->wgraph = nullptr;
 }
 
 int ensure_post(ddagpu_ctx *c, int ndir, int nplanes, int nangles)
@@ -337,6 +347,20 @@ FieldArgs fa_args(ddagpu_ctx *c, int nrhs, int nmat1, double d0, float tau)
     return f;
 }
 
+// Pinned block of a whole solve, after the staging of its inputs and results (ensure_pin): the
+// solver states on their way back, the active counts on their way in.
+struct alignas(16) PinnedSolve {
+    int last, werr;
+    RhsState *states() { return reinterpret_cast<RhsState *>(this + 1); }
+    int *nact(int cap) { return reinterpret_cast<int *>(states() + cap); }
+    static size_t bytes(int cap) { return sizeof(PinnedSolve) + (size_t)cap * (sizeof(RhsState) + sizeof(int)) + 16; }
+};
+
+PinnedSolve *pin_solve(ddagpu_ctx *c)
+{
+    return reinterpret_cast<PinnedSolve *>(c->pin + ((c->pin_bytes + 15) & ~(size_t)15));
+}
+
 struct SolveResult {
     std::vector<RhsState> st;
     std::vector<double> trace;
@@ -376,9 +400,9 @@ ddagpu_ctx::GraphKey whole_key(ddagpu_ctx *c, int nrhs, int solver, float tau, i
 
 // Records the whole solve into graph g as a branch with no dependencies; n_fixed and
 // n_per_iter receive the kernels of the fixed part and of one loop pass.
-template <class Step0, class Top, class Body>
+template <class Step0, class Body>
 int record_whole_solve(ddagpu_ctx *c, cudaGraph_t g, int nrhs, int max_step, float err_max, int nmat1,
-                       double d0, float tau, Step0 &step0, Top &top, Body &body,
+                       double d0, float tau, Step0 &step0, Body &body,
                        const std::function<int()> &post, long long &n_fixed, long long &n_per_iter)
 {
     cudaStream_t st = c->st;
@@ -402,12 +426,12 @@ int record_whole_solve(ddagpu_ctx *c, cudaGraph_t g, int nrhs, int max_step, flo
     e = cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return give_up(DDAGPU_OK, e, "capture");
     int rc = DDAGPU_OK;
-    e = launch_init_state(c->state, c->active, nrhs, (double)err_max, c->nact_dev, st);
-    if (e == cudaSuccess) rc = step0();
-    if (rc == DDAGPU_OK && e == cudaSuccess) e = launch_step_set(c->step_dev, 1, st);
-    if (rc == DDAGPU_OK && e == cudaSuccess) rc = top(max_step, c->step_dev);
-    if (rc == DDAGPU_OK && e == cudaSuccess)
-        e = launch_loop_control(c->active, nrhs, c->step_dev, max_step, h, st);
+    FieldArgs F = fa_args(c, nrhs, nmat1, d0, tau);
+    // (the sized passes' phase tables set the state up)
+    if (!c->fast) e = launch_init_state(c->state, c->active, nrhs, (double)err_max, c->nact_dev, st);
+    if (e == cudaSuccess) rc = step0(true);
+    if (rc == DDAGPU_OK) e = launch_step_top(c->state, c->active, nrhs, c->step_dev, 1, max_step, h, st);
+    if (rc == DDAGPU_OK && e == cudaSuccess) e = launch_gated_copy(F, 0, st);
     if (rc != DDAGPU_OK || e != cudaSuccess) return give_up(rc, e, "step 0");
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t *deps = nullptr;
@@ -418,7 +442,7 @@ int record_whole_solve(ddagpu_ctx *c, cudaGraph_t g, int nrhs, int max_step, flo
     cudaGraph_t t = nullptr;
     e = cudaStreamEndCapture(st, &t);
     if (e != cudaSuccess) return give_up(DDAGPU_OK, e, "end capture");
-    const long long n_head = c->launches - l0 + 3;   // + init, step set, loop control
+    const long long n_head = c->launches - l0 + (c->fast ? 2 : 3);   // + step top, copy, initial state
     // the while node and its body: one iteration, the next step's test, the condition
     cudaGraphNodeParams np{};
     np.type = cudaGraphNodeTypeConditional;
@@ -433,10 +457,8 @@ int record_whole_solve(ddagpu_ctx *c, cudaGraph_t g, int nrhs, int max_step, flo
                                       cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return give_up(DDAGPU_OK, e, "body capture");
     rc = body(max_step, c->step_dev, true);
-    if (rc == DDAGPU_OK) e = launch_step_advance(c->step_dev, st);
-    if (rc == DDAGPU_OK && e == cudaSuccess) rc = top(max_step, c->step_dev);
-    if (rc == DDAGPU_OK && e == cudaSuccess)
-        e = launch_loop_control(c->active, nrhs, c->step_dev, max_step, h, st);
+    if (rc == DDAGPU_OK) e = launch_step_top(c->state, c->active, nrhs, c->step_dev, 0, max_step, h, st);
+    if (rc == DDAGPU_OK && e == cudaSuccess) e = launch_gated_copy(F, 0, st);
     if (rc != DDAGPU_OK || e != cudaSuccess) return give_up(rc, e, "body");
     e = cudaStreamEndCapture(st, &t);
     if (e != cudaSuccess) return give_up(DDAGPU_OK, e, "end body capture");
@@ -445,14 +467,12 @@ int record_whole_solve(ddagpu_ctx *c, cudaGraph_t g, int nrhs, int max_step, flo
     const long long l2 = c->launches;
     e = cudaStreamBeginCaptureToGraph(st, g, &cn, nullptr, 1, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return give_up(DDAGPU_OK, e, "tail capture");
-    FieldArgs F = fa_args(c, nrhs, nmat1, d0, tau);
-    e = launch_scalar(c->state, nullptr, nullptr, nrhs, SC_FINAL, 0, nullptr, 0, st);
-    if (e == cudaSuccess) e = launch_gated_copy(F, 1, st);
+    e = launch_gated_copy(F, 2, st);
     if (e == cudaSuccess) rc = post();
     if (rc != DDAGPU_OK || e != cudaSuccess) return give_up(rc, e, "tail");
     e = cudaStreamEndCapture(st, &t);
     if (e != cudaSuccess) return give_up(DDAGPU_OK, e, "end tail capture");
-    const long long n_tail = c->launches - l2 + 2;
+    const long long n_tail = c->launches - l2 + 1;
     n_fixed = n_head + n_tail;
     n_per_iter = n_body;
     c->launches = l_save;
@@ -465,15 +485,14 @@ int read_whole_solve(ddagpu_ctx *c, int nrhs, SolveResult &res, long long n_fixe
                      int matvec0, int matvec_it, bool own_launch = true)
 {
     cudaStream_t st = c->st;
-    int last = 1;
-    res.st.resize((size_t)nrhs);
-    CK(cudaMemcpyAsync(res.st.data(), c->state, nrhs * sizeof(RhsState), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&last, c->step_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
-    int werr = 0;
-    CK(cudaMemcpyAsync(&werr, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
+    PinnedSolve *P = pin_solve(c);
+    CK(cudaMemcpyAsync(P->states(), c->state, nrhs * sizeof(RhsState), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&P->last, c->step_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&P->werr, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    RET(device_wait_error(c, werr));
-    c->launches += n_fixed + (long long)(last - 1) * n_per_iter;
+    res.st.assign(P->states(), P->states() + nrhs);
+    RET(device_wait_error(c, P->werr));
+    c->launches += n_fixed + (long long)(P->last - 1) * n_per_iter;
     res.matvec0 = matvec0;
     res.matvec_it = matvec_it;
     if (own_launch) c->graph_runs += 1;   // a group's launch is counted by the group
@@ -490,35 +509,33 @@ struct GroupRecord {
     int matvec0 = 0, matvec_it = 0;
 };
 
-template <class Step0, class Top, class Body>
+template <class Step0, class Body>
 int run_whole_graph(ddagpu_ctx *c, int nrhs, int solver, float tau, int max_step, float err_max,
                     int nmat1, double d0, int nact, const int *nact_per, SolveResult &res,
-                    Step0 &step0, Top &top, Body &body, const std::function<int()> &post,
-                    GroupRecord *rec)
+                    Step0 &step0, Body &body, const std::function<int()> &post,
+                    GroupRecord *rec, bool single)
 {
     cudaStream_t st = c->st;
-    std::vector<int> na((size_t)nrhs);
-    for (int k = 0; k < nrhs; k++) na[(size_t)k] = nact_per ? nact_per[k] : nact;
-    CK(cudaMemcpyAsync(c->nact_dev, na.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice, st));
+    int *na = pin_solve(c)->nact(c->cap);
+    for (int k = 0; k < nrhs; k++) na[k] = nact_per ? nact_per[k] : nact;
+    CK(cudaMemcpyAsync(c->nact_dev, na, nrhs * sizeof(int), cudaMemcpyHostToDevice, st));
     const ddagpu_ctx::GraphKey key = whole_key(c, nrhs, solver, tau, max_step, err_max, nmat1, d0);
     if (rec) {   // for the group's graph; the group launches it and reads the results
         rec->key = key;
         if (!rec->graph) return DDAGPU_OK;
-        RET(record_whole_solve(c, rec->graph, nrhs, max_step, err_max, nmat1, d0, tau, step0, top, body,
+        RET(record_whole_solve(c, rec->graph, nrhs, max_step, err_max, nmat1, d0, tau, step0, body,
                                post, rec->n_fixed, rec->n_per_iter));
         rec->matvec0 = res.matvec0;
         rec->matvec_it = res.matvec_it;
         return DDAGPU_OK;
     }
-    if (!c->wexec || std::memcmp(&key, &c->wkey, sizeof key) != 0) {
-        if (c->wexec) cudaGraphExecDestroy(c->wexec);
-        if (c->wgraph) cudaGraphDestroy(c->wgraph);
-        c->wexec = nullptr;
-        c->wgraph = nullptr;
+    ddagpu_ctx::WholeGraph &W = c->whole[single ? 1 : 0];
+    if (!W.exec || std::memcmp(&key, &W.key, sizeof key) != 0) {
+        W.drop();
         cudaGraph_t g = nullptr;
         CK(cudaGraphCreate(&g, 0));
         long long nf = 0, npi = 0;
-        const int rc = record_whole_solve(c, g, nrhs, max_step, err_max, nmat1, d0, tau, step0, top, body,
+        const int rc = record_whole_solve(c, g, nrhs, max_step, err_max, nmat1, d0, tau, step0, body,
                                           post, nf, npi);
         if (rc != DDAGPU_OK) {
             cudaGraphDestroy(g);
@@ -530,16 +547,16 @@ int run_whole_graph(ddagpu_ctx *c, int nrhs, int solver, float tau, int max_step
             cudaGraphDestroy(g);
             return fail(DDAGPU_ECUDA, std::string("solve graph (instantiate): ") + cudaGetErrorString(e));
         }
-        c->wgraph = g;
-        c->wexec = x;
-        c->wkey = key;
-        c->w_fixed = nf;
-        c->w_per_iter = npi;
-        c->w_matvec0 = res.matvec0;
-        c->w_matvec_it = res.matvec_it;
+        W.graph = g;
+        W.exec = x;
+        W.key = key;
+        W.fixed = nf;
+        W.per_iter = npi;
+        W.matvec0 = res.matvec0;
+        W.matvec_it = res.matvec_it;
     }
-    CK(cudaGraphLaunch(c->wexec, st));
-    return read_whole_solve(c, nrhs, res, c->w_fixed, c->w_per_iter, c->w_matvec0, c->w_matvec_it);
+    CK(cudaGraphLaunch(W.exec, st));
+    return read_whole_solve(c, nrhs, res, W.fixed, W.per_iter, W.matvec0, W.matvec_it);
 }
 
 // post (may be null): kernels issued after the solve on the context's stream (far field,
@@ -548,7 +565,7 @@ int run_whole_graph(ddagpu_ctx *c, int nrhs, int solver, float tau, int max_step
 int run_solver(ddagpu_ctx *c, int nrhs, int solver, float tau, int max_step, float err_max,
                int nmat1, double d0, int nact, SolveResult &res, bool want_trace,
                const float2 *rhs_in = nullptr, const int *nact_per = nullptr,
-               const std::function<int()> *post = nullptr, GroupRecord *rec = nullptr)
+               const std::function<int()> *post = nullptr, GroupRecord *rec = nullptr, bool single = false)
 {
     if (solver < 0 || solver > 3) return fail(DDAGPU_EINVAL, "solver must be 0..3");
     if (max_step < 0) return fail(DDAGPU_EINVAL, "Max_Step must be >= 0");
@@ -596,10 +613,12 @@ int run_solver(ddagpu_ctx *c, int nrhs, int solver, float tau, int max_step, flo
     };
 
     // ---- step 0 (dda_func.cpp:1102-1293): p = p_inc, or the given right-hand side
-    auto step0 = [&]() -> int {
+    // (recorded: the state is set up by the phase tables' launch and SC_START is left to step_top)
+    auto step0 = [&](bool recorded = false) -> int {
     if (!rhs_in && c->fast) {
         // the forward pass computes p_inc itself (from the phase tables) and stores it
-        CK(launch_inc_tables(F, c->inc_tab, st));
+        if (recorded) CK(launch_inc_tables(F, c->inc_tab, st, c->active, (double)err_max, c->nact_dev));
+        else CK(launch_inc_tables(F, c->inc_tab, st));
         MatvecArgs m = mv_args(c, nrhs, c->p, c->r, 1, 0.f, nullptr, 0, nmat1, true);
         m.inc = 1;
         m.pair = (c->pair_step0 && nrhs % 2 == 0) ? 1 : 0;
@@ -645,7 +664,7 @@ int run_solver(ddagpu_ctx *c, int nrhs, int solver, float tau, int max_step, flo
         CK(scal(SC_STEP0_ERR1, 0));
         break;
     }
-    CK(scal(SC_START, 0));
+    if (!recorded) CK(scal(SC_START, 0));
     // p_min = p (the step-0 iterate) is copied by the gated copy of the first iteration
     res.matvec_it = (solver == 1 || solver == 2) ? 2 : 1;
     return DDAGPU_OK;
@@ -715,7 +734,7 @@ int run_solver(ddagpu_ctx *c, int nrhs, int solver, float tau, int max_step, flo
         return DDAGPU_OK;
     };
     if (whole) return run_whole_graph(c, nrhs, solver, tau, max_step, err_max, nmat1, d0, nact,
-                                      nact_per, res, step0, top, body, *post, rec);
+                                      nact_per, res, step0, body, *post, rec, single);
     RET(step0());
     // iteration 1 (and all of them without the graph) from the host: the loop stops when
     // no right-hand side is left active (read back once per iteration)
@@ -1046,8 +1065,7 @@ int ddagpu_destroy(ddagpu_ctx *c)
     if (c->x64) cudaFree(c->x64);
     if (c->gexec) cudaGraphExecDestroy(c->gexec);
     if (c->graph) cudaGraphDestroy(c->graph);
-    if (c->wexec) cudaGraphExecDestroy(c->wexec);
-    if (c->wgraph) cudaGraphDestroy(c->wgraph);
+    for (auto &w : c->whole) w.drop();
     void *ptrs[] = {c->ahat, c->tw,     c->work,   c->p,       c->pmin,   c->r,     c->s,
                     c->w,    c->g,      c->h,      c->state,   c->active, c->trace, c->occ,
                     c->mv,   c->alpha,  c->kinc,   c->einc,    c->ksc,    c->esc_acc,
@@ -1275,11 +1293,31 @@ int upload_materials(ddagpu_ctx *c, const int *mv, int nmat1, const signed char 
 // nact: active cells per right-hand side, for the choice between the two forms.
 int upload_directions(ddagpu_ctx *c, const double *ks, int nrhs, int ndir, bool pairs, double nact)
 {
+    if (ndir <= 0) {
+        c->kz.groups = 0;
+        return DDAGPU_OK;
+    }
+    const size_t n = (size_t)nrhs * ndir * 3;
+    CK(cudaMemcpyAsync(c->ksc, ks, n * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    // the plan (and its tables on the device) of the last call's directions stands for the same
+    // values again: the samples of a fixed orientation, the two polarisations of a sample
+    const double shape[6] = {(double)nrhs, (double)ndir, pairs ? 1.0 : 0.0, (double)c->ff_mode, nact,
+                             c->kz_tab ? 1.0 : 0.0};
+    if (c->kz_dirs.size() == n && std::memcmp(c->kz_shape, shape, sizeof shape) == 0 &&
+        std::memcmp(c->kz_dirs.data(), ks, n * sizeof(double)) == 0)
+        return DDAGPU_OK;
+    c->kz_dirs.clear();
     c->kz.groups = 0;
-    if (ndir <= 0) return DDAGPU_OK;
-    CK(cudaMemcpyAsync(c->ksc, ks, (size_t)nrhs * ndir * 3 * sizeof(double), cudaMemcpyHostToDevice, c->st));
     plan_kz_groups(ks, nrhs, ndir, pairs, c->ni, c->nj, c->nl, nact, c->ff_mode, c->kz);
-    if (!c->kz.groups) return DDAGPU_OK;
+    auto remember = [&]() {
+        c->kz_dirs.assign(ks, ks + n);
+        std::memcpy(c->kz_shape, shape, sizeof shape);
+        c->kz_shape[5] = c->kz_tab ? 1.0 : 0.0;
+    };
+    if (!c->kz.groups) {
+        remember();
+        return DDAGPU_OK;
+    }
     auto grow = [&](auto *&buf, size_t &cap, size_t need) -> int {
         if (need <= cap) return DDAGPU_OK;
         drop_graphs(c);
@@ -1297,6 +1335,7 @@ int upload_directions(ddagpu_ctx *c, const double *ks, int nrhs, int ndir, bool 
     CK(cudaMemcpyAsync(c->kz_tab, c->kz.tab.data(), c->kz.tab.size() * sizeof(int), cudaMemcpyHostToDevice, c->st));
     CK(cudaMemcpyAsync(c->kz_val, c->kz.kz.data(), c->kz.kz.size() * sizeof(double), cudaMemcpyHostToDevice,
                        c->st));
+    remember();
     return DDAGPU_OK;
 }
 
@@ -1458,7 +1497,7 @@ int ensure_pin(ddagpu_ctx *c, size_t bytes)
     if (c->pin) cudaFreeHost(c->pin);
     c->pin = nullptr;
     c->pin_bytes = 0;
-    CK(cudaHostAlloc((void **)&c->pin, bytes, cudaHostAllocDefault));
+    CK(cudaHostAlloc((void **)&c->pin, ((bytes + 15) & ~(size_t)15) + PinnedSolve::bytes(c->cap), cudaHostAllocDefault));
     c->pin_bytes = bytes;
     return DDAGPU_OK;
 }
@@ -1625,34 +1664,61 @@ int ddagpu_dda_fft(ddagpu_ctx *c, int iNoIllumination, int solver, float rTau, i
     int nact = 0;
     RET(upload_materials(c, iListMV, nmat1, cAlpha, &nact));
     RET(ensure_post(c, std::max(ndir, 1), std::max(iNoScPl, 1), std::max(iNoA, 1)));
-    std::vector<float2> al((size_t)nmat1);
-    for (int m = 0; m < nmat1; m++) al[(size_t)m] = make_float2(cListMaterials[2 * m], cListMaterials[2 * m + 1]);
-    double kd3[3] = {kinc[0], kinc[1], kinc[2]};
-    double ed6[6];
+    // staging: inputs ks, kin, ein (double), al; outputs es, {Cabs, Cext}.  Pinned and the solve one
+    // graph launch once two solves of this shape have run (a sample's two polarisations; a worker's
+    // samples are thousands of them); those two take the host loop and pageable memory, as
+    // recording the graph and pinning cost more than a solve.
+    const size_t n_ks = (size_t)ndir * 3;
+    ddagpu_ctx::GraphKey seen{};
+    seen.solver = solver;
+    seen.max_step = Max_Step;
+    seen.nmat1 = nmat1;
+    seen.tau = rTau;
+    seen.err_max = Error_max;
+    seen.d0 = d0;
+    seen.post = ndir;
+    if (std::memcmp(&seen, &c->single_key, sizeof seen) != 0) c->single_seen = 0;
+    c->single_key = seen;
+    const bool again = !trace && c->graph_on && c->single_seen >= 2;
+    c->single_seen += c->single_seen < 2 ? 1 : 0;
+    const size_t o_kin = n_ks * 8, o_ein = o_kin + 24, o_al = o_ein + 48, o_es = o_al + (size_t)nmat1 * 8,
+                 o_c = o_es + n_ks * 8, total = o_c + 8;
+    std::vector<double> pageable;
+    unsigned char *buf;
+    if (again) {
+        RET(ensure_pin(c, total));
+        buf = c->pin;
+    } else {
+        pageable.resize((total + 7) / 8);
+        buf = reinterpret_cast<unsigned char *>(pageable.data());
+    }
+    double *kd = reinterpret_cast<double *>(buf), *kd3 = reinterpret_cast<double *>(buf + o_kin),
+           *ed6 = reinterpret_cast<double *>(buf + o_ein);
+    float *al = reinterpret_cast<float *>(buf + o_al), *es = reinterpret_cast<float *>(buf + o_es),
+          *cc = reinterpret_cast<float *>(buf + o_c);
+    for (size_t k = 0; k < n_ks; k++) kd[k] = ksc[k];
+    for (int k = 0; k < 3; k++) kd3[k] = kinc[k];
     for (int k = 0; k < 6; k++) ed6[k] = Einc[k];
-    std::vector<double> kd((size_t)ndir * 3);
-    for (size_t k = 0; k < kd.size(); k++) kd[k] = ksc[k];
-    CK(cudaMemcpyAsync(c->alpha, al.data(), nmat1 * sizeof(float2), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->kinc, kd3, sizeof kd3, cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->einc, ed6, sizeof ed6, cudaMemcpyHostToDevice, c->st));
-    RET(upload_directions(c, kd.data(), 1, ndir, false, nact));
+    std::memcpy(al, cListMaterials, (size_t)nmat1 * 8);
+    CK(cudaMemcpyAsync(c->alpha, al, (size_t)nmat1 * 8, cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(c->kinc, kd3, 24, cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(c->einc, ed6, 48, cudaMemcpyHostToDevice, c->st));
+    RET(upload_directions(c, kd, 1, ndir, false, nact));
     // nact: counted by upload_materials
     if (nact == 0) return fail(DDAGPU_EINVAL, "no active dipoles");
     SolveResult res;
-    RET(run_solver(c, 1, solver, rTau, Max_Step, Error_max, nmat1, d0, nact, res, trace != nullptr));
-    RET(run_post(c, 1, nmat1, d0, ndir));
-    std::vector<float2> esc((size_t)ndir * 3);
-    float ca = 0, ce = 0;
-    if (ndir) CK(cudaMemcpyAsync(esc.data(), c->esc, esc.size() * sizeof(float2), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(&ca, c->cabs, sizeof(float), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(&ce, c->cext, sizeof(float), cudaMemcpyDeviceToHost, c->st));
+    const std::function<int()> post = [&]() { return run_post(c, 1, nmat1, d0, ndir); };
+    c->post_key = -1 - (long long)ndir;   // (batched calls' keys are positive)
+    RET(run_solver(c, 1, solver, rTau, Max_Step, Error_max, nmat1, d0, nact, res, trace != nullptr, nullptr,
+                   nullptr, again ? &post : nullptr, nullptr, true));
+    if (!again) RET(post());
+    if (ndir) CK(cudaMemcpyAsync(es, c->esc, n_ks * 8, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(cc, c->cabs, sizeof(float), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(cc + 1, c->cext, sizeof(float), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    for (size_t k = 0; k < esc.size(); k++) {
-        Esc[2 * k] = esc[k].x;
-        Esc[2 * k + 1] = esc[k].y;
-    }
-    *rCabs = ca;
-    *rCext = ce;
+    if (ndir) std::memcpy(Esc, es, n_ks * 8);
+    *rCabs = cc[0];
+    *rCext = cc[1];
     const RhsState &S = res.st[0];
     if (info) {
         info->steps = S.steps;
@@ -2043,7 +2109,16 @@ int ddagpu_mueller(ddagpu_ctx *c, const float *kinc, const float *einc0, const f
     DevGuard dg(c->dev);
     const int ndir = nplanes * nangles;
     RET(ensure_post(c, ndir, nplanes, nangles));
-    std::vector<double> kd(6), ed(12), ks((size_t)2 * ndir * 3), nv((size_t)nplanes * 3);
+    // staging in the context's pinned block where it has one (it gets one with its first recorded
+    // solve), else pageable: kd, ed, ks, nv and the result in double, es in float
+    const size_t n_ks = (size_t)6 * ndir, n_mo = (size_t)nangles * 16,
+                 doubles = 6 + 12 + n_ks + (size_t)nplanes * 3 + n_mo + n_ks;
+    std::vector<double> pageable;
+    if (c->pin) RET(ensure_pin(c, doubles * sizeof(double)));
+    else pageable.resize(doubles);
+    double *kd = c->pin ? reinterpret_cast<double *>(c->pin) : pageable.data(), *ed = kd + 6, *ks = ed + 12,
+           *nv = ks + n_ks, *mo = nv + (size_t)nplanes * 3;
+    float *es = reinterpret_cast<float *>(mo + n_mo);
     for (int k = 0; k < 3; k++) kd[k] = kd[3 + k] = kinc[k];
     for (int k = 0; k < 6; k++) {
         ed[k] = einc0[k];
@@ -2051,22 +2126,18 @@ int ddagpu_mueller(ddagpu_ctx *c, const float *kinc, const float *einc0, const f
     }
     for (int k = 0; k < ndir * 3; k++) ks[k] = ks[(size_t)ndir * 3 + k] = ksc[k];
     for (int k = 0; k < nplanes * 3; k++) nv[k] = normals[k];
-    std::vector<float2> es((size_t)2 * ndir * 3);
-    for (int k = 0; k < ndir * 3; k++) {
-        es[k] = make_float2(esc0[2 * k], esc0[2 * k + 1]);
-        es[(size_t)ndir * 3 + k] = make_float2(esc1[2 * k], esc1[2 * k + 1]);
-    }
-    CK(cudaMemcpyAsync(c->kinc, kd.data(), kd.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->einc, ed.data(), ed.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->ksc, ks.data(), ks.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->normals, nv.data(), nv.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->esc, es.data(), es.size() * sizeof(float2), cudaMemcpyHostToDevice, c->st));
+    std::memcpy(es, esc0, n_ks * sizeof(float));
+    std::memcpy(es + n_ks, esc1, n_ks * sizeof(float));
+    CK(cudaMemcpyAsync(c->kinc, kd, 6 * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(c->einc, ed, 12 * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(c->ksc, ks, n_ks * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(c->normals, nv, (size_t)nplanes * 3 * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(c->esc, es, 2 * n_ks * sizeof(float), cudaMemcpyHostToDevice, c->st));
     MuellerArgs m{1, nplanes, nangles, ndir, c->kinc, c->einc, c->ksc, c->normals, c->esc, c->mueller};
     CK(launch_mueller(m, c->st));
-    std::vector<double> mo((size_t)nangles * 16);
-    CK(cudaMemcpyAsync(mo.data(), c->mueller, mo.size() * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(mo, c->mueller, n_mo * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    for (size_t k = 0; k < mo.size(); k++) out[k] = (float)mo[k];
+    for (size_t k = 0; k < n_mo; k++) out[k] = (float)mo[k];
     return DDAGPU_OK;
 }
 

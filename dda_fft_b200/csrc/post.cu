@@ -47,18 +47,26 @@ constexpr int FF_PLANES = 8;     // lattice planes per CTA at most
 __host__ __device__ constexpr int ff_cap(int nr) { return nr == 2 ? 512 : 1024; }
 
 struct FFShape {
-    int D, dpt, DG, RW, threads, planes;
+    int D, dpt, DG, RW, threads, planes, parts;
 };
 
 // blocks: right-hand-side blocks of the grid (nrhs / NR); the planes per CTA are the most
 // that still give the grid eight CTAs per SM (148 SMs), two at least, so that the plane
 // groups' unequal work (a target's middle planes hold more dipoles) is spread
-FFShape ff_shape(int ndir, int dpt, int ni = 1, int blocks = 1)
+// where that leaves fewer than four CTAs per SM (one or a few right-hand sides on a small lattice)
+// a CTA takes a part of one plane's rows, eight rows at least (32^3, 19 directions, one
+// right-hand side: 16 -> 128 CTAs, 26 -> 12 us)
+FFShape ff_shape(int ndir, int dpt, int ni = 1, int blocks = 1, int nj = 1)
 {
     FFShape s;
     const int chunks = (ndir + FF_DMAX - 1) / FF_DMAX;
     s.planes = FF_PLANES;
     while (s.planes > 2 && (long long)((ni + s.planes - 1) / s.planes) * chunks * blocks < 8 * 148) s.planes /= 2;
+    s.parts = 1;
+    if ((long long)((ni + s.planes - 1) / s.planes) * chunks * blocks < 4 * 148) {
+        s.planes = 1;
+        while ((long long)ni * s.parts * chunks * blocks < 4 * 148 && nj / (2 * s.parts) >= 8) s.parts *= 2;
+    }
     s.D = ndir >= FF_DMAX ? FF_DMAX : ((ndir + FF_DQ - 1) / FF_DQ) * FF_DQ;
     if (s.D < FF_DQ) s.D = FF_DQ;
     s.dpt = dpt;
@@ -119,7 +127,7 @@ DDA_DEV void cp_async8(void *dst, const void *src)
 DDA_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 DDA_DEV void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// grid (direction chunks of D, plane groups of s.planes, nrhs / NR); the lattice has
+// grid (direction chunks of D, plane groups of s.planes x s.parts, nrhs / NR); the lattice has
 // nj, nl < 4096
 template <bool CC, int NR, int DPT>
 __global__ void __launch_bounds__(256) farfield_sum(PostArgs a, FFShape s)
@@ -127,7 +135,9 @@ __global__ void __launch_bounds__(256) farfield_sum(PostArgs a, FFShape s)
     constexpr int CAP = ff_cap(NR);
     extern __shared__ __align__(16) unsigned char smraw[];
     const int nj = a.nj, nl = a.nl, D = s.D, T = blockDim.x, nmat1 = a.nmat1;
-    const int dbase = blockIdx.x * D, i0 = blockIdx.y * s.planes, rhs = NR * blockIdx.z;
+    const int dbase = blockIdx.x * D, i0 = blockIdx.y / s.parts * s.planes, rhs = NR * blockIdx.z;
+    // rows of the plane(s) this CTA sums
+    const int part = blockIdx.y % s.parts, ja = part * nj / s.parts, jb = (part + 1) * nj / s.parts;
     const int np = a.ni - i0 < s.planes ? a.ni - i0 : s.planes;
     const bool cc = CC && blockIdx.x == 0;
     const int dg = threadIdx.x % s.DG, w = threadIdx.x / s.DG;
@@ -153,6 +163,7 @@ __global__ void __launch_bounds__(256) farfield_sum(PostArgs a, FFShape s)
     const double *K = a.ksc + (size_t)rhs * a.ndir * 3;
     for (int e = threadIdx.x; e < (nl + nj + np) * D; e += T) {
         const int dl = e % D, pos = e / D, dd = dbase + dl;
+        if (pos >= nl && pos < nl + nj && (pos < nl + ja || pos >= nl + jb)) continue;   // another part's row
         float2 val = czero();
         if (dd < a.ndir) {
             double ph;
@@ -234,7 +245,7 @@ __global__ void __launch_bounds__(256) farfield_sum(PostArgs a, FFShape s)
             for (int e = threadIdx.x; e < (int)plane; e += T) occs[e] = occr[q0 + e];
         }
         // row factors exp(i (kx x + ky y)) of this plane
-        for (int e = threadIdx.x; e < nj * D; e += T) eyx[e] = cmul(ey[e], ex[ip * D + e % D]);
+        for (int e = ja * D + threadIdx.x; e < jb * D; e += T) eyx[e] = cmul(ey[e], ex[ip * D + e % D]);
         __syncthreads();
         // activity of a staged cell; nmat1 == 0: the activity list's length is not known
         // (allocation-free entry point), so it is read from global memory at the
@@ -245,7 +256,7 @@ __global__ void __launch_bounds__(256) farfield_sum(PostArgs a, FFShape s)
         // ---- active cells of every row (warp per row)
         for (int r = warp; r < nj; r += nwarps) {
             int cnt = 0;
-            for (int c0 = 0; c0 < nl; c0 += 32) {
+            for (int c0 = 0; c0 < nl && r >= ja && r < jb; c0 += 32) {
                 const int l = c0 + lane;
                 const bool act = l < nl && active(occs[r * nl + l]);
                 cnt += __popc(__ballot_sync(0xffffffffu, act));
@@ -387,7 +398,7 @@ __global__ void __launch_bounds__(256) farfield_sum(PostArgs a, FFShape s)
         if (slow_cc) {
             // materials with a polarisability but switched off in the activity list: their
             // dipoles were not staged and are read from global memory
-            for (int e = threadIdx.x; e < (int)plane; e += T) {
+            for (int e = ja * nl + threadIdx.x; e < jb * nl; e += T) {
                 const int m = occs[e];
                 if ((unsigned)m >= (unsigned)nmat1) continue;
                 const int row = e / nl, l = e - row * nl;
@@ -943,12 +954,12 @@ cudaError_t launch_post(const PostArgs &a, float2 *esc, float *cabs, float *cext
         // far field with the cross sections summed by the first direction chunk
         if (a.nj >= 4096 || a.nl >= 4096) return cudaErrorInvalidValue;   // packed list words
         if (a.pairs && a.nrhs % 2 == 0) {
-            const FFShape s = ff_shape(a.ndir, 2, a.ni, a.nrhs / 2);
-            farfield_sum<true, 2, 2><<<dim3(nblk(a.ndir, s.D), nblk(a.ni, s.planes), a.nrhs / 2), s.threads,
+            const FFShape s = ff_shape(a.ndir, 2, a.ni, a.nrhs / 2, a.nj);
+            farfield_sum<true, 2, 2><<<dim3(nblk(a.ndir, s.D), nblk(a.ni, s.planes) * s.parts, a.nrhs / 2), s.threads,
                                        ff_layout(s, a.nj, a.nl, a.nmat1, true, 2).total, st>>>(a, s);
         } else {
-            const FFShape s = ff_shape(a.ndir, 4, a.ni, a.nrhs);
-            farfield_sum<true, 1, 4><<<dim3(nblk(a.ndir, s.D), nblk(a.ni, s.planes), a.nrhs), s.threads,
+            const FFShape s = ff_shape(a.ndir, 4, a.ni, a.nrhs, a.nj);
+            farfield_sum<true, 1, 4><<<dim3(nblk(a.ndir, s.D), nblk(a.ni, s.planes) * s.parts, a.nrhs), s.threads,
                                        ff_layout(s, a.nj, a.nl, a.nmat1, true, 1).total, st>>>(a, s);
         }
         nk += 1;
@@ -1031,8 +1042,8 @@ cudaError_t farfield_noalloc(const PostArgs &in, const float *ksc_dev, float2 *e
     const int n3 = 3 * a.ndir;
     ksc_to_double<<<nblk((size_t)n3, 256), 256, 0, st>>>(ksc_dev, kscd, n3);
     if (a.nj >= 4096 || a.nl >= 4096) return cudaErrorInvalidValue;   // packed list words
-    const FFShape s = ff_shape(a.ndir, 4, a.ni, 1);
-    farfield_sum<false, 1, 4><<<dim3(nblk(a.ndir, s.D), nblk(a.ni, s.planes), 1), s.threads,
+    const FFShape s = ff_shape(a.ndir, 4, a.ni, 1, a.nj);
+    farfield_sum<false, 1, 4><<<dim3(nblk(a.ndir, s.D), nblk(a.ni, s.planes) * s.parts, 1), s.threads,
                                 ff_layout(s, a.nj, a.nl, a.nmat1, false, 1).total, st>>>(a, s);
     post_finalize<<<nblk((size_t)a.ndir, 256), 256, 0, st>>>(a, esc_dev, nullptr, nullptr);
     return cudaGetLastError();

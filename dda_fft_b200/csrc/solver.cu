@@ -265,12 +265,29 @@ DDA_DEV float2 inc_phase(const FieldArgs &a, const double *k, int e)
     return expi_reduced(ph);
 }
 
+// fresh scalars, threshold and active-cell count of one right-hand side
+DDA_DEV void fresh_state(RhsState &st, int &active, double err_max, int nact)
+{
+    RhsState S;
+    memset(&S, 0, sizeof S);
+    S.err_max = err_max;
+    S.active = 1;
+    S.nact = nact;
+    st = S;
+    active = 1;
+}
+
 // The phase tables of every right-hand side, [nrhs][nj + nl + ni], for the forward pass that
 // computes the incident dipoles itself (step 0 of a solve on the compile-time-sized passes).
-__global__ void __launch_bounds__(256) inc_tables(FieldArgs a, float2 *tab)
+// A recorded solve's fresh state is written here too (nact not null).
+__global__ void __launch_bounds__(256) inc_tables(FieldArgs a, float2 *tab, int *active, double err_max, const int *nact)
 {
     const int rhs = blockIdx.x, n = a.nj + a.nl + a.ni;
-    if (a.rhs_active && !a.rhs_active[rhs]) return;
+    if (nact) {
+        if (threadIdx.x == 0) fresh_state(a.st[rhs], active[rhs], err_max, nact[rhs]);
+    } else if (a.rhs_active && !a.rhs_active[rhs]) {
+        return;
+    }
     for (int e = threadIdx.x; e < n; e += blockDim.x) tab[(size_t)rhs * n + e] = inc_phase(a, a.kinc + 3 * rhs, e);
 }
 
@@ -326,6 +343,25 @@ __device__ float2 fmul_ref(float2 a, float2 b)
     // float complex product without contraction, as the reference's cplx operator*
     return make_float2(__fsub_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)),
                        __fadd_rn(__fmul_rn(a.x, b.y), __fmul_rn(a.y, b.x)));
+}
+
+// Convergence test and best-iterate bookkeeping at the top of step `step` (dda_func.cpp:1301-1313)
+// for an active right-hand side; past Max_Step (max_step >= 0) only the copy flag is cleared
+DDA_DEV void step_test(RhsState &S, int step, int max_step)
+{
+    S.need_copy = 0;
+    if (max_step >= 0 && step > max_step) return;   // the host loop has ended here
+    if (S.err <= S.err_max) {
+        S.active = 0;
+    } else if (step == 1) {
+        // the step-0 iterate is the best one so far (dda_func.cpp:1286-1293); it is
+        // stored only now, when an iteration is about to overwrite it
+        S.need_copy = 1;
+    } else if (S.err < S.err_min) {
+        S.err_min = S.err;
+        S.step_min = step - 1;
+        S.need_copy = 1;
+    }
 }
 
 __global__ void scalar_stage(RhsState *st, const int *rhs_active_in, int *rhs_active, int nrhs,
@@ -402,21 +438,7 @@ __global__ void scalar_stage(RhsState *st, const int *rhs_active_in, int *rhs_ac
         S.restored = 0;
         break;
     case SC_TOP: // dda_func.cpp:1301-1313
-        S.need_copy = 0;
-        if (step_dev && step > step_arg) {
-            // a graph-recorded iteration past Max_Step (step_arg): the host loop has ended
-            // here, so only the copy flag is cleared
-        } else if (S.err <= S.err_max) {
-            S.active = 0;
-        } else if (step == 1) {
-            // the step-0 iterate is the best one so far (dda_func.cpp:1286-1293); it is
-            // stored only now, when an iteration is about to overwrite it
-            S.need_copy = 1;
-        } else if (S.err < S.err_min) {
-            S.err_min = S.err;
-            S.step_min = step - 1;
-            S.need_copy = 1;
-        }
+        step_test(S, step, step_dev ? step_arg : -1);
         break;
     case SC_FINAL: // dda_func.cpp:1537-1548
         S.need_copy = (S.err > S.err_min) ? 1 : 0;
@@ -433,12 +455,20 @@ __global__ void scalar_stage(RhsState *st, const int *rhs_active_in, int *rhs_ac
     if (rhs_active) rhs_active[rhs] = S.active;
 }
 
-// need_copy-gated copies (best iterate p -> p_min, rollback p_min -> p)
+// need_copy-gated copies (dir 0: best iterate p -> p_min, 1: rollback p_min -> p), 2: rollback where
+// the final residual is above the best one
 __global__ void __launch_bounds__(256) gated_copy(FieldArgs a, int dir)
 {
     const int rhs = blockIdx.y;
-    const RhsState &S = a.st[rhs];
-    if (!S.need_copy) return;
+    RhsState &S = a.st[rhs];
+    if (dir == 2) {
+        // rollback of a recorded solve, its decision (SC_FINAL) included
+        const bool back = S.err > S.err_min;
+        if (blockIdx.x == 0 && threadIdx.x == 0) S.restored = back ? 1 : 0;
+        if (!back) return;
+    } else if (!S.need_copy) {
+        return;
+    }
     const size_t n3 = 3 * a.N, off = (size_t)rhs * n3;
     const float4 *src = reinterpret_cast<const float4 *>((dir ? a.pmin : a.p) + off);
     float4 *dst = reinterpret_cast<float4 *>((dir ? a.p : a.pmin) + off);
@@ -570,9 +600,10 @@ cudaError_t launch_field_op(int op, const FieldArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-cudaError_t launch_inc_tables(const FieldArgs &a, float2 *tab, cudaStream_t st)
+cudaError_t launch_inc_tables(const FieldArgs &a, float2 *tab, cudaStream_t st, int *active, double err_max,
+                              const int *nact)
 {
-    inc_tables<<<a.nrhs, 256, 0, st>>>(a, tab);
+    inc_tables<<<a.nrhs, 256, 0, st>>>(a, tab, active, err_max, nact);
     return cudaGetLastError();
 }
 
@@ -592,6 +623,49 @@ cudaError_t launch_scalar(RhsState *st_, const int *act_in, int *act_out, int nr
     return cudaGetLastError();
 }
 
+// Start of a recorded step in one launch (the host loop's SC_START, SC_TOP and loop test,
+// dda_func.cpp:1280-1313): with `start`, after step 0, the best iterate is step 0 and the step 1;
+// otherwise the step advances.  Then every right-hand side's convergence test and best-iterate
+// bookkeeping, and the loop condition.  One block; as separate launches (five after step 0, three
+// per iteration) they were most of a small lattice's solve.
+__global__ void __launch_bounds__(256) step_top(RhsState *st, int *active, int nrhs, int *step_dev, int start,
+                                                int max_step, cudaGraphConditionalHandle h)
+{
+    __shared__ int any;
+    const int step = start ? 1 : *step_dev + 1;
+    if (threadIdx.x == 0) any = 0;
+    __syncthreads();
+    int mine = 0;
+    for (int r = threadIdx.x; r < nrhs; r += blockDim.x) {
+        RhsState &S = st[r];
+        if (active[r]) {
+            for (int k = 0; k < kAcc; k++) S.acc[k] = 0.0;
+            if (start) {
+                S.err_min = S.err;
+                S.step_min = 0;
+                S.steps = 0;
+                S.restored = 0;
+            }
+            step_test(S, step, max_step);
+            active[r] = S.active;
+        }
+        mine |= active[r] != 0;
+    }
+    if (mine) atomicOr(&any, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *step_dev = step;
+        cudaGraphSetConditional(h, (any && step <= max_step) ? 1u : 0u);
+    }
+}
+
+cudaError_t launch_step_top(RhsState *st_, int *active, int nrhs, int *step_dev, int start, int max_step,
+                            cudaGraphConditionalHandle h, cudaStream_t st)
+{
+    step_top<<<1, 256, 0, st>>>(st_, active, nrhs, step_dev, start, max_step, h);
+    return cudaGetLastError();
+}
+
 // Last kernel of one iteration of a solve recorded in a CUDA graph, after the convergence
 // test of the next step: keep looping while some right-hand side is active and the step
 // has not passed Max_Step (the host loop's test, dda_func.cpp:1301-1313).
@@ -608,21 +682,11 @@ __global__ void __launch_bounds__(256) loop_control(const int *active, int nrhs,
     if (threadIdx.x == 0) cudaGraphSetConditional(h, (any && *step_dev <= max_step) ? 1u : 0u);
 }
 
-// ++*step_dev, or *step_dev = value
-__global__ void step_advance(int *step_dev, int set, int value)
-{
-    *step_dev = set ? value : *step_dev + 1;
-}
+__global__ void step_advance(int *step_dev) { ++*step_dev; }
 
 cudaError_t launch_step_advance(int *step_dev, cudaStream_t st)
 {
-    step_advance<<<1, 1, 0, st>>>(step_dev, 0, 0);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_step_set(int *step_dev, int value, cudaStream_t st)
-{
-    step_advance<<<1, 1, 0, st>>>(step_dev, 1, value);
+    step_advance<<<1, 1, 0, st>>>(step_dev);
     return cudaGetLastError();
 }
 
@@ -632,13 +696,7 @@ __global__ void init_state(RhsState *st, int *active, int nrhs, double err_max, 
 {
     const int rhs = blockIdx.x * blockDim.x + threadIdx.x;
     if (rhs >= nrhs) return;
-    RhsState S;
-    memset(&S, 0, sizeof S);
-    S.err_max = err_max;
-    S.active = 1;
-    S.nact = nact[rhs];
-    st[rhs] = S;
-    active[rhs] = 1;
+    fresh_state(st[rhs], active[rhs], err_max, nact[rhs]);
 }
 
 cudaError_t launch_init_state(RhsState *st_, int *active, int nrhs, double err_max, const int *nact,

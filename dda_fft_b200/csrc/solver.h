@@ -45,7 +45,9 @@ struct FieldArgs {
 cudaError_t launch_field_op(int op, const FieldArgs &a, cudaStream_t st);
 cudaError_t launch_first_approx(const FieldArgs &a, cudaStream_t st);
 // phase tables [nrhs][nj + nl + ni] of the incident field (y, z, x), the values first_approx uses
-cudaError_t launch_inc_tables(const FieldArgs &a, float2 *tab, cudaStream_t st);
+// nact (may be null): the solver state of every right-hand side is set up too (launch_init_state)
+cudaError_t launch_inc_tables(const FieldArgs &a, float2 *tab, cudaStream_t st, int *active = nullptr,
+                              double err_max = 0.0, const int *nact = nullptr);
 // step_dev (may be null): read the step number from device memory; `step` then holds
 // Max_Step, past which SC_TOP only clears the copy flag
 cudaError_t launch_scalar(RhsState *st_, const int *act_in, int *act_out, int nrhs, int stage,
@@ -55,9 +57,13 @@ cudaError_t launch_scalar(RhsState *st_, const int *act_in, int *act_out, int nr
 cudaError_t launch_loop_control(const int *active, int nrhs, const int *step_dev, int max_step,
                                 cudaGraphConditionalHandle h, cudaStream_t st);
 cudaError_t launch_step_advance(int *step_dev, cudaStream_t st);
-cudaError_t launch_step_set(int *step_dev, int value, cudaStream_t st);
+// start of a step of a recorded solve: SC_START (start != 0), SC_TOP, the step counter and the loop
+// condition in one launch
+cudaError_t launch_step_top(RhsState *st_, int *active, int nrhs, int *step_dev, int start, int max_step,
+                            cudaGraphConditionalHandle h, cudaStream_t st);
 cudaError_t launch_init_state(RhsState *st_, int *active, int nrhs, double err_max, const int *nact,
                               cudaStream_t st);
+// dir 0: p -> p_min, 1: p_min -> p where need_copy is set; 2: SC_FINAL and its rollback
 cudaError_t launch_gated_copy(const FieldArgs &a, int dir, cudaStream_t st);
 
 // refinement passes: 0 x64 = b; 1 r = b - (x64 - alpha conv) with conv in w, error into
