@@ -153,6 +153,7 @@ struct ddagpu_ctx {
     size_t worm_bytes = 0;
     int wait_selftest = 0;           // 1: the x pass's wait waits for a phase nothing completes
     long long post_key = 0;          // shape of the post-processing recorded with a solve
+    ddagpu::Segments results{};      // results a recorded solve's last kernel writes to the pinned block
     // far field by kz groups: the plan of the directions last uploaded, its device tables
     ddagpu::KzPlan kz;
     int ff_mode = 0;                 // ddagpu_set_farfield_mode
@@ -365,6 +366,7 @@ struct SolveResult {
     std::vector<RhsState> st;
     std::vector<double> trace;
     int matvec0 = 0, matvec_it = 0;
+    bool results_in = false;   // a recorded solve has written the results to the pinned block
 };
 
 // The whole solve of a batch as graph nodes: step 0, the iterations as a conditional
@@ -469,10 +471,20 @@ int record_whole_solve(ddagpu_ctx *c, cudaGraph_t g, int nrhs, int max_step, flo
     if (e != cudaSuccess) return give_up(DDAGPU_OK, e, "tail capture");
     e = launch_gated_copy(F, 2, st);
     if (e == cudaSuccess) rc = post();
+    if (rc == DDAGPU_OK && e == cudaSuccess) {
+        // the results, the solver states, the last step and the wait flag in one kernel that writes
+        // the pinned block: as copies they followed each other at 6 us apiece
+        Segments seg = c->results;
+        PinnedSolve *P = pin_solve(c);
+        seg.add(P->states(), c->state, nrhs * sizeof(RhsState));
+        seg.add(&P->last, c->step_dev, sizeof(int));
+        seg.add(&P->werr, c->err_dev, sizeof(int));
+        e = launch_segments(seg, st);
+    }
     if (rc != DDAGPU_OK || e != cudaSuccess) return give_up(rc, e, "tail");
     e = cudaStreamEndCapture(st, &t);
     if (e != cudaSuccess) return give_up(DDAGPU_OK, e, "end tail capture");
-    const long long n_tail = c->launches - l2 + 1;
+    const long long n_tail = c->launches - l2 + 2;
     n_fixed = n_head + n_tail;
     n_per_iter = n_body;
     c->launches = l_save;
@@ -486,10 +498,8 @@ int read_whole_solve(ddagpu_ctx *c, int nrhs, SolveResult &res, long long n_fixe
 {
     cudaStream_t st = c->st;
     PinnedSolve *P = pin_solve(c);
-    CK(cudaMemcpyAsync(P->states(), c->state, nrhs * sizeof(RhsState), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&P->last, c->step_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&P->werr, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    res.results_in = true;
     res.st.assign(P->states(), P->states() + nrhs);
     RET(device_wait_error(c, P->werr));
     c->launches += n_fixed + (long long)(P->last - 1) * n_per_iter;
@@ -1494,7 +1504,10 @@ struct OccBatch {
 int ensure_pin(ddagpu_ctx *c, size_t bytes)
 {
     if (bytes <= c->pin_bytes) return DDAGPU_OK;
-    if (c->pin) cudaFreeHost(c->pin);
+    if (c->pin) {
+        drop_graphs(c);   // recorded solves write their results there
+        cudaFreeHost(c->pin);
+    }
     c->pin = nullptr;
     c->pin_bytes = 0;
     CK(cudaHostAlloc((void **)&c->pin, ((bytes + 15) & ~(size_t)15) + PinnedSolve::bytes(c->cap), cudaHostAllocDefault));
@@ -1537,10 +1550,12 @@ int batch_chunk_finish(ddagpu_ctx *c, const BatchGeom &g, int no, const SolveRes
     const ChunkLayout Lc(no, g.ndir, g.nP, g.nA, g.nmat1);
     float *ca = (float *)(c->pin + Lc.o_ca), *ce = (float *)(c->pin + Lc.o_ce);
     double *mo = (double *)(c->pin + Lc.o_mo);
-    CK(cudaMemcpyAsync(ca, c->cabs, nr * sizeof(float), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(ce, c->cext, nr * sizeof(float), cudaMemcpyDeviceToHost, c->st));
-    if (mueller) CK(cudaMemcpyAsync(mo, c->mueller, Lc.n_mo * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
+    if (!res.results_in) {
+        CK(cudaMemcpyAsync(ca, c->cabs, nr * sizeof(float), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaMemcpyAsync(ce, c->cext, nr * sizeof(float), cudaMemcpyDeviceToHost, c->st));
+        if (mueller) CK(cudaMemcpyAsync(mo, c->mueller, Lc.n_mo * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+    }
     for (int o = 0; o < no; o++) {
         if (cabs) cabs[o] = 0.5 * ca[(size_t)2 * o] + 0.5 * ca[(size_t)2 * o + 1];
         if (cext) cext[o] = 0.5 * ce[(size_t)2 * o] + 0.5 * ce[(size_t)2 * o + 1];
@@ -1630,6 +1645,10 @@ int batch_chunk(ddagpu_ctx *c, const ddagpu_batch_cfg *cfg, const BatchGeom &g, 
         same = std::memcmp(al + (size_t)2 * o * nmat1, al + (size_t)(2 * o + 1) * nmat1,
                            nmat1 * sizeof(float2)) == 0;
     c->pair_step0 = same ? 1 : 0;
+    c->results = Segments{};
+    c->results.add(c->pin + Lc.o_ca, c->cabs, nr * sizeof(float));
+    c->results.add(c->pin + Lc.o_ce, c->cext, nr * sizeof(float));
+    c->results.add(c->pin + Lc.o_mo, c->mueller, Lc.n_mo * sizeof(double));
     const int rc = run_solver(c, nr, cfg->solver, cfg->tau, cfg->max_step, cfg->err_max, nmat1, d0, nact,
                               res, false, nullptr, nact_per, &post, rec);
     c->pair_step0 = 0;
@@ -1709,13 +1728,21 @@ int ddagpu_dda_fft(ddagpu_ctx *c, int iNoIllumination, int solver, float rTau, i
     SolveResult res;
     const std::function<int()> post = [&]() { return run_post(c, 1, nmat1, d0, ndir); };
     c->post_key = -1 - (long long)ndir;   // (batched calls' keys are positive)
+    c->results = Segments{};
+    if (again) {
+        c->results.add(es, c->esc, n_ks * 8);
+        c->results.add(cc, c->cabs, sizeof(float));
+        c->results.add(cc + 1, c->cext, sizeof(float));
+    }
     RET(run_solver(c, 1, solver, rTau, Max_Step, Error_max, nmat1, d0, nact, res, trace != nullptr, nullptr,
                    nullptr, again ? &post : nullptr, nullptr, true));
-    if (!again) RET(post());
-    if (ndir) CK(cudaMemcpyAsync(es, c->esc, n_ks * 8, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(cc, c->cabs, sizeof(float), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(cc + 1, c->cext, sizeof(float), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
+    if (!again) {
+        RET(post());
+        if (ndir) CK(cudaMemcpyAsync(es, c->esc, n_ks * 8, cudaMemcpyDeviceToHost, c->st));
+        CK(cudaMemcpyAsync(cc, c->cabs, sizeof(float), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaMemcpyAsync(cc + 1, c->cext, sizeof(float), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+    }
     if (ndir) std::memcpy(Esc, es, n_ks * 8);
     *rCabs = cc[0];
     *rCext = cc[1];
@@ -2128,14 +2155,20 @@ int ddagpu_mueller(ddagpu_ctx *c, const float *kinc, const float *einc0, const f
     for (int k = 0; k < nplanes * 3; k++) nv[k] = normals[k];
     std::memcpy(es, esc0, n_ks * sizeof(float));
     std::memcpy(es + n_ks, esc1, n_ks * sizeof(float));
-    CK(cudaMemcpyAsync(c->kinc, kd, 6 * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->einc, ed, 12 * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->ksc, ks, n_ks * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->normals, nv, (size_t)nplanes * 3 * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(c->esc, es, 2 * n_ks * sizeof(float), cudaMemcpyHostToDevice, c->st));
-    MuellerArgs m{1, nplanes, nangles, ndir, c->kinc, c->einc, c->ksc, c->normals, c->esc, c->mueller};
-    CK(launch_mueller(m, c->st));
-    CK(cudaMemcpyAsync(mo, c->mueller, n_mo * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    if (c->pin) {
+        // every value is read once: the kernel reads and writes the pinned block itself
+        MuellerArgs m{1, nplanes, nangles, ndir, kd, ed, ks, nv, reinterpret_cast<const float2 *>(es), mo};
+        CK(launch_mueller(m, c->st));
+    } else {
+        CK(cudaMemcpyAsync(c->kinc, kd, 6 * sizeof(double), cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpyAsync(c->einc, ed, 12 * sizeof(double), cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpyAsync(c->ksc, ks, n_ks * sizeof(double), cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpyAsync(c->normals, nv, (size_t)nplanes * 3 * sizeof(double), cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpyAsync(c->esc, es, 2 * n_ks * sizeof(float), cudaMemcpyHostToDevice, c->st));
+        MuellerArgs m{1, nplanes, nangles, ndir, c->kinc, c->einc, c->ksc, c->normals, c->esc, c->mueller};
+        CK(launch_mueller(m, c->st));
+        CK(cudaMemcpyAsync(mo, c->mueller, n_mo * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    }
     CK(cudaStreamSynchronize(c->st));
     for (size_t k = 0; k < n_mo; k++) out[k] = (float)mo[k];
     return DDAGPU_OK;

@@ -713,6 +713,19 @@ cudaError_t launch_loop_control(const int *active, int nrhs, const int *step_dev
     return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256) copy_segments(Segments s)
+{
+    for (int k = 0; k < s.n; k++)
+        for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < s.words[k]; q += (size_t)gridDim.x * blockDim.x)
+            s.dst[k][q] = s.src[k][q];
+}
+
+cudaError_t launch_segments(const Segments &s, cudaStream_t st)
+{
+    copy_segments<<<32, 256, 0, st>>>(s);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_gated_copy(const FieldArgs &a, int dir, cudaStream_t st)
 {
     // most right-hand sides copy nothing at a given step: a capped grid (grid-stride loop)

@@ -66,6 +66,23 @@ cudaError_t launch_init_state(RhsState *st_, int *active, int nrhs, double err_m
 // dir 0: p -> p_min, 1: p_min -> p where need_copy is set; 2: SC_FINAL and its rollback
 cudaError_t launch_gated_copy(const FieldArgs &a, int dir, cudaStream_t st);
 
+// Copies of up to 8 segments (sizes and addresses multiples of 4 bytes) in one kernel; either side
+// may be pinned host memory.
+struct Segments {
+    int n = 0;
+    const int *src[8];
+    int *dst[8];
+    size_t words[8];
+    void add(void *d, const void *s, size_t bytes)
+    {
+        if (!bytes) return;
+        src[n] = static_cast<const int *>(s);
+        dst[n] = static_cast<int *>(d);
+        words[n++] = bytes / 4;
+    }
+};
+cudaError_t launch_segments(const Segments &s, cudaStream_t st);
+
 // refinement passes: 0 x64 = b; 1 r = b - (x64 - alpha conv) with conv in w, error into
 // acc[0], inner rhs rb = float(r); 2 x64 += p; 3 p = float(x64); 4 p = rhs_in
 cudaError_t launch_refine(int op, const FieldArgs &a, cudaStream_t st);
