@@ -149,7 +149,7 @@ struct ddagpu_ctx {
     int single_seen = 0;             // the third is recorded
     int *nact_dev = nullptr;         // [cap] active cells per right-hand side
     int *err_dev = nullptr;          // set by a kernel whose bounded wait gave up
-    void *worm_buf = nullptr;        // monomers of the realisation being rasterised
+    void *worm_buf = nullptr;        // monomers and tile lists of the realisations being rasterised
     size_t worm_bytes = 0;
     int wait_selftest = 0;           // 1: the x pass's wait waits for a phase nothing completes
     long long post_key = 0;          // shape of the post-processing recorded with a solve
@@ -1461,24 +1461,18 @@ int agglomerate_rasterize(ddagpu_ctx *c, const BatchGeom &g, const float *monome
                           const std::vector<size_t> &first, int r0, int no, int *ndip,
                           std::vector<int> &nact)
 {
-    const size_t N = c->N;
-    for (int k = 0; k < no; k++) {
-        const int r = r0 + k;
-        const size_t need = anthrax_scratch_bytes(counts[r]);
-        if (need > c->worm_bytes) {   // grow the context's monomer buffer (stream-ordered)
-            CK(cudaStreamSynchronize(c->st));
-            cudaFree(c->worm_buf);
-            c->worm_buf = nullptr;
-            c->worm_bytes = 0;
-            CK(cudaMalloc(&c->worm_buf, need));
-            c->worm_bytes = need;
-        }
-        CK(anthrax_rasterize(monomers + 13 * first[(size_t)r], counts[r], c->ni, c->nj, c->nl,
-                             c->occ_b + 2 * k * N, c->ndip + k, c->st, c->worm_buf, c->worm_bytes));
-        CK(cudaMemcpyAsync(c->occ_b + (2 * k + 1) * N, c->occ_b + 2 * k * N, N,
-                           cudaMemcpyDeviceToDevice, c->st));
-        c->launches += 1;
+    const size_t need = anthrax_batch_scratch(c->ni, c->nj, c->nl, no, first[(size_t)r0 + no] - first[(size_t)r0]);
+    if (need > c->worm_bytes) {   // grow the context's scratch (stream-ordered)
+        CK(cudaStreamSynchronize(c->st));
+        cudaFree(c->worm_buf);
+        c->worm_buf = nullptr;
+        c->worm_bytes = 0;
+        CK(cudaMalloc(&c->worm_buf, need));
+        c->worm_bytes = need;
     }
+    CK(anthrax_rasterize_batch(monomers + 13 * first[(size_t)r0], counts + r0, no, c->ni, c->nj, c->nl, c->occ_b,
+                               c->ndip, c->st, c->worm_buf));
+    c->launches += 2;
     std::vector<int> nd((size_t)no, 0);
     CK(cudaMemcpyAsync(nd.data(), c->ndip, no * sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));

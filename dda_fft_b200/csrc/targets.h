@@ -13,6 +13,11 @@ size_t anthrax_scratch_bytes(int count);
 cudaError_t anthrax_rasterize(const float *cyl13, int count, int ni, int nj, int nl,
                               signed char *occ_dev, int *ndip_dev, cudaStream_t st,
                               void *scratch = nullptr, size_t scratch_bytes = 0);
+// no realisations (monomer lists one after the other in cyl13) into occ_dev [2 no][N], each at 2k
+// and 2k + 1 (both polarisations), and their dipole counts; scratch holds anthrax_batch_scratch bytes
+size_t anthrax_batch_scratch(int ni, int nj, int nl, int no, size_t total);
+cudaError_t anthrax_rasterize_batch(const float *cyl13, const int *counts, int no, int ni, int nj, int nl,
+                                    signed char *occ_dev, int *ndip_dev, cudaStream_t st, void *scratch);
 
 int random_ellipsoid_seeds(unsigned long long *state, int ni, int nj, int nl, float b_a, float c_a,
                            int nseeds, float *seeds3);

@@ -201,3 +201,32 @@ def test_realizations_far_field_by_kz_groups(D, oracle):
         o = orientation_solves(oracle, n, x, mats, 1, occ=occ, nplanes=12, theta_step=5.0,
                                err_max=1e-4, max_step=60)
         check(res[2], k, o)
+
+
+@pytest.mark.parametrize("grid,counts", [((8, 8, 8), (1, 64, 65, 300)), ((4, 16, 32), (2, 300)),
+                                         ((32, 32, 32), (40, 65, 700))])
+def test_batched_rasterisation_equals_single(D, grid, counts):
+    """Monomers of all radii and lengths, some reaching out of the lattice, in one tile, across
+    tiles and in tile lists below, at and above their capacity: the batch fills the cells that
+    the rasterisation of each realisation alone fills (counts exact; the solves on them agree to
+    the rounding of their sums, 1e-5)."""
+    rng = np.random.default_rng(5)
+    mons = []
+    for c in counts:
+        m = np.zeros((c, 13), np.float32)
+        m[:, 0] = rng.uniform(0.4, 0.3 * min(grid) + 0.5, c)
+        m[:, 1] = rng.uniform(0.0, 0.5 * max(grid), c)
+        m[:, 2:5] = rng.uniform(-0.5, 0.5, (c, 3)) * np.array(grid)
+        m[0, 0:5] = (1.2, 1.0, 0.1, 0.2, 0.3)   # every realisation fills a cell
+        a = rng.normal(size=(c, 3))
+        m[:, 8:11] = a / np.linalg.norm(a, axis=1, keepdims=True)
+        m[:, 5:8] = m[:, 2:5] + m[:, 1:2] * m[:, 8:11]
+        mons.append(m)
+    single = [D.Agglomerate.rasterize(grid, m) for m in mons]
+    cfg = D.BatchConfig(occ=None, materials=[(1.4, 0.01)], err_max=1e-4, max_step=40)
+    with D.Context(grid, 0.2, max_rhs=2 * len(counts)) as ctx:
+        g = ctx.agglomerate_solves(cfg, mons)
+        h = ctx.realization_solves(cfg, np.stack([o for o, _ in single]))
+    assert list(g["ndip"]) == [n for _, n in single]
+    for q in ("cabs", "cext"):
+        np.testing.assert_allclose(g[q], h[q], rtol=1e-5)
