@@ -873,9 +873,11 @@ int count_active(const signed char *occ, size_t N, const int *mv, int nmat1)
 
 int check_occ(const signed char *occ, size_t N, int nmat1)
 {
-    for (size_t q = 0; q < N; q++)
-        if ((int)occ[q] < 0 || (int)occ[q] >= nmat1)
-            return fail(DDAGPU_EINVAL, "cAlpha holds a material index outside 0..n_mat");
+    // the largest index as an unsigned byte (negative ones are 128 and above)
+    unsigned char top = 0;
+    for (size_t q = 0; q < N; q++) top = std::max(top, (unsigned char)occ[q]);
+    if ((signed char)top < 0 || (int)top >= nmat1)
+        return fail(DDAGPU_EINVAL, "cAlpha holds a material index outside 0..n_mat");
     return DDAGPU_OK;
 }
 
@@ -2472,14 +2474,18 @@ int ddagpu_realization_solves(ddagpu_ctx *c, const ddagpu_batch_cfg *cfg, int n_
     std::vector<double> rots;
     for (int o0 = 0; o0 < n_real; o0 += per) {
         const int no = std::min(per, n_real - o0);
+        // the matvec's scratch is free between solves and larger than the occupancies
+        signed char *up = reinterpret_cast<signed char *>(c->work);
+        CK(cudaMemcpyAsync(up, occ + (size_t)o0 * N, (size_t)no * N, cudaMemcpyHostToDevice, c->st));
+        CK(launch_spread_occupancies(up, c->occ_b, N, no, c->mv, g.nmat1, c->ndip, c->st));
+        c->launches++;
+        std::vector<int> active((size_t)no);
+        CK(cudaMemcpyAsync(active.data(), c->ndip, no * sizeof(int), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
         nact.assign((size_t)2 * no, 0);
         for (int k = 0; k < no; k++) {
-            const signed char *src = occ + (size_t)(o0 + k) * N;
-            nact[2 * k] = nact[2 * k + 1] = count_active(src, N, g.mv.data(), g.nmat1);
+            nact[2 * k] = nact[2 * k + 1] = active[(size_t)k];
             if (nact[2 * k] == 0) return fail(DDAGPU_EINVAL, "a realisation has no active dipoles");
-            CK(cudaMemcpyAsync(c->occ_b + 2 * k * N, src, N, cudaMemcpyHostToDevice, c->st));
-            CK(cudaMemcpyAsync(c->occ_b + (2 * k + 1) * N, c->occ_b + 2 * k * N, N,
-                               cudaMemcpyDeviceToDevice, c->st));
         }
         batch_rotations(rot, o0, no, rots);
         OccBatch ob(c);

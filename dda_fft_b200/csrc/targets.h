@@ -18,6 +18,10 @@ cudaError_t anthrax_rasterize(const float *cyl13, int count, int ni, int nj, int
 size_t anthrax_batch_scratch(int ni, int nj, int nl, int no, size_t total);
 cudaError_t anthrax_rasterize_batch(const float *cyl13, const int *counts, int no, int ni, int nj, int nl,
                                     signed char *occ_dev, int *ndip_dev, cudaStream_t st, void *scratch);
+// occupancies src [no][N] to occ [2 no][N] (each twice) and their active cells to nact [no];
+// src and occ 16-byte aligned
+cudaError_t launch_spread_occupancies(const signed char *src, signed char *occ, size_t N, int no, const int *mv,
+                                      int nmat1, int *nact, cudaStream_t st);
 
 int random_ellipsoid_seeds(unsigned long long *state, int ni, int nj, int nl, float b_a, float c_a,
                            int nseeds, float *seeds3);

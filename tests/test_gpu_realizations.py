@@ -230,3 +230,29 @@ def test_batched_rasterisation_equals_single(D, grid, counts):
     assert list(g["ndip"]) == [n for _, n in single]
     for q in ("cabs", "cext"):
         np.testing.assert_allclose(g[q], h[q], rtol=1e-5)
+
+
+@pytest.mark.parametrize("grid", [2, 4, (16, 8, 32)])
+def test_realization_occupancies_reach_both_polarisations(D, grid):
+    """Occupancies of 8 cells (below one 16-byte group) and more, three materials of which one is
+    vacuum: each realisation equals the single-occupancy batch (1e-5, both in FP32); a
+    realisation of vacuum only and an index out of range in a later chunk are refused."""
+    edges = (grid,) * 3 if isinstance(grid, int) else grid
+    rng = np.random.default_rng(2)
+    occs = rng.integers(0, 4, (5,) + edges).astype(np.int8)
+    occs[:, 0, 0, 0] = 3
+    mats = [(1.4, 0.01), (1.0, 0.0), (1.6, 0.1)]
+    cfg = dict(materials=mats, err_max=1e-4, max_step=40)
+    rot = D.mc_rotations(3, len(occs))
+    with D.Context(grid, 0.3, max_rhs=4) as ctx:
+        r = ctx.realization_solves(D.BatchConfig(occ=None, **cfg), occs, rot)
+        for k, occ in enumerate(occs):
+            s = ctx.orientation_solves(D.BatchConfig(occ=occ, **cfg), rot[k:k + 1])
+            for q in ("cabs", "cext"):
+                np.testing.assert_allclose(r[q][k], s[q][0], rtol=1e-5)
+        for bad in (2, 4, -1):
+            wrong = occs.copy()
+            wrong[4] = 2 if bad == 2 else wrong[4]
+            wrong[4, -1, -1, -1] = bad
+            with pytest.raises(D.DDAGPUError):
+                ctx.realization_solves(D.BatchConfig(occ=None, **cfg), wrong, rot)
