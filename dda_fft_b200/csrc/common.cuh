@@ -11,6 +11,16 @@
 
 #define DDA_DEV __device__ __forceinline__
 
+// First statement of a kernel launched by launch_chained: lets the next kernel of the stream take
+// the places that this one's last wave leaves free, and waits for the end (and the writes) of
+// the kernel before it.  Every block passes here, so a kernel that has ended has seen all
+// earlier ones end.  Without effect after a plain launch.
+DDA_DEV void chain_enter()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 DDA_DEV float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 DDA_DEV float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 DDA_DEV float2 cmul(float2 a, float2 b)

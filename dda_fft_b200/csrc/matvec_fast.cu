@@ -57,6 +57,9 @@ cudaError_t launch_matvec_fast(const MatvecArgs &args, cudaStream_t st)
     if (args.fx >= 9 && args.L.nl >= 8 && !args.tmaps) return cudaErrorInvalidValue;   // no tensor maps for the TMA variants
     MatvecArgs a = args;
     a.zs = matvec_z_split(a.L.nj, a.L.nl);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaError_t e = cudaStreamIsCapturing(st, &cap)) return e;
+    a.chained = cap == cudaStreamCaptureStatusNone;
     cudaError_t e = yz(a, 1, st);
     if (e != cudaSuccess) return e;
     switch (a.L.ni) {

@@ -215,6 +215,7 @@ k2q(MatvecArgs a, const __grid_constant__ CUtensorMap tmap)
     extern __shared__ __align__(128) float4 Bq[];   // [3][2][NI][XC]
     constexpr bool rhs_fast = k2_rhs_fastest(NI);
     const int js = rhs_fast ? blockIdx.z : blockIdx.x, rhs = rhs_fast ? blockIdx.x : blockIdx.z;
+    chain_enter();
     if (a.rhs_active && !a.rhs_active[rhs]) return;
     const int nj = a.L.nj, nl = a.L.nl, z0 = blockIdx.y * XC;
     const int t = threadIdx.x % XC, sub = threadIdx.x / XC, col = z0 + t;
@@ -349,6 +350,7 @@ __global__ void __launch_bounds__(Sx<NI>::RM * TL, 512 / (Sx<NI>::RM * TL)) k2f(
     extern __shared__ __align__(128) float2 B[];   // [6][NI][TL]
     constexpr bool rhs_fast = k2_rhs_fastest(NI);
     const int js = rhs_fast ? blockIdx.z : blockIdx.x, rhs = rhs_fast ? blockIdx.x : blockIdx.z;
+    chain_enter();
     if (a.rhs_active && !a.rhs_active[rhs]) return;
     const int nj = a.L.nj, nl = a.L.nl;
     const int l0 = blockIdx.y * TL;
@@ -485,6 +487,7 @@ __global__ void __launch_bounds__(Sx<NI>::RM * TL, pair_min_blocks<NI>() * XC / 
     extern __shared__ __align__(128) float4 Bq[];   // [3][2][NI][TL]
     constexpr bool rhs_fast = k2_rhs_fastest(NI);
     const int js = rhs_fast ? blockIdx.z : blockIdx.x, rhs0 = 2 * (rhs_fast ? blockIdx.x : blockIdx.z);
+    chain_enter();
     if (a.rhs_active && !a.rhs_active[rhs0]) return;
     const int nj = a.L.nj, nl = a.L.nl, t = threadIdx.x % TL, sub = threadIdx.x / TL, col = blockIdx.y * TL + t;
     const size_t plane = (size_t)(2 * nj) * (2 * nl), cstr = (size_t)NI * plane, off = (size_t)js * (2 * nl) + col;
@@ -589,19 +592,20 @@ __global__ void __launch_bounds__(Sx<NI>::RM * TL, pair_min_blocks<NI>() * XC / 
 
 // ---- launches
 template <int NI, int LD>
-void launch_packed(const MatvecArgs &a, cudaStream_t st)
+cudaError_t launch_packed(const MatvecArgs &a, cudaStream_t st)
 {
     const unsigned ct = (unsigned)((a.L.nl + XC - 1) / XC), js = 2 * a.L.nj;
     static const CUtensorMap none{};
     const CUtensorMap &map = LD == 2 ? *static_cast<const CUtensorMap *>(a.tmaps) : none;
-    k2q<NI, LD><<<k2_rhs_fastest(NI) ? dim3(a.nrhs, ct, js) : dim3(js, ct, a.nrhs), Sx<NI>::RM * XC,
-                  6 * NI * XC * sizeof(float4), st>>>(a, map);
+    return launch_chained(a.chained, k2q<NI, LD>, k2_rhs_fastest(NI) ? dim3(a.nrhs, ct, js) : dim3(js, ct, a.nrhs),
+                          Sx<NI>::RM * XC, 6 * NI * XC * sizeof(float4), st, 1, a, map);
 }
 
 template <int TL>
-void launch_unpacked(const MatvecArgs &a, cudaStream_t st)
+cudaError_t launch_unpacked(const MatvecArgs &a, cudaStream_t st)
 {
-    k2f<64, TL><<<dim3(2 * a.L.nj, 2 * a.L.nl / TL, a.nrhs), Sx<64>::RM * TL, (size_t)6 * 64 * TL * sizeof(float2), st>>>(a);
+    return launch_chained(a.chained, k2f<64, TL>, dim3(2 * a.L.nj, 2 * a.L.nl / TL, a.nrhs), Sx<64>::RM * TL,
+                          (size_t)6 * 64 * TL * sizeof(float2), st, 1, a);
 }
 
 // columns per CTA of the pair form: whole 128-byte lines where two CTAs of that size fit an SM's
@@ -611,37 +615,35 @@ template <int NI>
 constexpr int pair_columns() { return NI <= 32 ? 16 : 8; }
 
 template <int NI, int TL>
-void launch_pair(const MatvecArgs &a, cudaStream_t st)
+cudaError_t launch_pair(const MatvecArgs &a, cudaStream_t st)
 {
     const unsigned ct = 2 * a.L.nl / TL, js = 2 * a.L.nj, np = a.nrhs / 2;
-    k2r<NI, TL><<<k2_rhs_fastest(NI) ? dim3(np, ct, js) : dim3(js, ct, np), Sx<NI>::RM * TL,
-                  (size_t)6 * NI * TL * sizeof(float4), st>>>(a);
+    return launch_chained(a.chained, k2r<NI, TL>, k2_rhs_fastest(NI) ? dim3(np, ct, js) : dim3(js, ct, np),
+                          Sx<NI>::RM * TL, (size_t)6 * NI * TL * sizeof(float4), st, 1, a);
 }
 
 // x variants: 0..2 the unpacked form with 32 / 16 / 8 columns at edge 64 (packed with register
 // loads elsewhere); the packed form with bulk copies of the rows (3..5), register loads (6..8)
 // or one TMA tensor tile per component (9..11; register loads where a row is shorter)
 template <int NI>
-void launch_x(const MatvecArgs &a, cudaStream_t st)
+cudaError_t launch_x(const MatvecArgs &a, cudaStream_t st)
 {
     if (a.inc && a.pair) {
-        if (2 * a.L.nl >= pair_columns<NI>()) launch_pair<NI, pair_columns<NI>()>(a, st);
-        else launch_pair<NI, 8>(a, st);
-        return;
+        if (2 * a.L.nl >= pair_columns<NI>()) return launch_pair<NI, pair_columns<NI>()>(a, st);
+        return launch_pair<NI, 8>(a, st);
     }
     if constexpr (NI == 64) {
         if (a.fx < 3) {
             // the widest tile of the variant that the row holds
             const int tl = 32 >> a.fx;
-            if (tl >= 32 && 2 * a.L.nl >= 32) launch_unpacked<32>(a, st);
-            else if (tl >= 16 && 2 * a.L.nl >= 16) launch_unpacked<16>(a, st);
-            else launch_unpacked<8>(a, st);
-            return;
+            if (tl >= 32 && 2 * a.L.nl >= 32) return launch_unpacked<32>(a, st);
+            if (tl >= 16 && 2 * a.L.nl >= 16) return launch_unpacked<16>(a, st);
+            return launch_unpacked<8>(a, st);
         }
     }
-    if (a.fx >= 9 && a.L.nl >= XC) launch_packed<NI, 2>(a, st);
-    else if (a.fx >= 3 && a.fx < 6) launch_packed<NI, 1>(a, st);
-    else launch_packed<NI, 0>(a, st);
+    if (a.fx >= 9 && a.L.nl >= XC) return launch_packed<NI, 2>(a, st);
+    if (a.fx >= 3 && a.fx < 6) return launch_packed<NI, 1>(a, st);
+    return launch_packed<NI, 0>(a, st);
 }
 
 template <int NI>
@@ -673,8 +675,7 @@ cudaError_t x_prepare<X_NI>() { return prep_x<X_NI>(); }
 template <>
 cudaError_t x_launch<X_NI>(const MatvecArgs &a, cudaStream_t st)
 {
-    launch_x<X_NI>(a, st);
-    return cudaGetLastError();
+    return launch_x<X_NI>(a, st);
 }
 
 }  // namespace ddagpu

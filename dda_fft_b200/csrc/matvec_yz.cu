@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(NT, Yz<NJ, NL, NT, MB>::MINB) k1p(MatvecArgs a
     extern __shared__ float4 S[];
     const int r = ZS > 1 ? blockIdx.x % ZS : 0, i = blockIdx.x / ZS, c = blockIdx.y;
     const int rhs = IM == 2 ? 2 * (int)blockIdx.z : (int)blockIdx.z;
+    chain_enter();
     if (a.rhs_active && !a.rhs_active[rhs]) return;
     const int ni = a.L.ni;
     // twiddles in the order the lanes read them: tz[k1 R2 + t2] = W_ML^(t2 k1), ty likewise for
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(NT, Yz<NJ, NL, NT, MB>::MINB) k1p(MatvecArgs a
                             const bool act = rt ? ((m & 1) ? mv1 : mv0) : ep.mv[m] != 0;
                             float2 val = czero();
                             if (act) {
-                                val = cmul(cmul(txy, __ldg(&pt[NJ + l])), rt ? ((m & 1) ? al1 : al0) : al[m]);
+                                val = cmul(cmul(txy, pt[NJ + l]), rt ? ((m & 1) ? al1 : al0) : al[m]);
                                 if (IM == 1) val = cmul(val, Ef);
                             }
                             if (b == r) {
@@ -336,6 +337,7 @@ __global__ void __launch_bounds__(NT, Yz<NJ, NL, NT, MB>::MINB) k3p(MatvecArgs a
     constexpr int ZS = Y::ZS, ML = Y::ML;
     extern __shared__ float4 S[];
     const int r = ZS > 1 ? blockIdx.x % ZS : 0, i = blockIdx.x / ZS, c = blockIdx.y, rhs = blockIdx.z;
+    chain_enter();
     if (a.rhs_active && !a.rhs_active[rhs]) return;   // uniform over a cluster
     const int ni = a.L.ni;
     // twiddles in the order the lanes read them: tz[k1 R2 + t2] = W_ML^(t2 k1), ty likewise for
@@ -574,25 +576,11 @@ cudaError_t launch_yz_v(const MatvecArgs &a, int fwd, cudaStream_t st)
     constexpr int NT = yz_threads(V), MB = yz_blocks(V);
     using Y = Yz<NJ, NL, NT, MB>;
     const unsigned gx = Y::ZS * a.L.ni;
-    if (fwd && a.inc && a.pair) k1p<NJ, NL, NT, MB, 2><<<dim3(gx, 1, a.nrhs / 2), NT, Y::SMEM, st>>>(a);
-    else if (fwd && a.inc) k1p<NJ, NL, NT, MB, 1><<<dim3(gx, 3, a.nrhs), NT, Y::SMEM, st>>>(a);
-    else if (fwd) k1p<NJ, NL, NT, MB, 0><<<dim3(gx, 3, a.nrhs), NT, Y::SMEM, st>>>(a);
-    else if (Y::ZS == 1) k3p<NJ, NL, NT, MB><<<dim3(gx, 3, a.nrhs), NT, Y::SMEM, st>>>(a);
-    else {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(gx, 3, a.nrhs);
-        cfg.blockDim = dim3(NT);
-        cfg.dynamicSmemBytes = Y::SMEM;
-        cfg.stream = st;
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = Y::ZS;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k3p<NJ, NL, NT, MB>, a);
-    }
-    return cudaGetLastError();
+    const dim3 g3(gx, 3, a.nrhs), g1(gx, 1, a.nrhs / 2);
+    if (fwd && a.inc && a.pair) return launch_chained(a.chained, k1p<NJ, NL, NT, MB, 2>, g1, NT, Y::SMEM, st, 1, a);
+    if (fwd && a.inc) return launch_chained(a.chained, k1p<NJ, NL, NT, MB, 1>, g3, NT, Y::SMEM, st, 1, a);
+    if (fwd) return launch_chained(a.chained, k1p<NJ, NL, NT, MB, 0>, g3, NT, Y::SMEM, st, 1, a);
+    return launch_chained(a.chained, k3p<NJ, NL, NT, MB>, g3, NT, Y::SMEM, st, Y::ZS, a);
 }
 
 template <int NJ, int NL, int V>

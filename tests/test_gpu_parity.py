@@ -429,3 +429,25 @@ def test_batched_polarizability_models_vs_oracle(D, oracle, model, err_max, solv
     M, Mo = r["mueller"][0].reshape(-1, 16), o["mueller"].reshape(-1, 16)
     sig = np.abs(Mo) > 1e-3 * np.abs(Mo).max()
     assert (np.abs(M - Mo)[sig] / np.abs(Mo)[sig]).max() < 1e-4
+
+
+@pytest.mark.parametrize("grid,nrhs", [((4, 4, 4), 1), ((16, 16, 16), 2), ((8, 128, 64), 1), ((64, 64, 64), 2)])
+def test_products_in_flight_do_not_overtake(D, grid, nrhs):
+    """Products launched one into the other's end without a wait in between, each reading what the
+    one before wrote, equal the same chain with a synchronisation after every product (the same
+    kernels on the same inputs: bit for bit)."""
+    import torch
+    with D.Context(grid, 0.3, max_rhs=nrhs) as ctx:
+        x = torch.randn((nrhs, 3) + grid, dtype=torch.complex64, generator=torch.Generator().manual_seed(3)).cuda()
+        runs = []
+        for wait in (True, False):
+            f = [x.clone(), torch.empty_like(x), torch.empty_like(x)]
+            torch.cuda.synchronize()
+            for k in range(12):
+                ctx.convolution_dev(f[k % 3], f[(k + 1) % 3], nrhs, conj=k % 4 == 3)
+                if wait:
+                    torch.cuda.synchronize()
+            torch.cuda.synchronize()
+            runs.append([g.cpu().numpy() for g in f])
+    for a, b in zip(*runs):
+        np.testing.assert_array_equal(a, b)
