@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "internal.h"
 #include "fp64.h"
 
 namespace ddagpu {
@@ -153,8 +154,9 @@ __device__ __forceinline__ void step_a(double2 (&v)[Line<N>::R1], int t2, const 
 // Z: rows (c, i, j0 ..) of the field, forward along l.  Items of a block are spread over its
 // threads with the parity half fastest, so a warp's loads and stores are runs of the row.
 template <int N>
-__global__ void __launch_bounds__(kF) z_fwd(Mv64 a, const double2 *__restrict__ src)
+__global__ void __launch_bounds__(kF) z_fwd(Mv64 a, const double2 *src)
 {
+    chain_enter();
     using S = Line<N>;
     constexpr int R1 = S::R1, R2 = S::R2, G = S::ROWS;
     __shared__ double2 sm[G * 2 * S::LEN];
@@ -190,6 +192,7 @@ __global__ void __launch_bounds__(kF) z_fwd(Mv64 a, const double2 *__restrict__ 
 template <int N>
 __global__ void __launch_bounds__(kF) y_fwd(Mv64 a)
 {
+    chain_enter();
     using S = Line<N>;
     constexpr int R1 = S::R1, R2 = S::R2, TC = S::YC;
     __shared__ double2 sm[2][R1][R2][TC];
@@ -228,6 +231,7 @@ __global__ void __launch_bounds__(kF) y_fwd(Mv64 a)
 template <int N>
 __global__ void __launch_bounds__(kF) y_inv(Mv64 a)
 {
+    chain_enter();
     using S = Line<N>;
     constexpr int R1 = S::R1, R2 = S::R2, TC = S::YC;
     __shared__ double2 sm[2][R1][R2][TC];
@@ -269,6 +273,7 @@ __global__ void __launch_bounds__(kF) y_inv(Mv64 a)
 template <int N>
 __global__ void __launch_bounds__(kF) x_pass(Mv64 a)
 {
+    chain_enter();
     using S = Line<N>;
     constexpr int R1 = S::R1, R2 = S::R2, TC = S::XC;
     extern __shared__ double2 smd[];   // [3][2][R1][R2][TC]
@@ -356,8 +361,9 @@ __global__ void __launch_bounds__(kF) x_pass(Mv64 a)
 
 // ZI: rows (c, i, j0 ..), inverse along l, l < N kept, epilogue
 template <int N>
-__global__ void __launch_bounds__(kF) z_inv(Mv64 a, Ep64 ep, double2 *__restrict__ out)
+__global__ void __launch_bounds__(kF) z_inv(Mv64 a, Ep64 ep, double2 *out)
 {
+    chain_enter();
     using S = Line<N>;
     constexpr int R1 = S::R1, R2 = S::R2, G = S::ROWS;
     __shared__ double2 sm[G * 2 * S::LEN];
@@ -430,33 +436,28 @@ cudaError_t matvec64(const Mv64 &a, const Ep64 &ep, const double2 *src, double2 
     const int ni = a.ni, nj = a.nj, nl = a.nl;
     cudaError_t e = with_edge(nl, [&](auto n) {
         constexpr int N = decltype(n)::value;
-        z_fwd<N><<<dim3(nb(nj, Line<N>::ROWS), ni, 3), kF, 0, st>>>(a, src);
-        return cudaGetLastError();
+        return launch_chained(true, z_fwd<N>, dim3(nb(nj, Line<N>::ROWS), ni, 3), kF, 0, st, 1, a, src);
     });
     if (e == cudaSuccess)
         e = with_edge(nj, [&](auto n) {
             constexpr int N = decltype(n)::value;
-            y_fwd<N><<<dim3(nb(2 * nl, Line<N>::YC), ni, 3), kF, 0, st>>>(a);
-            return cudaGetLastError();
+            return launch_chained(true, y_fwd<N>, dim3(nb(2 * nl, Line<N>::YC), ni, 3), kF, 0, st, 1, a);
         });
     if (e == cudaSuccess)
         e = with_edge(ni, [&](auto n) {
             constexpr int N = decltype(n)::value;
             if (cudaError_t r = raise_smem_limit((const void *)x_pass<N>, (int)Line<N>::XSMEM)) return r;
-            x_pass<N><<<dim3(nb(2 * nl, Line<N>::XC), 2 * nj), kF, Line<N>::XSMEM, st>>>(a);
-            return cudaGetLastError();
+            return launch_chained(true, x_pass<N>, dim3(nb(2 * nl, Line<N>::XC), 2 * nj), kF, Line<N>::XSMEM, st, 1, a);
         });
     if (e == cudaSuccess)
         e = with_edge(nj, [&](auto n) {
             constexpr int N = decltype(n)::value;
-            y_inv<N><<<dim3(nb(2 * nl, Line<N>::YC), ni, 3), kF, 0, st>>>(a);
-            return cudaGetLastError();
+            return launch_chained(true, y_inv<N>, dim3(nb(2 * nl, Line<N>::YC), ni, 3), kF, 0, st, 1, a);
         });
     if (e == cudaSuccess)
         e = with_edge(nl, [&](auto n) {
             constexpr int N = decltype(n)::value;
-            z_inv<N><<<dim3(nb(nj, Line<N>::ROWS), ni, 3), kF, 0, st>>>(a, ep, out);
-            return cudaGetLastError();
+            return launch_chained(true, z_inv<N>, dim3(nb(nj, Line<N>::ROWS), ni, 3), kF, 0, st, 1, a, ep, out);
         });
     return e;
 }
@@ -758,6 +759,7 @@ __device__ __forceinline__ void bil_add(double &re, double &im, double2 a, doubl
 __global__ void __launch_bounds__(kT) two_dots(F64 f, const double2 *a, const double2 *b, const double2 *c,
                                                const double2 *d, double *acc)
 {
+    chain_enter();
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < f.N; q += (size_t)gridDim.x * blockDim.x) {
         if (!active(f, q)) continue;
@@ -774,6 +776,7 @@ __global__ void __launch_bounds__(kT) two_dots(F64 f, const double2 *a, const do
 __global__ void __launch_bounds__(kT) mixed_apply_dots(F64 f, const double2 *s, const float2 *conv, const double2 *r,
                                                        double2 *w, double *acc)
 {
+    chain_enter();
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < f.N; q += (size_t)gridDim.x * blockDim.x) {
         const int m = f.occ[q];
@@ -794,10 +797,11 @@ __global__ void __launch_bounds__(kT) mixed_apply_dots(F64 f, const double2 *s, 
     block_add<4>(v, acc);
 }
 
-// a = <r,s> / <s,w>: x -= a s; r -= a w on active cells; set[4..5] += sum r w, set[6] += sum |r|
-__global__ void __launch_bounds__(kT) cg_update(F64 f, double2 *x, double2 *r, const double2 *s, const double2 *w,
-                                                double *set)
+// a = <r,s> / <s,w>: x = x0 - a s (x0 may be x); r -= a w on active cells; set[4..5] += sum r w, set[6] += sum |r|
+__global__ void __launch_bounds__(kT) cg_update(F64 f, const double2 *x0, double2 *x, double2 *r, const double2 *s,
+                                                const double2 *w, double *set)
 {
+    chain_enter();
     const double2 a = ddiv(set_at(set, 2), set_at(set, 0));
     double v[3] = {0.0, 0.0, 0.0};
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < f.N; q += (size_t)gridDim.x * blockDim.x) {
@@ -806,7 +810,7 @@ __global__ void __launch_bounds__(kT) cg_update(F64 f, double2 *x, double2 *r, c
         for (int c = 0; c < 3; c++) {
             const size_t k = c * f.N + q;
             const double2 sv = s[k], wv = w[k];
-            x[k] = dsub(x[k], dmul(a, sv));
+            x[k] = dsub(x0[k], dmul(a, sv));
             const double2 rv = dsub(r[k], dmul(a, wv));
             r[k] = rv;
             bil_add(v[0], v[1], rv, wv);
@@ -818,10 +822,14 @@ __global__ void __launch_bounds__(kT) cg_update(F64 f, double2 *x, double2 *r, c
 }
 
 // b = <r,w> / <s,w>: s = r - b s on active cells (inactive cells keep their zeros); s32 (may
-// be null) = float(s)
-__global__ void cg_dir(F64 f, const double *set, const double2 *r, double2 *s, float2 *s32)
+// be null) = float(s).  Posts the step's residual sum to the host and clears the next set: a
+// copy and a clearing operation of their own between the kernels of a step cost 10 us
+__global__ void cg_dir(F64 f, const double *set, double *next, double *post, const double2 *r, double2 *s, float2 *s32)
 {
+    chain_enter();
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (q < kSet) next[q] = 0.0;
+    if (q == 0) *post = set[6];
     if (q >= f.N) return;
     const double2 b = ddiv(set_at(set, 4), set_at(set, 0));
     const bool act = active(f, q);
@@ -835,10 +843,14 @@ __global__ void cg_dir(F64 f, const double *set, const double2 *r, double2 *s, f
 }
 
 // BiCGStab (dda_func.cpp:1423-1469): la = rho / <g,h>, lw = <w,r> / <w,w> of a set
-// s = r + lb s - lb lw h, lb = (rho la1) / (rho1 lw1), from the new rho and the last set
-__global__ void bi_dir(F64 f, const double *last, const double *cur, const double2 *r, const double2 *h, double2 *s)
+// s = r + lb s - lb lw h, lb = (rho la1) / (rho1 lw1), from the new rho and the last set;
+// posts the last step's residual sum to the host (post may be null)
+__global__ void bi_dir(F64 f, const double *last, const double *cur, double *post, const double2 *r, const double2 *h,
+                       double2 *s)
 {
+    chain_enter();
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (post && q == 0) *post = last[8];
     if (q >= f.N) return;
     const double2 rho1 = set_at(last, 0), la = ddiv(rho1, set_at(last, 2)), lw = ddiv(set_at(last, 4), set_at(last, 6));
     const double2 lb = ddiv(dmul(set_at(cur, 0), la), dmul(rho1, lw)), c2 = dmul(lb, lw);
@@ -849,10 +861,12 @@ __global__ void bi_dir(F64 f, const double *last, const double *cur, const doubl
     }
 }
 
-// r -= la h on active cells
-__global__ void bi_r(F64 f, const double *set, const double2 *h, double2 *r)
+// r -= la h on active cells; clears the next set
+__global__ void bi_r(F64 f, const double *set, double *next, const double2 *h, double2 *r)
 {
+    chain_enter();
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (q < kSet) next[q] = 0.0;
     if (q >= f.N || !active(f, q)) return;
     const double2 la = ddiv(set_at(set, 0), set_at(set, 2));
     for (int c = 0; c < 3; c++) {
@@ -865,6 +879,7 @@ __global__ void bi_r(F64 f, const double *set, const double2 *h, double2 *r)
 __global__ void __launch_bounds__(kT) bi_update(F64 f, double *set, double *next, double2 *p, double2 *r,
                                                 const double2 *s, const double2 *w, const double2 *g)
 {
+    chain_enter();
     const double2 la = ddiv(set_at(set, 0), set_at(set, 2)), lw = ddiv(set_at(set, 4), set_at(set, 6));
     double e[1] = {0.0}, v[2] = {0.0, 0.0};
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < f.N; q += (size_t)gridDim.x * blockDim.x) {
@@ -940,8 +955,10 @@ cudaError_t KrylovScalars::zero(int k, cudaStream_t st) const
 cudaError_t KrylovScalars::send(const double *from, cudaStream_t st) const
 {
     const cudaError_t e = cudaMemcpyAsync(pin, from, sizeof(double), cudaMemcpyDeviceToHost, st);
-    return e == cudaSuccess ? cudaEventRecord(ready, st) : e;
+    return e == cudaSuccess ? sent(st) : e;
 }
+
+cudaError_t KrylovScalars::sent(cudaStream_t st) const { return cudaEventRecord(ready, st); }
 
 cudaError_t KrylovScalars::wait(double &v) const
 {
@@ -1066,25 +1083,31 @@ struct Fp64Run {
     }
     cudaError_t dots(const double2 *a, const double2 *b, const double2 *c, const double2 *d, double *acc)
     {
-        two_dots<<<4 * 148, kT, 0, st>>>(f, a, b, c, d, acc);
         *launches += 1;
-        return cudaGetLastError();
+        return launch_chained(true, two_dots, 4 * 148, kT, 0, st, 1, f, a, b, c, d, acc);
     }
-    // the rest of a BiCGStab step after h = A s: set cur holds its rho, next (zeroed here) the
-    // next step's; p, r updated and the residual sum sent to the host
+    // the rest of a BiCGStab step after h = A s: set cur holds its rho, next (cleared on the way)
+    // the next step's; p, r updated, the residual sum in set cur
     cudaError_t bicg_step(double2 *p, double2 *r, const double2 *s, const double2 *g, const double2 *h, double2 *w,
                           int cur, int next)
     {
         const KrylovScalars &K = B.scal;
         cudaError_t e = dots(g, h, nullptr, nullptr, K.set(cur) + 2);
         if (e) return e;
-        bi_r<<<nb(f.N, kT), kT, 0, st>>>(f, K.set(cur), h, r);
+        if ((e = launch_chained(true, bi_r, nb(f.N, kT), kT, 0, st, 1, f, K.set(cur), K.set(next), h, r))) return e;
         if ((e = matvec(r, w, 1.0, r, 0))) return e;
         if ((e = dots(w, r, w, w, K.set(cur) + 4))) return e;
-        if ((e = K.zero(next, st))) return e;
-        bi_update<<<4 * 148, kT, 0, st>>>(f, K.set(cur), K.set(next), p, r, s, w, g);
         *launches += 2;
-        return K.send(K.set(cur) + 8, st);
+        return launch_chained(true, bi_update, 4 * 148, kT, 0, st, 1, f, K.set(cur), K.set(next), p, r, s, w, g);
+    }
+    // a BiCGStab step's direction; post: the last step's residual sum goes to the host
+    cudaError_t bicg_dir(const double2 *r, const double2 *h, double2 *s, int last, int cur, bool post)
+    {
+        const KrylovScalars &K = B.scal;
+        *launches += 1;
+        const cudaError_t e = launch_chained(true, bi_dir, nb(f.N, kT), kT, 0, st, 1, f, K.set(last), K.set(cur),
+                                             post ? K.pin : nullptr, r, h, s);
+        return e == cudaSuccess && post ? K.sent(st) : e;
     }
     cudaError_t copy(double2 *dst, const double2 *src)
     {
@@ -1148,6 +1171,7 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
         CKE(X.dots(r, g, nullptr, nullptr, B.scal.set(0)));
         CKE(X.matvec(s, h, 1.0, s, 0));
         CKE(X.bicg_step(p, r, s, g, h, w, 0, 1));
+        CKE(B.scal.send(B.scal.set(0) + 8, st));
     }
     if (solver == 3) {
         CKE(X.copy(s, p));
@@ -1166,36 +1190,40 @@ cudaError_t solve_fp64(Fp64Buffers &B, const Fp64Problem &P, cudaStream_t st, Fp
     nt++;
     CKE(X.copy(pmin, p));
     const KrylovScalars &K = B.scal;
+    if (solver == 0) CKE(K.zero(1, st));   // CG steps alternate between sets 0 and 1, from 1
     bool ahead = false;   // the next step's first matvec is already in the stream
     for (int o = 1; o <= P.max_step; o++) {   // dda_func.cpp:1301-1535
         if (err <= P.err_max) break;
-        if (err < err_min) {
+        const bool best = err < err_min;
+        if (best) {
             err_min = err;
             step_min = o - 1;
-            CKE(X.copy(pmin, p));
+            // CG writes its next iterate to the other buffer; the two agree on inactive cells
+            if (solver == 0) std::swap(p, pmin);
+            else CKE(X.copy(pmin, p));
         }
         if (solver == 2) {
             if (!ahead) {
-                bi_dir<<<nb(N, kT), kT, 0, st>>>(f, K.set((o - 1) & 1), K.set(o & 1), r, h, s);
-                *launches += 1;
+                CKE(X.bicg_dir(r, h, s, (o - 1) & 1, o & 1, false));
                 CKE(X.matvec(s, h, 1.0, s, 0));
             }
             CKE(X.bicg_step(p, r, s, g, h, w, o & 1, (o + 1) & 1));
             // the next step's direction and first product run while the residual travels;
             // neither p nor r changes, so a step that turns out not to be needed costs nothing else
             if ((ahead = o < P.max_step)) {
-                bi_dir<<<nb(N, kT), kT, 0, st>>>(f, K.set(o & 1), K.set((o + 1) & 1), r, h, s);
-                *launches += 1;
+                CKE(X.bicg_dir(r, h, s, o & 1, (o + 1) & 1, true));
                 CKE(X.matvec(s, h, 1.0, s, 0));
+            } else {
+                CKE(K.send(K.set(o & 1) + 8, st));
             }
             CKE(K.wait(err));
         } else if (solver == 0) {
             if (!ahead) CKE(X.matvec(s, w, 1.0, s, 0));
-            CKE(K.zero(0, st));
-            CKE(X.dots(s, w, r, s, K.set(0)));
-            cg_update<<<4 * 148, kT, 0, st>>>(f, p, r, s, w, K.set(0));
-            CKE(K.send(K.set(0) + 6, st));
-            cg_dir<<<nb(N, kT), kT, 0, st>>>(f, K.set(0), r, s, nullptr);
+            double *set = K.set(o & 1), *next = K.set((o + 1) & 1);
+            CKE(X.dots(s, w, r, s, set));
+            CKE(launch_chained(true, cg_update, 4 * 148, kT, 0, st, 1, f, best ? pmin : p, p, r, s, w, set));
+            CKE(launch_chained(true, cg_dir, nb(N, kT), kT, 0, st, 1, f, set, next, K.pin, r, s, nullptr));
+            CKE(K.sent(st));
             *launches += 2;
             if ((ahead = o < P.max_step)) CKE(X.matvec(s, w, 1.0, s, 0));
             CKE(K.wait(err));
@@ -1330,11 +1358,11 @@ cudaError_t mixed_cg(MixedCgBuffers &B, const Field64View &f, const double2 *alp
     auto true_residual = [&](double &err) -> cudaError_t {
         to_f32<<<red, kT, 0, st>>>(B.x, x32, n3);
         CKE(conv(x32, conv32));
-        CKE(K.zero(1, st));
-        mixed_apply<<<red, kT, 0, st>>>(f, B.x, conv32, B.b, B.r, K.set(1));
+        CKE(K.zero(2, st));
+        mixed_apply<<<red, kT, 0, st>>>(f, B.x, conv32, B.b, B.r, K.set(2));
         *launches += 2;
         R.matvecs++;
-        CKE(K.send(K.set(1), st));
+        CKE(K.send(K.set(2), st));
         CKE(K.wait(err));
         err /= nact;
         return cudaSuccess;
@@ -1348,6 +1376,7 @@ cudaError_t mixed_cg(MixedCgBuffers &B, const Field64View &f, const double2 *alp
     double err_best = err, anchor = err;
     CKE(cudaMemcpyAsync(B.best, B.x, bytes, cudaMemcpyDeviceToDevice, st));
     if (err > err_max) {
+        CKE(K.zero(0, st));   // steps alternate between sets 0 and 1; set 2 is the true residual's
         CKE(cudaMemcpyAsync(B.s, B.r, bytes, cudaMemcpyDeviceToDevice, st));
         to_f32<<<red, kT, 0, st>>>(B.s, s32, n3);
         *launches += 1;
@@ -1358,12 +1387,12 @@ cudaError_t mixed_cg(MixedCgBuffers &B, const Field64View &f, const double2 *alp
             // w = A s (dda_func.cpp:1325-1357) and the dots of the step (1359-1371, without the
             // float casts); the residual travels to the host while the next convolution runs
             if (!ahead) CKE(conv(s32, conv32));
-            CKE(K.zero(0, st));
-            mixed_apply_dots<<<red, kT, 0, st>>>(f, B.s, conv32, B.r, B.w, K.set(0));
+            double *set = K.set(it & 1), *next = K.set((it + 1) & 1);
+            CKE(launch_chained(true, mixed_apply_dots, red, kT, 0, st, 1, f, B.s, conv32, B.r, B.w, set));
             R.matvecs++;
-            cg_update<<<red, kT, 0, st>>>(f, B.x, B.r, B.s, B.w, K.set(0));
-            CKE(K.send(K.set(0) + 6, st));
-            cg_dir<<<nb(N, kT), kT, 0, st>>>(f, K.set(0), B.r, B.s, s32);
+            CKE(launch_chained(true, cg_update, red, kT, 0, st, 1, f, B.x, B.x, B.r, B.s, B.w, set));
+            CKE(launch_chained(true, cg_dir, nb(N, kT), kT, 0, st, 1, f, set, next, K.pin, B.r, B.s, s32));
+            CKE(K.sent(st));
             *launches += 3;
             if ((ahead = it + 1 < cap)) CKE(conv(s32, conv32));
             double err_rec;

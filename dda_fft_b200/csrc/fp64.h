@@ -20,6 +20,7 @@ struct KrylovScalars {
     double *set(int k) const;
     cudaError_t zero(int k, cudaStream_t st) const;
     cudaError_t send(const double *from, cudaStream_t st) const;
+    cudaError_t sent(cudaStream_t st) const;   // what the stream holds so far posts to pin
     cudaError_t wait(double &v) const;
 };
 
