@@ -45,6 +45,11 @@ struct Yz {
     using SY = Split<NJ>;
     static constexpr int RG = SZ::R1 / SZ::R2;              // rows a lane group starts together
     static constexpr int ROWS = NT / SZ::R1 * RG;           // rows per pass of the block
+    // A warp loads whole rows (forward) where the R2 elements of a lane group are 32-byte runs of the
+    // field, eight lines per warp access; with that, without the next rows' prefetch where it
+    // spilled (ZS 4) and with at()'s row term k1p takes 321 instead of 398 us (128^3 x 4) and 70
+    // instead of 74 (32 x 128 x 64 x 6).  Longer runs (ML 64) gain nothing from the extra hop.
+    static constexpr bool WIDE = ZS > 1 && ML == 32;
     static constexpr int CW = 8;                            // columns of a lane group: 128-byte runs
     static constexpr int GT = CW * SY::R1;                  // its threads (1, 2 or 4 warps)
     static constexpr int GROUPS = NT / GT;
@@ -59,8 +64,13 @@ struct Yz {
     static constexpr int MINB = FIT < WANT ? (FIT < 1 ? 1 : FIT) : WANT;
 
     // Position of bin p of row `row`: within an aligned run of eight pairs (128 bytes) the order is
-    // permuted by p >> 3, as a row's lanes read runs of stride R2.
-    __device__ static int at(int row, int p) { return row * ML + (ML >= 8 ? p ^ ((p >> 3) & 7) : p); }
+    // permuted by p >> 3, as a row's lanes read runs of stride R2, and by the row where eight
+    // lanes access R2 < 8 pairs each of consecutive rows.
+    __device__ static int at(int row, int p)
+    {
+        constexpr int RR = SZ::R2 < 8 ? 8 / SZ::R2 : 1;
+        return row * ML + (ML >= 8 ? p ^ (((p >> 3) ^ (row % RR * SZ::R2)) & 7) : p);
+    }
     // barrier of one column group
     __device__ static void sync(int group)
     {
@@ -69,43 +79,39 @@ struct Yz {
     }
 };
 
-// One row's inputs x[b][rr] (element t2 + R2 rr + ML b) -> the pair line of rank r, v[rr]
-// (element t2 + R2 rr of ML): bins s = 2 r, 2 r + 1 (mod 2 ZS), v_s = W^(s l') sum_b W^(s ML b) x_b.
-template <int NL, int ZS, int R1, int R2>
-DDA_DEV void fold_rows(const float2 (&x)[ZS][R1], P2 (&v)[R1], int r, int t2, const float2 *__restrict__ fz)
+// One element's inputs x[b] (element l + ML b of the row) -> element l of the pair line of rank
+// r: bins s = 2 r, 2 r + 1 (mod 2 ZS), v_s = W^(s l) sum_b W^(s ML b) x_b.
+template <int NL, int ZS>
+DDA_DEV P2 fold(const float2 (&x)[ZS], int r, int l, const float2 *__restrict__ fz)
 {
     constexpr int ML = NL / ZS;
-#pragma unroll
-    for (int k = 0; k < R1; k++) {
-        const int l = t2 + R2 * k;
-        float2 h0, h1;
-        if constexpr (ZS == 1) {
-            h0 = x[0][k];
-            h1 = x[0][k];
-        } else if constexpr (ZS == 2) {
-            // W^ML = -i
-            const float2 a = x[0][k], b = x[1][k];
-            h0 = r ? csub(a, b) : cadd(a, b);
-            h1 = r ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, a.y - b.x);
-        } else {
-            // W^ML = exp(-i pi / 4)
-            const float2 s = cadd(x[0][k], x[2][k]), d = csub(x[0][k], x[2][k]);
-            const float2 q = cadd(x[1][k], x[3][k]), n = csub(x[1][k], x[3][k]);
-            const float sg = r & 2 ? -1.f : 1.f;
-            if (r & 1) h0 = make_float2(fmaf(sg, n.y, d.x), fmaf(-sg, n.x, d.y));   // d - sg i n
-            else h0 = make_float2(fmaf(sg, q.x, s.x), fmaf(sg, q.y, s.y));
-            // odd bin s = 2 r + 1: x0 -+ i x2 + w (x1 -+' i x3) with w = exp(-i pi s / 4)
-            const float sr = r & 1 ? -1.f : 1.f;   // (-1)^r: W^(2 s ML) = -i (-1)^r
-            const float2 a = make_float2(fmaf(sr, x[2][k].y, x[0][k].x), fmaf(-sr, x[2][k].x, x[0][k].y));
-            const float2 b = make_float2(fmaf(sr, x[3][k].y, x[1][k].x), fmaf(-sr, x[3][k].x, x[1][k].y));
-            const float2 w = __ldg(&fz[(2 * r + 1) * NL + ML]);
-            const float2 t = cmul(b, w);
-            h1 = cadd(a, t);
-        }
-        if (ZS > 1 && r) h0 = cmul(h0, __ldg(&fz[2 * r * NL + l]));
-        h1 = cmul(h1, __ldg(&fz[(2 * r + 1) * NL + l]));
-        v[k] = ppack(h0, h1);
+    float2 h0, h1;
+    if constexpr (ZS == 1) {
+        h0 = x[0];
+        h1 = x[0];
+    } else if constexpr (ZS == 2) {
+        // W^ML = -i
+        const float2 a = x[0], b = x[1];
+        h0 = r ? csub(a, b) : cadd(a, b);
+        h1 = r ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, a.y - b.x);
+    } else {
+        // W^ML = exp(-i pi / 4)
+        const float2 s = cadd(x[0], x[2]), d = csub(x[0], x[2]);
+        const float2 q = cadd(x[1], x[3]), n = csub(x[1], x[3]);
+        const float sg = r & 2 ? -1.f : 1.f;
+        if (r & 1) h0 = make_float2(fmaf(sg, n.y, d.x), fmaf(-sg, n.x, d.y));   // d - sg i n
+        else h0 = make_float2(fmaf(sg, q.x, s.x), fmaf(sg, q.y, s.y));
+        // odd bin s = 2 r + 1: x0 -+ i x2 + w (x1 -+' i x3) with w = exp(-i pi s / 4)
+        const float sr = r & 1 ? -1.f : 1.f;   // (-1)^r: W^(2 s ML) = -i (-1)^r
+        const float2 a = make_float2(fmaf(sr, x[2].y, x[0].x), fmaf(-sr, x[2].x, x[0].y));
+        const float2 b = make_float2(fmaf(sr, x[3].y, x[1].x), fmaf(-sr, x[3].x, x[1].y));
+        const float2 w = __ldg(&fz[(2 * r + 1) * NL + ML]);
+        const float2 t = cmul(b, w);
+        h1 = cadd(a, t);
     }
+    if (ZS > 1 && r) h0 = cmul(h0, __ldg(&fz[2 * r * NL + l]));
+    h1 = cmul(h1, __ldg(&fz[(2 * r + 1) * NL + l]));
+    return ppack(h0, h1);
 }
 
 // ------------------------------------------------------------------------------ K1
@@ -134,6 +140,11 @@ __global__ void __launch_bounds__(NT, Yz<NJ, NL, NT, MB>::MINB) k1p(MatvecArgs a
     {
         constexpr int R1 = Y::SZ::R1, R2 = Y::SZ::R2, RG = Y::RG;
         const int sub = threadIdx.x % R1, g = threadIdx.x / R1, ar = sub / R2, t2 = sub % R2;
+        // what load number k of a pass fetches: element t2 + R2 k of the lane's row, or, WIDE, element
+        // `lane` of row k of the warp's R1 rows (which it hands over through the plane)
+        static_assert(!Y::WIDE || (32 / R1 * RG == R1 && NJ % Y::ROWS == 0), "a warp's rows of a pass");
+        auto row_of = [&](int r0, int k) { return Y::WIDE ? r0 + (int)threadIdx.x / 32 * R1 + k : r0 + g * RG + ar; };
+        auto elem = [&](int k) { return Y::WIDE ? (int)threadIdx.x % 32 : t2 + R2 * k; };
         const float2 *src = a.src + (size_t)rhs * a.fstride + ((size_t)c * ni + i) * (NJ * NL);
         // incident field: ((x phase * y phase) * z phase) * alpha_m * E_c, the products of the
         // separate pass in its order (FirstApproximation, dda_func.cpp:654-689)
@@ -156,34 +167,37 @@ __global__ void __launch_bounds__(NT, Yz<NJ, NL, NT, MB>::MINB) k1p(MatvecArgs a
         const bool mv0 = IM && ep.mv[0] != 0, mv1 = IM && ep.nmat1 > 1 && ep.mv[1] != 0;
         const float2 al0 = IM ? al[0] : czero(), al1 = IM && ep.nmat1 > 1 ? al[1] : czero();
         float2 *pout = IM ? a.inc_out + (size_t)rhs * a.fstride + ((size_t)c * ni + i) * (NJ * NL) : nullptr;
-        auto load = [&](int row, float2 (&x)[ZS][R1], int (&o)[ZS][R1]) {
-            if (row >= NJ) return;
+        auto load = [&](int r0, float2 (&x)[R1][ZS], int (&o)[R1][ZS]) {
+            if (row_of(r0, 0) >= NJ) return;   // (a warp's rows are in the plane or all past it)
 #pragma unroll
-            for (int b = 0; b < ZS; b++)
+            for (int k = 0; k < R1; k++)
 #pragma unroll
-                for (int k = 0; k < R1; k++) {
-                    const int e = row * NL + t2 + R2 * k + ML * b;
-                    if (IM) o[b][k] = ob[e];
-                    else x[b][k] = src[e];
+                for (int b = 0; b < ZS; b++) {
+                    const int e = row_of(r0, k) * NL + elem(k) + ML * b;
+                    if (IM) o[k][b] = ob[e];
+                    else x[k][b] = src[e];
                 }
         };
-        float2 x[ZS][R1], xn[ZS][R1];
-        int o[ZS][R1], on[ZS][R1];
-        load(g * RG + ar, x, o);
+        float2 x[R1][ZS], xn[R1][ZS];
+        int o[R1][ZS], on[R1][ZS];
+        constexpr bool AHEAD = ZS < 4;   // (with four parts of a row both sets do not fit the registers)
+        if (AHEAD) load(0, x, o);
 #pragma unroll 1
         for (int r0 = 0; r0 < NJ; r0 += Y::ROWS) {
             const int row0 = r0 + g * RG, row = row0 + ar;
             const bool ok = row < NJ;
+            if (!AHEAD) load(r0, x, o);
             // the next pass's row is loaded while this one is transformed
-            if (r0 + Y::ROWS < NJ) load(row + Y::ROWS, xn, on);
+            if (AHEAD && r0 + Y::ROWS < NJ) load(r0 + Y::ROWS, xn, on);
             if (ok) {
                 if constexpr (IM != 0) {
-                    const float2 txy = cmul(tx, pt[row]);
 #pragma unroll
-                    for (int b = 0; b < ZS; b++)
+                    for (int k = 0; k < R1; k++) {
+                        const int rk = row_of(r0, k);
+                        const float2 txy = cmul(tx, pt[rk]);
 #pragma unroll
-                        for (int k = 0; k < R1; k++) {
-                            const int l = t2 + R2 * k + ML * b, m = o[b][k];
+                        for (int b = 0; b < ZS; b++) {
+                            const int l = elem(k) + ML * b, m = o[k][b];
                             const bool act = rt ? ((m & 1) ? mv1 : mv0) : ep.mv[m] != 0;
                             float2 val = czero();
                             if (act) {
@@ -191,7 +205,7 @@ __global__ void __launch_bounds__(NT, Yz<NJ, NL, NT, MB>::MINB) k1p(MatvecArgs a
                                 if (IM == 1) val = cmul(val, Ef);
                             }
                             if (b == r) {
-                                const size_t q = (size_t)row * NL + l;
+                                const size_t q = (size_t)rk * NL + l;
                                 if (IM == 1) {
                                     pout[q] = val;
                                 } else {
@@ -202,11 +216,20 @@ __global__ void __launch_bounds__(NT, Yz<NJ, NL, NT, MB>::MINB) k1p(MatvecArgs a
                                             pout[p * a.fstride + (size_t)d * ni * (NJ * NL) + q] = cmul(val, Ep[p][d]);
                                 }
                             }
-                            x[b][k] = val;
+                            x[k][b] = val;
                         }
+                    }
                 }
                 P2 v[R1];
-                fold_rows<NL, ZS, R1, R2>(x, v, r, t2, fz);
+#pragma unroll
+                for (int k = 0; k < R1; k++) v[k] = fold<NL, ZS>(x[k], r, elem(k), fz);
+                if constexpr (Y::WIDE) {
+#pragma unroll
+                    for (int k = 0; k < R1; k++) S[Y::at(row_of(r0, k), elem(k))] = f4_of(v[k]);
+                    __syncwarp();
+#pragma unroll
+                    for (int k = 0; k < R1; k++) v[k] = p_of(S[Y::at(row, t2 + R2 * k)]);
+                }
                 dftp<R1, false>(v);
 #pragma unroll
                 for (int k1 = 0; k1 < R1; k1++) {
@@ -230,13 +253,14 @@ __global__ void __launch_bounds__(NT, Yz<NJ, NL, NT, MB>::MINB) k1p(MatvecArgs a
                     for (int k2 = 0; k2 < R2; k2++) S[Y::at(rw, sub + R1 * k2)] = f4_of(u[k2]);
                 }
             }
+            if (AHEAD)
 #pragma unroll
-            for (int b = 0; b < ZS; b++)
+                for (int k = 0; k < R1; k++)
 #pragma unroll
-                for (int k = 0; k < R1; k++) {
-                    x[b][k] = xn[b][k];
-                    o[b][k] = on[b][k];
-                }
+                    for (int b = 0; b < ZS; b++) {
+                        x[k][b] = xn[k][b];
+                        o[k][b] = on[k][b];
+                    }
         }
     }
     __syncthreads();

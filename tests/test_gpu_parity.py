@@ -451,3 +451,31 @@ def test_products_in_flight_do_not_overtake(D, grid, nrhs):
             runs.append([g.cpu().numpy() for g in f])
     for a, b in zip(*runs):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("grid", [(4, 128, 64), (4, 128, 128), (16, 32, 8), (4, 4, 32)])
+def test_split_and_permuted_planes_vs_generic(D, grid):
+    """Sized y/z passes on planes split over two and four CTAs and on rows whose shared-memory order
+    depends on the row: products (three right-hand sides, both operators) and the incident-field
+    start of paired solves equal the run-time-sized passes (2e-6 of the field, two FP32 transforms;
+    1e-5 of the cross sections after three steps)."""
+    import torch
+    rng = np.random.default_rng(11)
+    x = torch.from_numpy(crand(rng, (3, 3) + grid)).cuda()
+    occ = rng.integers(0, 3, grid).astype(np.int8)
+    cfg = D.BatchConfig(occ=occ, materials=[(1.3, 0.01), (1.5, 0.1)], err_max=1e-12, max_step=3)
+    rot = D.mc_rotations(2, 2)
+    outs = []
+    for fast in (True, False):
+        with D.Context(grid, 0.2, max_rhs=4) as ctx:
+            ctx.set_kernels(fast)
+            y = [torch.empty_like(x) for _ in range(2)]
+            for k in range(2):
+                ctx.convolution_dev(x, y[k], 3, conj=k == 1)
+            torch.cuda.synchronize()
+            r = ctx.orientation_solves(cfg, rot)
+            outs.append(([v.cpu().numpy() for v in y], r))
+    for a, b in zip(outs[0][0], outs[1][0]):
+        assert rel(a, b) < 2e-6
+    for q in ("cabs", "cext"):
+        np.testing.assert_allclose(outs[0][1][q], outs[1][1][q], rtol=1e-5)
