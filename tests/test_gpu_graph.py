@@ -126,3 +126,36 @@ def test_bounded_wait_reports_and_recovers(D, oracle, xv):
         np.testing.assert_array_equal(again, ref)
         r = ctx.dda_fft(occ, alpha, [0, 1], kd, (0, 0, 1), (1, 0, 0), ksc, max_step=5)
         assert r["steps"] >= 1
+
+
+@pytest.mark.parametrize("grid,solver", [((8, 8, 8), 0), ((16, 16, 16), 2), ((4, 8, 16), 1)])
+def test_recorded_single_solves_follow_their_arguments(D, oracle, grid, solver):
+    """From its third call on a single solve of one shape is replayed.  Between replays everything a
+    call passes changes -- occupancy, polarisabilities, activity list, incident field, directions,
+    their number (the pinned staging is laid out anew) -- and each call equals the unrecorded
+    solve on a context of its own (same kernels on the same inputs; 1e-6 for the order of the
+    atomic sums)."""
+    rng = np.random.default_rng(7)
+    kd = 0.3
+    base = dict(occ=(rng.random(grid) < 0.7).astype(np.int8), alpha=np.array([0, 0.02 + 0.002j], np.complex64),
+                mv=[0, 1], kinc=(0, 0, 1), einc=(1, 0, 0), ksc=oracle.scattering_geometry(2, 7, 0.0, 30.0)[1])
+    other = (rng.random(grid) < 0.4).astype(np.int8)
+    changes = [{}, {}, {}, {}, dict(occ=other), dict(alpha=np.array([0, 0.03 + 0.001j], np.complex64)),
+               dict(kinc=(1, 0, 0), einc=(0, 1, 0)), dict(ksc=oracle.scattering_geometry(4, 37, 0.0, 5.0)[1]),
+               dict(ksc=base["ksc"]), {}, {}]
+
+    def run(ctx, s):
+        return ctx.dda_fft(s["occ"], s["alpha"], s["mv"], kd, s["kinc"], s["einc"], s["ksc"], solver=solver,
+                           max_step=12, err_max=1e-5, trace=False)
+
+    state = dict(base)
+    with D.Context(grid, kd) as ctx:
+        for ch in changes:
+            state.update(ch)
+            got = run(ctx, state)
+            with D.Context(grid, kd) as plain:
+                plain.set_solver_graph(False)
+                ref = run(plain, state)
+            assert np.abs(got["esc"] - ref["esc"]).max() <= 1e-6 * np.abs(ref["esc"]).max()
+            for q in ("cabs", "cext"):
+                assert abs(got[q] - ref[q]) <= 1e-6 * abs(ref[q])
