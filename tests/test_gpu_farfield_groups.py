@@ -91,3 +91,26 @@ def test_mid_configuration_both_forms(D, oracle):
     err = (np.abs(M - M1)[sig] / np.abs(M1)[sig]).max()
     print(f"mid configuration: grouped vs direct far field, significant Mueller max {err:.2e}")
     assert err < 1e-5
+
+
+@pytest.mark.parametrize("grid", [(4, 4, 2), (2, 64, 4), (2, 2, 128), (4, 32, 8)])
+def test_farfield_small_and_long_rows_vs_oracle(D, oracle, grid):
+    """Rows of one mirrored pair of z cells, of fewer pairs than a staged chunk and of several
+    chunks, pairs with one active cell, dipoles left on inactive cells (both forms must not read
+    them), and few planes (the direct form splits their rows over CTAs): FP64 oracle, 1e-5 as
+    for the larger lattices."""
+    rng = np.random.default_rng(6)
+    kd = 0.3
+    occ = rng.integers(0, 3, size=grid).astype(np.int8)
+    occ[0, 0, 0] = 1
+    mv = np.array([0, 1, 0])
+    p = crand(rng, grid + (3,))
+    q = p.copy()
+    q[occ != 1] = 0
+    _, ksc = oracle.scattering_geometry(5, 7, 0.0, 30.0)
+    with D.Context(grid, kd) as ctx:
+        for mode in (1, 2):
+            ctx.set_farfield_mode(mode)
+            out = ctx.farfield(occ, mv, kd, p, ksc)
+            ref = np.array([oracle.farfield(occ, mv, kd, q, k) for k in ksc.reshape(-1, 3)])
+            assert rel(out, ref) < 1e-5, mode
