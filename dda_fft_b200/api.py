@@ -620,8 +620,8 @@ class Context:
         _check(lib().ddagpu_set_tiling(self._h, tile_x, rows_g))
 
     def set_fast_variant(self, x_variant: int = 0, yz_variant: int = 0):
-        """Launch variants of the compile-time-sized passes: x 0..11 (tiles, bulk copies,
-        second line factorisation, TMA tensor tiles), y/z 0..2 (block sizes)."""
+        """Launch variants of the compile-time-sized passes: x 0..11 (unpacked tiles at edge 64,
+        then packed with bulk copies, register loads, TMA tensor tiles), y/z 0..2 (block sizes)."""
         _check(lib().ddagpu_set_fast_variant(self._h, x_variant, yz_variant))
 
     def set_farfield_mode(self, mode: int = 0):
