@@ -116,7 +116,7 @@ class ClockSampler:
 # ------------------------------------------------------------------ reference / CPU arm
 def cpu_reference(n_samples: int, threads: int):
     """The reference's own sample loop (oracle/_ref, physicist2018/dda-fft compiled from its
-    sources) on this workload; returns (orientation-solves/s, kind, seconds)."""
+    sources) on this workload; returns (orientation-solves/s, kind, seconds, threads)."""
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import pyoracle as P
     if os.path.exists(P.REF_SO):
@@ -125,7 +125,8 @@ def cpu_reference(n_samples: int, threads: int):
                              orientation=1, seed=SEED)
         secs, *_ = R.run_samples(cfg, n_samples, threads)
         return n_samples / secs, "reference", secs, threads
-    O = P.Oracle()   # the FP64 restatement, single thread
+    O = P.Oracle()   # the FP64 restatement, single thread: about a second per sample
+    n_samples = min(n_samples, 8)
     t0 = time.perf_counter()
     P.orientation_solves(O, GRID, X, [MAT], n_samples, target=2, b_a=BA, c_a=CA, orientation=1,
                          seed=SEED)
@@ -396,7 +397,7 @@ def main():
         ns = args.cpu_samples or max(24 * threads, 64)   # about 10 s of the host's threads
         v, kind, secs, used = cpu_reference(ns, threads)
         cpu = {"value": v, "unit": "orientation-solves/s", "cores": used, "kind": kind,
-               "sample": f"{ns} orientation-solves of the same workload, {secs:.1f} s wall "
+               "sample": f"{round(v * secs)} orientation-solves of the same workload, {secs:.1f} s wall "
                          f"(setup excluded)"}
         cpu["cross_check"] = cross_check(ctx, occ, 8)
 
