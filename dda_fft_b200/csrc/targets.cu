@@ -721,11 +721,8 @@ int anthrax_place(unsigned long long *state, int ni, float radius, float length,
     return 0;
 }
 
-size_t anthrax_scratch_bytes(int count) { return (size_t)(count ? count : 1) * sizeof(DW); }
-
 cudaError_t anthrax_rasterize(const float *cyl13, int count, int ni, int nj, int nl,
-                              signed char *occ_dev, int *ndip_dev, cudaStream_t st, void *scratch,
-                              size_t scratch_bytes)
+                              signed char *occ_dev, int *ndip_dev, cudaStream_t st)
 {
     // iGenerateAnthrax rasterisation, particle.cpp:62-83: centre n/2 - 0.5, radius n/2
     std::vector<DW> h((size_t)count);
@@ -733,10 +730,8 @@ cudaError_t anthrax_rasterize(const float *cyl13, int count, int ni, int nj, int
         const float *c = cyl13 + 13 * (size_t)k;
         h[(size_t)k] = DW{c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9], c[10]};
     }
-    // the caller's device scratch when it is large enough, else a stream-ordered allocation
-    const bool own = !scratch || scratch_bytes < anthrax_scratch_bytes(count);
-    DW *d = own ? nullptr : static_cast<DW *>(scratch);
-    cudaError_t e = own ? cudaMallocAsync(&d, anthrax_scratch_bytes(count), st) : cudaSuccess;
+    DW *d = nullptr;
+    cudaError_t e = cudaMallocAsync(&d, (size_t)(count ? count : 1) * sizeof(DW), st);
     if (e) return e;
     // pageable source: the copy has taken the host data when the call returns
     if (count) e = cudaMemcpyAsync(d, h.data(), count * sizeof(DW), cudaMemcpyHostToDevice, st);
@@ -751,7 +746,7 @@ cudaError_t anthrax_rasterize(const float *cyl13, int count, int ni, int nj, int
         rasterize<<<tiles, 256, 0, st>>>(d, count, ni, nj, nl, cx, cy, cz, R * R, occ_dev, ndip_dev);
         e = cudaGetLastError();
     }
-    if (own) cudaFreeAsync(d, st);
+    cudaFreeAsync(d, st);
     return e;
 }
 

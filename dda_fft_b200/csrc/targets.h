@@ -7,12 +7,8 @@ namespace ddagpu {
 long long anthrax_count(int ni, int nj, int nl, float packing, float radius, float ratio);
 int anthrax_place(unsigned long long *state, int ni, float radius, float length, int count,
                   float *cyl13, long long max_tries);
-// scratch (may be null): device memory for the monomers, used when it holds
-// anthrax_scratch_bytes(count); otherwise the call allocates stream-ordered memory
-size_t anthrax_scratch_bytes(int count);
 cudaError_t anthrax_rasterize(const float *cyl13, int count, int ni, int nj, int nl,
-                              signed char *occ_dev, int *ndip_dev, cudaStream_t st,
-                              void *scratch = nullptr, size_t scratch_bytes = 0);
+                              signed char *occ_dev, int *ndip_dev, cudaStream_t st);
 // no realisations (monomer lists one after the other in cyl13) into occ_dev [2 no][N], each at 2k
 // and 2k + 1 (both polarisations), and their dipole counts; scratch holds anthrax_batch_scratch bytes
 size_t anthrax_batch_scratch(int ni, int nj, int nl, int no, size_t total);
