@@ -744,10 +744,18 @@ constexpr int kSet = 12;
 // BiCGStab set: rho (0,1), <g,h> (2,3), <w,r> (4,5), <w,w> (6,7), sum |r| (8)
 
 __device__ __forceinline__ double2 set_at(const double *a, int k) { return make_double2(a[k], a[k + 1]); }
+// a / b with b brought to [1, 2) by a power of two: unscaled, its square leaves the doubles' range for
+// sums below 1e-154 or above 1e154 (a converged residual, right-hand sides in small or large
+// units) while the quotient is an ordinary number.  By zero or infinity part by part: infinite and
+// zero coefficients, as a complex division gives them.
 __device__ __forceinline__ double2 ddiv(double2 a, double2 b)
 {
-    const double d = b.x * b.x + b.y * b.y;
-    return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
+    const double m = fmax(fabs(b.x), fabs(b.y));
+    if (!(m > 0.0) || isinf(m)) return make_double2(a.x / m, a.y / m);
+    const int e = ilogb(m);
+    const double2 c = make_double2(scalbn(b.x, -e), scalbn(b.y, -e));
+    const double d = c.x * c.x + c.y * c.y;
+    return make_double2(scalbn((a.x * c.x + a.y * c.y) / d, -e), scalbn((a.y * c.x - a.x * c.y) / d, -e));
 }
 __device__ __forceinline__ void bil_add(double &re, double &im, double2 a, double2 b)
 {

@@ -140,3 +140,23 @@ def test_fp64_passes_every_edge_vs_oracle(D, oracle, grid):
     assert rel(r["trace"], o["trace"]) < 1e-10
     assert rel(r["p"], o["p"]) < 1e-10
     assert rel(r["esc"], o["esc"].reshape(-1, 3)) < 1e-10
+
+
+@pytest.mark.parametrize("exponent", [-300, 300])
+@pytest.mark.parametrize("solver", [0, 2])
+def test_fp64_solve_in_any_units(D, oracle, solver, exponent):
+    """A right-hand side times 2^300 or 2^-300: every step of the recurrences scales by that power
+    exactly, their products (2^600) stay inside the doubles' range and so must the quotients, whose
+    divisors' squares (2^1200) do not.  The solution and the trace are those of the unscaled
+    system, up to the order of the FP64 atomic sums (2^-53 each) that eight steps amplify: 1e-9."""
+    grid, kd = (8, 4, 16), 0.5
+    rng = np.random.default_rng(4)
+    occ = (rng.random(grid) < 0.7).astype(np.int8)
+    alpha = np.array([0, oracle.polarizability(2, kd, 1.5 + 0.1j)])
+    rhs = rng.standard_normal(grid + (3,)) + 1j * rng.standard_normal(grid + (3,))
+    with D.Context(grid, kd) as ctx:
+        r = [ctx.solve_fp64(occ, alpha, [0, 1], kd, (0, 0, 1), (1, 0, 0), solver=solver, max_step=8,
+                            err_max=0.0, rhs=rhs * s, want_p=True) for s in (1.0, 2.0 ** exponent)]
+    assert r[1]["steps"] == r[0]["steps"] == 8 and r[1]["step_min"] == r[0]["step_min"]
+    assert rel(r[1]["trace"] * 2.0 ** -exponent, r[0]["trace"]) < 1e-9
+    assert rel(r[1]["p"] * 2.0 ** -exponent, r[0]["p"]) < 1e-9
