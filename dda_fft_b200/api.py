@@ -110,6 +110,7 @@ def lib():
         L.ddagpu_mc_rotations.argtypes = [C.c_ulonglong, _i, _i, _p]
         L.ddagpu_fixed_rotation.argtypes = [_d, _d, _d, _p]
         L.ddagpu_convolution_dev.argtypes = [_p, _p, _p, _i, _i]
+        L.ddagpu_synchronize.argtypes = [_p]
         L.ddagpu_stream.argtypes = [_p]
         L.ddagpu_stream.restype = _p
         L.ddagpu_kernel_launches.argtypes = [_p]
@@ -615,6 +616,11 @@ class Context:
         context's stream."""
         _check(lib().ddagpu_convolution_dev(self._h, C.c_void_p(p_dev.data_ptr()),
                                             C.c_void_p(out_dev.data_ptr()), nrhs, int(conj)))
+
+    def synchronize(self) -> None:
+        """Wait for this context's stream; raises if a bounded wait of a device-resident product
+        enqueued before ran out (its output is then not a number)."""
+        _check(lib().ddagpu_synchronize(self._h))
 
     def set_tiling(self, tile_x=0, rows_g=0):
         _check(lib().ddagpu_set_tiling(self._h, tile_x, rows_g))

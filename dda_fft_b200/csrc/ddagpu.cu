@@ -241,6 +241,15 @@ int device_wait_error(ddagpu_ctx *c, int flag)
     return fail(DDAGPU_ECUDA, "a device wait ran out (asynchronous copy not completed)");
 }
 
+// The flag of the context's stream so far, read and reported.
+int check_waits(ddagpu_ctx *c)
+{
+    int flag = 0;
+    CK(cudaMemcpyAsync(&flag, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    return device_wait_error(c, flag);
+}
+
 // Forget the recorded solve graphs (they hold buffer addresses about to change).
 void drop_graphs(ddagpu_ctx *c)
 {
@@ -1163,6 +1172,14 @@ int ddagpu_convolution_dev(ddagpu_ctx *c, const void *p_dev, void *out_dev, int 
     return DDAGPU_OK;
 }
 
+int ddagpu_synchronize(ddagpu_ctx *c)
+{
+    if (!c) return fail(DDAGPU_EINVAL, "null context");
+    std::lock_guard<std::mutex> lk(c->mu);
+    DevGuard dg(c->dev);
+    return check_waits(c);
+}
+
 int ddagpu_autotune(ddagpu_ctx *c, int nrhs)
 {
     if (!c) return fail(DDAGPU_EINVAL, "null context");
@@ -1218,6 +1235,7 @@ int ddagpu_autotune(ddagpu_ctx *c, int nrhs)
                 c->fyz = vyz;
                 float ms = 0;
                 RET(time_it(&ms));
+                if (fast_x_waits(vx) && check_waits(c) != DDAGPU_OK) continue;   // it gave up
                 if (ms < best) {
                     best = ms;
                     bfast = 1;
@@ -1264,10 +1282,7 @@ int ddagpu_convolution(ddagpu_ctx *c, const float *p, float *out, int conj)
     CK(launch_matvec(a, c->st));
     CK(field_to_aos(c->r, c->w, N, c->st));
     CK(cudaMemcpyAsync(out, c->w, 3 * N * sizeof(float2), cudaMemcpyDeviceToHost, c->st));
-    int werr = 0;
-    CK(cudaMemcpyAsync(&werr, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    return device_wait_error(c, werr);
+    return check_waits(c);
 }
 
 }  // extern "C"
@@ -1803,6 +1818,7 @@ int refine_loop(ddagpu_ctx *c, int solver, float rTau, int nmat1, double d0, int
         CK(launch_refine(2, F, c->st));
         c->launches += 1;
     }
+    RET(check_waits(c));   // of the last product (run_solver has checked those before)
     ri.err = err;
     ri.matvecs += ri.outer + 1;
     CK(launch_refine(3, F, c->st));
@@ -1839,11 +1855,7 @@ int mixed_refine(ddagpu_ctx *c, const float *cListMaterials, int nmat1, int nact
     ri.matvecs = R.matvecs;
     ri.err = R.err;
     for (int k = 0; k < 64; k++) ri.err_history[k] = R.history[k];
-    int werr = 0;
-    CK(cudaMemcpyAsync(&werr, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    RET(device_wait_error(c, werr));
-    return DDAGPU_OK;
+    return check_waits(c);
 }
 
 }  // namespace

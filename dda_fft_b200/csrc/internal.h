@@ -140,6 +140,7 @@ constexpr int kXVariants = 12;     // launch variants of the fast x pass (9..11:
 constexpr int kYZVariants = 3;     // launch variants of the fast y/z passes
 cudaError_t matvec_fast_prepare(const Lat &L);
 int matvec_fast_x_tile(int nl);           // spectral columns per TMA tile, 0: row too short
+constexpr bool fast_x_waits(int fx) { return (fx >= 3 && fx < 6) || fx >= 9; }   // x variants with a bounded wait
 void matvec_fast_defaults(const Lat &L, bool has_tmap, int *fx, int *fyz);   // untuned launch variants
 cudaError_t launch_matvec_fast(const MatvecArgs &a, cudaStream_t st);
 // CTAs per plane of the y/z passes: at most 4096 pairs (64 KB of shared memory) each

@@ -203,6 +203,15 @@ DDA_DEV void pair_step_b(Load load, int sub, const float2 *hw, Put put)
     }
 }
 
+// A block whose wait for its inputs ran out leaves its columns not a number, which the inverse
+// spreads over the whole product: a caller that does not ask for the error flag sees it too.
+// (A function of its own: inlined, its loop changes the kernels around it.)
+__device__ __noinline__ void gave_up(float4 *col, size_t step, int n)
+{
+    const float nan = __int_as_float(0x7fffffff);
+    for (int k = 0; k < n; k++) col[k * step] = make_float4(nan, nan, nan, nan);
+}
+
 template <int NI>
 constexpr int pair_min_blocks() { return NI >= 128 ? 2 : NI >= 64 ? 4 : NI >= 32 ? 7 : 12; }
 
@@ -260,6 +269,7 @@ k2q(MatvecArgs a, const __grid_constant__ CUtensorMap tmap)
         bool got = mbar_wait(&bar, 0);
         if (got && a.wait_selftest) got = mbar_wait(&bar, 1, 1 << 10);
         if (!__syncthreads_and(got)) {   // the same decision for every thread
+            if (ok) gave_up(base + (size_t)sub * plane, (size_t)R1 * plane, 3 * NI / R1);
             if (threadIdx.x == 0 && a.err) atomicExch(a.err, 1);
             mbar_wait(&bar, 0);           // one more bounded wait for the copies in flight
             return;

@@ -368,8 +368,14 @@ int ddagpu_farfield_noalloc(int device, int i_max, int j_max, int l_max, float d
 
 /* ---------------------------------------------------------------- device-resident form
  * G*p for nrhs fields already in device memory ([nrhs][3][i][j][l] complex float, SoA),
- * on the context's stream; nrhs <= max_rhs. */
+ * on the context's stream; nrhs <= max_rhs.  The passes are only enqueued.  Where
+ * their bounded wait for asynchronous copies ran out (x variants 3..5 and 9..11, see
+ * ddagpu_set_fast_variant), the product is not a number, and ddagpu_synchronize, or the next
+ * call on the context that returns results, reports it. */
 int ddagpu_convolution_dev(ddagpu_ctx *ctx, const void *p_dev, void *out_dev, int nrhs, int conj);
+/* Waits for the context's stream.  DDAGPU_ECUDA if a device wait of the work enqueued before
+ * ran out (that work's outputs are not usable); the report is cleared. */
+int ddagpu_synchronize(ddagpu_ctx *ctx);
 /* The context's CUDA stream (cudaStream_t), for callers that time or order work on it. */
 void *ddagpu_stream(ddagpu_ctx *ctx);
 /* Number of CUDA kernels this context has launched so far. */

@@ -159,3 +159,67 @@ def test_recorded_single_solves_follow_their_arguments(D, oracle, grid, solver):
             assert np.abs(got["esc"] - ref["esc"]).max() <= 1e-6 * np.abs(ref["esc"]).max()
             for q in ("cabs", "cext"):
                 assert abs(got[q] - ref[q]) <= 1e-6 * abs(ref[q])
+
+
+@pytest.mark.parametrize("xv", [None, 3, 9])
+def test_device_products_that_gave_up_are_reported(D, xv):
+    """convolution_dev only enqueues its passes.  Where a wait ran out (the variant a context starts
+    with, bulk copies, TMA tiles) the product is not a number everywhere, and synchronize() reports
+    it and clears the report: the calls after it are their own."""
+    import torch
+    grid = (16, 16, 16)
+    rng = np.random.default_rng(13)
+    p = (rng.standard_normal((1, 3) + grid) + 1j * rng.standard_normal((1, 3) + grid)).astype(np.complex64)
+    x = torch.from_numpy(p).cuda()
+    y = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    with D.Context(grid, 0.4) as ctx:
+        if xv is not None:
+            ctx.set_fast_variant(xv, 0)
+        assert ctx.fast_variant[0] in (3, 9)
+        ctx.convolution_dev(x, y, 1)
+        ctx.synchronize()
+        ref = y.cpu().numpy()
+        assert np.isfinite(ref).all()
+        ctx.selftest_wait_timeout(True)
+        ctx.convolution_dev(x, y, 1)
+        with pytest.raises(D.DDAGPUError, match="wait ran out"):
+            ctx.synchronize()
+        assert np.isnan(y.cpu().numpy()).all()
+        ctx.selftest_wait_timeout(False)
+        ctx.synchronize()
+        ctx.convolution_dev(x, y, 1)
+        ctx.synchronize()
+        np.testing.assert_array_equal(y.cpu().numpy(), ref)
+
+
+def test_autotune_takes_no_variant_that_gives_up(D, oracle):
+    """Variants whose wait runs out while they are timed are not picked, and leave no error."""
+    grid = (16, 16, 16)
+    rng = np.random.default_rng(14)
+    p = (rng.standard_normal(grid + (3,)) + 1j * rng.standard_normal(grid + (3,))).astype(np.complex64)
+    ref = oracle.convolution(oracle.green_hat(*grid, 0.4), p.astype(np.complex128))
+    with D.Context(grid, 0.4) as ctx:
+        ctx.selftest_wait_timeout(True)
+        ctx.autotune(1)
+        out = ctx.convolution(p)   # (the pick does not wait)
+        assert not ctx.fast_kernels or ctx.fast_variant[0] in (0, 1, 2, 6, 7, 8)
+        ctx.selftest_wait_timeout(False)
+        again = ctx.convolution(p)
+    for o in (out, again):
+        assert np.abs(o - ref).max() < 2e-5 * np.abs(ref).max()
+
+
+def test_refinement_reports_its_last_product(D, oracle):
+    """The product behind the last true residual of a refinement is checked like the others."""
+    occ, kd, alpha, ksc = problem(oracle)
+    rhs = np.ones(occ.shape + (3,), np.complex64)
+    with D.Context(occ.shape, kd) as ctx:
+        ctx.set_fast_variant(9, 0)
+        ctx.selftest_wait_timeout(True)
+        with pytest.raises(D.DDAGPUError, match="wait ran out"):
+            ctx.solve_linear(occ, alpha, [0, 1], rhs, solver=2, max_step=0, refine=True)
+        with pytest.raises(D.DDAGPUError, match="wait ran out"):
+            ctx.dda_fft_refined(occ, alpha, [0, 1], kd, (0, 0, 1), (1, 0, 0), ksc, solver=2, max_outer=0)
+        ctx.selftest_wait_timeout(False)
+        ctx.solve_linear(occ, alpha, [0, 1], rhs, solver=2, max_step=0, refine=True)
