@@ -1321,7 +1321,8 @@ int upload_materials(ddagpu_ctx *c, const int *mv, int nmat1, const signed char 
 int upload_directions(ddagpu_ctx *c, const double *ks, int nrhs, int ndir, bool pairs, double nact)
 {
     if (ndir <= 0) {
-        c->kz.groups = 0;
+        c->kz.groups = 0;   // no plan stands any more
+        c->kz_dirs.clear();
         return DDAGPU_OK;
     }
     const size_t n = (size_t)nrhs * ndir * 3;

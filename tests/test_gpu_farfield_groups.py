@@ -114,3 +114,24 @@ def test_farfield_small_and_long_rows_vs_oracle(D, oracle, grid):
             out = ctx.farfield(occ, mv, kd, p, ksc)
             ref = np.array([oracle.farfield(occ, mv, kd, q, k) for k in ksc.reshape(-1, 3)])
             assert rel(out, ref) < 1e-5, mode
+
+
+def test_farfield_plan_survives_a_call_without_directions(D, oracle):
+    """The plan of the last directions is kept for the next call with the same ones.  After a call
+    without any directions the next call with the earlier ones has to sum by groups again (four
+    launches; the direct form takes two), and gives what it gave before (1e-6: the order of the
+    FP64 atomic sums)."""
+    grid, kd = (8, 16, 8), 0.4
+    rng = np.random.default_rng(9)
+    occ = rng.integers(0, 2, size=grid).astype(np.int8)
+    p = crand(rng, grid + (3,))
+    _, ksc = oracle.scattering_geometry(12, 19, 0.0, 10.0)
+    with D.Context(grid, kd) as ctx:
+        ctx.set_farfield_mode(2)
+        out = []
+        for _ in range(2):
+            n0 = ctx.kernel_launches
+            out.append(ctx.farfield(occ, [0, 1], kd, p, ksc))
+            assert ctx.kernel_launches - n0 == 4
+            assert ctx.farfield(occ, [0, 1], kd, p, ksc[:0]).shape == (0, 3)
+    assert rel(out[1], out[0]) < 1e-6
