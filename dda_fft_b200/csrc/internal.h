@@ -83,7 +83,9 @@ cudaError_t launch_chained(bool chained, void (*kernel)(P...), dim3 grid, dim3 b
         cfg.numAttrs++;
     }
     cfg.attrs = at;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    if (e != cudaSuccess) cudaGetLastError();   // reported here, not by whoever asks next
+    return e;
 }
 
 struct MatvecArgs {

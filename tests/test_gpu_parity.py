@@ -479,3 +479,19 @@ def test_split_and_permuted_planes_vs_generic(D, grid):
         assert rel(a, b) < 2e-6
     for q in ("cabs", "cext"):
         np.testing.assert_allclose(outs[0][1][q], outs[1][1][q], rtol=1e-5)
+
+
+def test_a_refused_product_leaves_no_error_behind(D, oracle):
+    """More right-hand sides than a launch grid holds (65535) are refused by the CUDA runtime when the
+    product is launched.  The next calls, of this context and of another one, are not affected."""
+    import torch
+    g, kd, n = (4, 4, 4), 0.4, 65536
+    p = crand(np.random.default_rng(3), g + (3,))
+    ref = oracle.convolution(oracle.green_hat(*g, kd), p.astype(np.complex128))
+    with D.Context(g, kd, max_rhs=n) as big, D.Context(g, kd) as other:
+        x = torch.zeros((n, 3) + g, dtype=torch.complex64, device="cuda")
+        y = torch.empty_like(x)
+        with pytest.raises(D.DDAGPUError):
+            big.convolution_dev(x, y, n)
+        for ctx in (other, big):
+            assert rel(ctx.convolution(p), ref) < CONV_TOL
