@@ -1527,6 +1527,12 @@ int ensure_pin(ddagpu_ctx *c, size_t bytes)
     return DDAGPU_OK;
 }
 
+// Doubles of ddagpu_mueller's staging: kd, ed, ks, nv and the result in double, es in float.
+size_t mueller_doubles(int nplanes, int nangles)
+{
+    return 6 + 12 + (size_t)12 * nplanes * nangles + (size_t)3 * nplanes + (size_t)16 * nangles;
+}
+
 // Offsets of a batched chunk's pinned staging: inputs kin, ein, ks, nv (double), al
 // (float2); outputs ca, ce (float), mo (double); every block 16-byte aligned.
 struct ChunkLayout {
@@ -1717,7 +1723,8 @@ int ddagpu_dda_fft(ddagpu_ctx *c, int iNoIllumination, int solver, float rTau, i
     std::vector<double> pageable;
     unsigned char *buf;
     if (again) {
-        RET(ensure_pin(c, total));
+        // (wide enough for the sample's ddagpu_mueller too)
+        RET(ensure_pin(c, std::max(total, 8 * mueller_doubles(iNoScPl, iNoA))));
         buf = c->pin;
     } else {
         pageable.resize((total + 7) / 8);
@@ -2145,14 +2152,14 @@ int ddagpu_mueller(ddagpu_ctx *c, const float *kinc, const float *einc0, const f
     DevGuard dg(c->dev);
     const int ndir = nplanes * nangles;
     RET(ensure_post(c, ndir, nplanes, nangles));
-    // staging in the context's pinned block where it has one (it gets one with its first recorded
-    // solve), else pageable: kd, ed, ks, nv and the result in double, es in float
-    const size_t n_ks = (size_t)6 * ndir, n_mo = (size_t)nangles * 16,
-                 doubles = 6 + 12 + n_ks + (size_t)nplanes * 3 + n_mo + n_ks;
+    // staging in the context's pinned block where it has one that is wide enough (from its first
+    // recorded solve on), else pageable; never a wider block, which would cost the recorded
+    // solves that write to this one
+    const size_t n_ks = (size_t)6 * ndir, n_mo = (size_t)nangles * 16, doubles = mueller_doubles(nplanes, nangles);
+    const bool pinned = doubles * sizeof(double) <= c->pin_bytes;
     std::vector<double> pageable;
-    if (c->pin) RET(ensure_pin(c, doubles * sizeof(double)));
-    else pageable.resize(doubles);
-    double *kd = c->pin ? reinterpret_cast<double *>(c->pin) : pageable.data(), *ed = kd + 6, *ks = ed + 12,
+    if (!pinned) pageable.resize(doubles);
+    double *kd = pinned ? reinterpret_cast<double *>(c->pin) : pageable.data(), *ed = kd + 6, *ks = ed + 12,
            *nv = ks + n_ks, *mo = nv + (size_t)nplanes * 3;
     float *es = reinterpret_cast<float *>(mo + n_mo);
     for (int k = 0; k < 3; k++) kd[k] = kd[3 + k] = kinc[k];
@@ -2164,8 +2171,10 @@ int ddagpu_mueller(ddagpu_ctx *c, const float *kinc, const float *einc0, const f
     for (int k = 0; k < nplanes * 3; k++) nv[k] = normals[k];
     std::memcpy(es, esc0, n_ks * sizeof(float));
     std::memcpy(es + n_ks, esc1, n_ks * sizeof(float));
-    if (c->pin) {
-        // every value is read once: the kernel reads and writes the pinned block itself
+    if (pinned) {
+        // the kernel reads and writes the pinned block itself: the fields and directions are read once,
+        // the few values that all threads share again and again (29 us against 51 with copies at
+        // 19 directions, 57 against 95 at 12 x 181, 290 against 307 at 90 x 181)
         MuellerArgs m{1, nplanes, nangles, ndir, kd, ed, ks, nv, reinterpret_cast<const float2 *>(es), mo};
         CK(launch_mueller(m, c->st));
     } else {

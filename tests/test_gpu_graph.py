@@ -223,3 +223,41 @@ def test_refinement_reports_its_last_product(D, oracle):
             ctx.dda_fft_refined(occ, alpha, [0, 1], kd, (0, 0, 1), (1, 0, 0), ksc, solver=2, max_outer=0)
         ctx.selftest_wait_timeout(False)
         ctx.solve_linear(occ, alpha, [0, 1], rhs, solver=2, max_step=0, refine=True)
+
+
+def test_mueller_between_recorded_solves_keeps_the_recording(D, oracle):
+    """The drop-in sample loop: solves of both polarisations, then their Mueller matrix.  The first
+    mueller() after a recorded solve finds the pinned block wide enough: it does not release the
+    block that the recording writes to and allocate another (milliseconds against the 40 us of a
+    call; the medians of nine contexts, a factor of five between the first call and the second).
+    A wider one goes by the pageable copies.  All give what a context without a recording gives,
+    and the solves around them what they gave."""
+    import time
+    occ, kd, alpha, ksc = problem(oracle, 8)
+    nrm, ksc = oracle.scattering_geometry(4, 37, 0.0, 5.0)
+    wide, wksc = oracle.scattering_geometry(9, 37, 0.0, 5.0)
+    k, E = (0, 0, 1), ((1, 0, 0), (0, 1, 0))
+    rng = np.random.default_rng(15)
+    wesc = (rng.standard_normal(wksc.shape) + 1j * rng.standard_normal(wksc.shape)).astype(np.complex64)
+    times = []
+    for _ in range(9):
+        with D.Context(occ.shape, kd, max_rhs=2) as ctx, D.Context(occ.shape, kd, max_rhs=2) as fresh:
+            def solve():
+                return ctx.dda_fft(occ, alpha, [0, 1], kd, k, E[0], ksc, max_step=20, err_max=1e-3, trace=False)["esc"]
+
+            def mueller():
+                t = time.perf_counter()
+                M = ctx.mueller(k, *E, ksc, nrm, esc, wesc[:4])
+                return time.perf_counter() - t, M
+            for _ in range(4):
+                esc = solve()
+            (t0, M0), (t1, M1) = mueller(), mueller()
+            times.append((t0, t1))
+            Mw = ctx.mueller(k, *E, wksc, wide, wesc, wesc[::-1])
+            np.testing.assert_array_equal(M0, fresh.mueller(k, *E, ksc, nrm, esc, wesc[:4]))
+            np.testing.assert_array_equal(M1, M0)
+            np.testing.assert_array_equal(Mw, fresh.mueller(k, *E, wksc, wide, wesc, wesc[::-1]))
+            again = solve()
+            assert np.abs(again - esc).max() <= 1e-6 * np.abs(esc).max()
+    first, second = np.median(np.array(times), axis=0)
+    assert first < 5 * second
