@@ -97,7 +97,7 @@ struct ddagpu_ctx {
     // pinned host staging of the batched calls' inputs and outputs, grown on demand (the
     // copies from and to it are asynchronous, unlike those of pageable memory)
     unsigned char *pin = nullptr;
-    size_t pin_bytes = 0;
+    size_t pin_bytes = 0, pin_size = 0;   // of the staging, of the block
     // post-processing buffers, grown on demand
     int ndir_cap = 0;
     double *ksc = nullptr, *esc_acc = nullptr, *cc_acc = nullptr, *normals = nullptr,
@@ -1095,7 +1095,7 @@ int ddagpu_destroy(ddagpu_ctx *c)
                     c->inc_tab, c->kz_tab, c->kz_val, c->kz_sum};
     for (void *q : ptrs)
         if (q) cudaFree(q);
-    if (c->pin) cudaFreeHost(c->pin);
+    pinned_give(c->pin, c->pin_size);   // (the stream is idle)
     delete c->f64;
     delete c->mcg;
     if (c->st) cudaStreamDestroy(c->st);
@@ -1518,11 +1518,12 @@ int ensure_pin(ddagpu_ctx *c, size_t bytes)
     if (bytes <= c->pin_bytes) return DDAGPU_OK;
     if (c->pin) {
         drop_graphs(c);   // recorded solves write their results there
-        cudaFreeHost(c->pin);
+        CK(cudaStreamSynchronize(c->st));   // (a call that failed may have left copies in flight)
+        pinned_give(c->pin, c->pin_size);
     }
     c->pin = nullptr;
     c->pin_bytes = 0;
-    CK(cudaHostAlloc((void **)&c->pin, ((bytes + 15) & ~(size_t)15) + PinnedSolve::bytes(c->cap), cudaHostAllocDefault));
+    CK(pinned_take(((bytes + 15) & ~(size_t)15) + PinnedSolve::bytes(c->cap), &c->pin, &c->pin_size));
     c->pin_bytes = bytes;
     return DDAGPU_OK;
 }

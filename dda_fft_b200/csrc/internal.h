@@ -164,6 +164,11 @@ template <int NI> cudaError_t x_launch(const MatvecArgs &a, cudaStream_t st);
 DDA_EDGES(DDA_DECLARE)
 #undef DDA_DECLARE
 
+// Pinned host memory of at least `bytes` (*size), from blocks given back before where one fits
+// (pinned.cu).  No work on the device may use a block that is given back.
+cudaError_t pinned_take(size_t bytes, unsigned char **p, size_t *size);
+void pinned_give(unsigned char *p, size_t size);
+
 // smaller factor R2 of an edge's line split (pair.cuh line_split)
 constexpr int line_r2(int n) { return n <= 8 ? 2 : n <= 32 ? 4 : 8; }
 
