@@ -597,6 +597,9 @@ int run_solver(ddagpu_ctx *c, int nrhs, int solver, float tau, int max_step, flo
         CK(dalloc(&c->trace, (size_t)c->cap * tl));
         c->trace_len = tl;
     }
+    // (before a recording: the limits are set on the host)
+    const int pair = c->pair_step0 && nrhs % 2 == 0 ? 1 : 0;
+    if (!rhs_in && c->fast) CK(matvec_fast_prepare(c->L, c->fx, c->fyz, 1 + pair));
     double *trace = want_trace ? c->trace : nullptr;
     const int tlen = want_trace ? tl : 0;
     const bool whole = post && (c->graph_on || rec) && !want_trace && !rhs_in;
@@ -640,7 +643,7 @@ int run_solver(ddagpu_ctx *c, int nrhs, int solver, float tau, int max_step, flo
         else CK(launch_inc_tables(F, c->inc_tab, st));
         MatvecArgs m = mv_args(c, nrhs, c->p, c->r, 1, 0.f, nullptr, 0, nmat1, true);
         m.inc = 1;
-        m.pair = (c->pair_step0 && nrhs % 2 == 0) ? 1 : 0;
+        m.pair = pair;
         m.inc_tab = c->inc_tab;
         m.einc = c->einc;
         m.inc_out = c->p;
@@ -1059,8 +1062,7 @@ int ddagpu_create(ddagpu_ctx **out, int device, int i_max, int j_max, int l_max,
     c->L.fz = c->L.tz + l_max / zs;
     if ((e = cudaMemcpyAsync(c->tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice,
                              c->st)) != cudaSuccess ||
-        (e = matvec_prepare(c->L, c->tile_x, c->rows_g)) != cudaSuccess ||
-        (fast && (e = matvec_fast_prepare(c->L)) != cudaSuccess) ||
+        (!fast && (e = matvec_prepare(c->L, c->tile_x, c->rows_g)) != cudaSuccess) ||
         (e = post_prepare(j_max, l_max)) != cudaSuccess ||
         (e = green_build_octant(i_max, j_max, l_max, kd, c->ahat, c->st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(c->st)) != cudaSuccess)
@@ -1069,6 +1071,8 @@ int ddagpu_create(ddagpu_ctx **out, int device, int i_max, int j_max, int l_max,
     if (c->fast) {
         c->has_tmap = encode_work_maps(c);
         matvec_fast_defaults(c->L, c->has_tmap, &c->fx, &c->fyz);
+        if ((e = matvec_fast_prepare(c->L, c->fx, c->fyz, 0)) != cudaSuccess)
+            return bail(fail(DDAGPU_ECUDA, std::string("setup: ") + cudaGetErrorString(e)));
     }
     if (cudaMemset(c->err_dev, 0, sizeof(int)) != cudaSuccess)
         return bail(fail(DDAGPU_ECUDA, "setup: error flag"));
@@ -1146,6 +1150,8 @@ int ddagpu_set_kernels(ddagpu_ctx *c, int fast)
     if (!c) return fail(DDAGPU_EINVAL, "null context");
     if (fast && !matvec_fast_supported(c->L))
         return fail(DDAGPU_EINVAL, "compile-time-sized passes need edges of 4 at least");
+    DevGuard dg(c->dev);
+    if (!fast) CK(matvec_prepare(c->L, c->tile_x, c->rows_g));
     c->fast = fast ? 1 : 0;
     return DDAGPU_OK;
 }
@@ -1233,6 +1239,7 @@ int ddagpu_autotune(ddagpu_ctx *c, int nrhs)
             for (int vyz = 0; vyz < 2; vyz++) {   // (2 is 0)
                 c->fx = vx;
                 c->fyz = vyz;
+                CK(matvec_fast_prepare(c->L, vx, vyz, 0));
                 float ms = 0;
                 RET(time_it(&ms));
                 if (fast_x_waits(vx) && check_waits(c) != DDAGPU_OK) continue;   // it gave up
@@ -2315,6 +2322,10 @@ int ddagpu_set_fast_variant(ddagpu_ctx *c, int x_variant, int yz_variant)
         return fail(DDAGPU_EINVAL, "launch variants: x 0..11, y/z 0..2");
     if (x_variant >= 9 && !c->has_tmap) return fail(DDAGPU_EINVAL, "no tensor maps on this device");
     std::lock_guard<std::mutex> lk(c->mu);
+    if (matvec_fast_supported(c->L)) {
+        DevGuard dg(c->dev);
+        CK(matvec_fast_prepare(c->L, x_variant, yz_variant, 0));
+    }
     c->fx = x_variant;
     c->fyz = yz_variant;
     return DDAGPU_OK;

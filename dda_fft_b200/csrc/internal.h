@@ -140,26 +140,27 @@ cudaError_t matvec_prepare(const Lat &L, int tile_x, int rows_g);
 bool matvec_fast_supported(const Lat &L);
 constexpr int kXVariants = 12;     // launch variants of the fast x pass (9..11: TMA tensor tiles)
 constexpr int kYZVariants = 3;     // launch variants of the fast y/z passes
-cudaError_t matvec_fast_prepare(const Lat &L);
+// Shared-memory limits of the passes that a variant launches for `form` (0 a field, 1 the incident
+// field, 2 that of a polarisation pair), no others: asking for one loads the kernel.  The carveout
+// stays the driver's choice (the largest one cost 15%: what the passes leave, L1 uses for the
+// Green tensor, twiddles and row sectors).
+cudaError_t matvec_fast_prepare(const Lat &L, int fx, int fyz, int form);
 int matvec_fast_x_tile(int nl);           // spectral columns per TMA tile, 0: row too short
 constexpr bool fast_x_waits(int fx) { return (fx >= 3 && fx < 6) || fx >= 9; }   // x variants with a bounded wait
 void matvec_fast_defaults(const Lat &L, bool has_tmap, int *fx, int *fyz);   // untuned launch variants
 cudaError_t launch_matvec_fast(const MatvecArgs &a, cudaStream_t st);
 // CTAs per plane of the y/z passes: at most 4096 pairs (64 KB of shared memory) each
 __host__ __device__ constexpr int matvec_z_split(int nj, int nl) { return nj * nl <= 4096 ? 1 : nj * nl <= 8192 ? 2 : 4; }
-// dynamic shared memory of a matvec kernel; the carveout stays the driver's choice (the largest
-// one cost 15%: what the passes leave, L1 uses for the Green tensor, twiddles and row sectors)
-cudaError_t matvec_kernel_smem(const void *kernel, int bytes);
 // per edge, one object each (Makefile)
-template <int NJ> cudaError_t yz_prepare(int nl);
+template <int NJ> cudaError_t yz_prepare(int nl, int fyz, int form);
 template <int NJ> cudaError_t yz_launch(const MatvecArgs &a, int fwd, cudaStream_t st);
-template <int NI> cudaError_t x_prepare();
+template <int NI> cudaError_t x_prepare(int nl, int fx, int form);
 template <int NI> cudaError_t x_launch(const MatvecArgs &a, cudaStream_t st);
 #define DDA_EDGES(F) F(4) F(8) F(16) F(32) F(64) F(128)
 #define DDA_DECLARE(N)                                                                        \
-    template <> cudaError_t yz_prepare<N>(int nl);                                            \
+    template <> cudaError_t yz_prepare<N>(int nl, int fyz, int form);                         \
     template <> cudaError_t yz_launch<N>(const MatvecArgs &a, int fwd, cudaStream_t st);      \
-    template <> cudaError_t x_prepare<N>();                                                   \
+    template <> cudaError_t x_prepare<N>(int nl, int fx, int form);                           \
     template <> cudaError_t x_launch<N>(const MatvecArgs &a, cudaStream_t st);
 DDA_EDGES(DDA_DECLARE)
 #undef DDA_DECLARE

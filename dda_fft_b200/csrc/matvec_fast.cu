@@ -14,28 +14,23 @@ bool matvec_fast_supported(const Lat &L) { return fast_edge(L.ni) && fast_edge(L
 // spectral columns per TMA tile of the x pass; 0 where the rows are shorter
 int matvec_fast_x_tile(int nl) { return nl >= 8 ? 16 : 0; }
 
-cudaError_t matvec_kernel_smem(const void *kernel, int bytes)
-{
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 void matvec_fast_defaults(const Lat &L, bool has_tmap, int *fx, int *fyz)
 {
     *fx = L.ni == 64 ? 1 : has_tmap ? 9 : 6;
     *fyz = (long long)L.nj * L.nl <= 1024 ? 1 : 0;
 }
 
-cudaError_t matvec_fast_prepare(const Lat &L)
+cudaError_t matvec_fast_prepare(const Lat &L, int fx, int fyz, int form)
 {
     cudaError_t e = cudaErrorInvalidValue;
     switch (L.nj) {
-#define CASE(N) case N: e = yz_prepare<N>(L.nl); break;
+#define CASE(N) case N: e = yz_prepare<N>(L.nl, fyz, form); break;
         DDA_EDGES(CASE)
 #undef CASE
     }
     if (e != cudaSuccess) return e;
     switch (L.ni) {
-#define CASE(N) case N: return x_prepare<N>();
+#define CASE(N) case N: return x_prepare<N>(L.nl, fx, form);
         DDA_EDGES(CASE)
 #undef CASE
     }

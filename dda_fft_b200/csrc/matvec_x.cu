@@ -658,31 +658,32 @@ cudaError_t launch_x(const MatvecArgs &a, cudaStream_t st)
     return launch_packed<NI, 0>(a, st);
 }
 
+// the kernel that launch_x takes for the same arguments
 template <int NI>
-cudaError_t prep_x()
+cudaError_t prep_x(int nl, int fx, int form)
 {
-    auto set = [](const void *k, size_t bytes) {
-        return matvec_kernel_smem(k, (int)bytes);
-    };
-    constexpr size_t P = (size_t)6 * NI * XC * sizeof(float4);
-    cudaError_t e = set((const void *)k2q<NI, 0>, P);
-    if (e == cudaSuccess) e = set((const void *)k2q<NI, 1>, P);
-    if (e == cudaSuccess) e = set((const void *)k2q<NI, 2>, P);
-    if (e == cudaSuccess) e = set((const void *)k2r<NI, pair_columns<NI>()>, (size_t)6 * NI * pair_columns<NI>() * sizeof(float4));
-    if (e == cudaSuccess) e = set((const void *)k2r<NI, 8>, (size_t)6 * NI * 8 * sizeof(float4));
+    auto set = [](const void *k, size_t bytes) { return raise_smem_limit(k, (int)bytes); };
+    if (form == 2) {
+        constexpr int PC = pair_columns<NI>();
+        if (2 * nl >= PC) return set((const void *)k2r<NI, PC>, (size_t)6 * NI * PC * sizeof(float4));
+        return set((const void *)k2r<NI, 8>, (size_t)6 * NI * 8 * sizeof(float4));
+    }
     if constexpr (NI == 64) {
         constexpr size_t C = (size_t)6 * 64 * sizeof(float2);
-        if (e == cudaSuccess) e = set((const void *)k2f<64, 32>, 32 * C);
-        if (e == cudaSuccess) e = set((const void *)k2f<64, 16>, 16 * C);
-        if (e == cudaSuccess) e = set((const void *)k2f<64, 8>, 8 * C);
+        if (fx == 0 && 2 * nl >= 32) return set((const void *)k2f<64, 32>, 32 * C);
+        if (fx < 2 && 2 * nl >= 16) return set((const void *)k2f<64, 16>, 16 * C);
+        if (fx < 3) return set((const void *)k2f<64, 8>, 8 * C);
     }
-    return e;
+    constexpr size_t P = (size_t)6 * NI * XC * sizeof(float4);
+    if (fx >= 9 && nl >= XC) return set((const void *)k2q<NI, 2>, P);
+    if (fx >= 3 && fx < 6) return set((const void *)k2q<NI, 1>, P);
+    return set((const void *)k2q<NI, 0>, P);
 }
 
 }  // namespace
 
 template <>
-cudaError_t x_prepare<X_NI>() { return prep_x<X_NI>(); }
+cudaError_t x_prepare<X_NI>(int nl, int fx, int form) { return prep_x<X_NI>(nl, fx, form); }
 
 template <>
 cudaError_t x_launch<X_NI>(const MatvecArgs &a, cudaStream_t st)

@@ -610,14 +610,13 @@ cudaError_t launch_yz_v(const MatvecArgs &a, int fwd, cudaStream_t st)
 }
 
 template <int NJ, int NL, int V>
-cudaError_t prep_yz_v()
+cudaError_t prep_yz_v(int form)
 {
     constexpr int NT = yz_threads(V), MB = yz_blocks(V), B = (int)Yz<NJ, NL, NT, MB>::SMEM;
-    const void *ks[4] = {(const void *)k1p<NJ, NL, NT, MB, 0>, (const void *)k1p<NJ, NL, NT, MB, 1>,
-                         (const void *)k1p<NJ, NL, NT, MB, 2>, (const void *)k3p<NJ, NL, NT, MB>};
-    for (const void *k : ks)
-        if (cudaError_t e = matvec_kernel_smem(k, B)) return e;
-    return cudaSuccess;
+    const void *k1[3] = {(const void *)k1p<NJ, NL, NT, MB, 0>, (const void *)k1p<NJ, NL, NT, MB, 1>,
+                         (const void *)k1p<NJ, NL, NT, MB, 2>};
+    const cudaError_t e = raise_smem_limit(k1[form], B);
+    return e == cudaSuccess ? raise_smem_limit((const void *)k3p<NJ, NL, NT, MB>, B) : e;
 }
 
 template <class F>
@@ -637,12 +636,11 @@ cudaError_t with_nl(int nl, F f)
 }  // namespace
 
 template <>
-cudaError_t yz_prepare<YZ_NJ>(int nl)
+cudaError_t yz_prepare<YZ_NJ>(int nl, int fyz, int form)
 {
-    return with_nl(nl, [](auto l) {
+    return with_nl(nl, [&](auto l) {
         constexpr int NL = decltype(l)::value;
-        const cudaError_t e = prep_yz_v<YZ_NJ, NL, 0>();
-        return e == cudaSuccess ? prep_yz_v<YZ_NJ, NL, 1>() : e;
+        return fyz == 1 ? prep_yz_v<YZ_NJ, NL, 1>(form) : prep_yz_v<YZ_NJ, NL, 0>(form);
     });
 }
 
