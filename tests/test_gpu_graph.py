@@ -302,3 +302,45 @@ def test_pinned_blocks_go_from_context_to_context(D, oracle):
     for t in threads:
         t.join()
     assert len(worst) == 4 * 4 * 3 * len(scale) and max(worst) <= 1e-6
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("grid,solver", [((8, 8, 8), 0), ((16, 8, 4), 2)])
+def test_replayed_solves_take_every_value_of_their_call(D, oracle, grid, solver, mode):
+    """Replays of one recording with new values of the same shape -- the activity list (a material
+    switched off and on), directions of the same number (with mode 2 by kz groups, one plan after
+    the other and the first again), an incident field -- then recordings for a second and again
+    the first number of directions, whose pinned layouts differ, with Mueller averages in between.
+    Each call equals the unrecorded one on a context of its own (1e-6: the order of the atomic
+    sums, at discrepancies near 1e-3)."""
+    rng = np.random.default_rng(17)
+    kd = 0.3
+    geom = lambda step, na: oracle.scattering_geometry(3, na, 0.0, step)
+    nrm, a = geom(30.0, 7)
+    b, c, many = geom(25.0, 7)[1], geom(12.0, 7)[1], geom(5.0, 37)[1]
+    base = dict(mv=[0, 1, 1], kinc=(0, 0, 1), einc=(1, 0, 0), ksc=a)
+    occ = (rng.integers(0, 3, grid) * (rng.random(grid) < 0.8)).astype(np.int8)
+    alpha = np.array([0, 0.02 + 0.002j, 0.03 + 0.001j], np.complex64)
+    changes = [{}, {}, {}, dict(mv=[0, 1, 0]), dict(mv=[0, 0, 1]), dict(mv=[0, 1, 1]), dict(ksc=b), dict(ksc=a),
+               dict(ksc=c, einc=(0, 1, 0)), dict(ksc=a), dict(ksc=many), {}, {}, {}, dict(einc=(1, 0, 0)),
+               dict(ksc=b), {}, {}, dict(ksc=a)]
+
+    def run(ctx, s):
+        return ctx.dda_fft(occ, alpha, s["mv"], kd, s["kinc"], s["einc"], s["ksc"], solver=solver, max_step=6,
+                           err_max=1e-5, trace=False)
+    state = dict(base)
+    with D.Context(grid, kd, max_rhs=2) as ctx, D.Context(grid, kd, max_rhs=2) as plain:
+        ctx.set_farfield_mode(mode)
+        plain.set_farfield_mode(mode)
+        plain.set_solver_graph(False)
+        runs = ctx.solver_graph_runs
+        for ch in changes:
+            state.update(ch)
+            got, ref = run(ctx, state), run(plain, state)
+            assert np.abs(got["esc"] - ref["esc"]).max() <= 1e-6 * np.abs(ref["esc"]).max()
+            for q in ("cabs", "cext"):
+                assert abs(got[q] - ref[q]) <= 1e-6 * abs(ref[q])
+            if state["ksc"].shape == a.shape:
+                args = ((0, 0, 1), (1, 0, 0), (0, 1, 0), state["ksc"], nrm, got["esc"], got["esc"][::-1])
+                np.testing.assert_array_equal(ctx.mueller(*args), plain.mueller(*args))
+        assert ctx.solver_graph_runs - runs >= 13

@@ -495,3 +495,62 @@ def test_a_refused_product_leaves_no_error_behind(D, oracle):
             big.convolution_dev(x, y, n)
         for ctx in (other, big):
             assert rel(ctx.convolution(p), ref) < CONV_TOL
+
+
+@pytest.mark.parametrize("grid", [(4, 4, 4), (8, 8, 8), (4, 8, 16), (16, 4, 32), (8, 16, 4), (64, 4, 4), (64, 8, 8),
+                                  (128, 4, 8), (4, 128, 64), (8, 64, 128), (32, 16, 4)])
+def test_sized_passes_at_small_edges_vs_oracle(D, oracle, grid):
+    """The sized passes at edges 4 and 8 on every axis, both operators: every kernel that the variant
+    numbers stand for (rows shorter than a tile of the x pass in its register and bulk-copy forms;
+    planes split over two CTAs with both block sizes at 64 x 128 and 128 x 64), against the oracle.  Numbers that
+    stand for the same kernel are accepted; TMA tiles are refused where a row is shorter than one."""
+    import torch
+    rng = np.random.default_rng(sum(grid))
+    kd = 0.5
+    p = crand(rng, (2, 3) + grid)
+    A = oracle.green_hat(*grid, kd)
+    ref = {conj: np.stack([oracle.convolution(A, q.transpose(1, 2, 3, 0).astype(np.complex128), conj=conj)
+                           for q in p]) for conj in (False, True)}
+    with D.Context(grid, kd, max_rhs=2) as ctx:
+        assert ctx.fast_kernels
+        x = torch.from_numpy(p).cuda()
+        kernels = [3, 6] + ([0, 1, 2] if grid[0] == 64 else [])
+        if grid[2] >= 8:
+            kernels += [9]
+            for alias in (10, 11):
+                ctx.set_fast_variant(alias, 2)
+        else:
+            with pytest.raises(D.DDAGPUError):
+                ctx.set_fast_variant(9, 0)
+        for alias in (0, 1, 2, 4, 5, 7, 8):
+            ctx.set_fast_variant(alias, 2)
+        for vx in kernels:
+            for vyz in (0, 1):
+                ctx.set_fast_variant(vx, vyz)
+                for conj in (False, True):
+                    y = torch.empty_like(x)
+                    ctx.convolution_dev(x, y, 2, conj=conj)
+                    ctx.synchronize()
+                    assert rel(y.cpu().numpy().transpose(0, 2, 3, 4, 1), ref[conj]) < CONV_TOL, (vx, vyz, conj)
+
+
+@pytest.mark.parametrize("grid", [(4, 4, 4), (8, 8, 4), (16, 4, 8), (64, 4, 4), (128, 4, 4), (4, 64, 128)])
+@pytest.mark.parametrize("model", [1, 5])
+def test_sized_solves_at_small_edges_equal_generic(D, grid, model):
+    """Step 0 from the incident field at edges 4 and 8, of polarisation pairs (CM) and of single
+    right-hand sides (LDR), and two CG steps: the sized passes against the generic ones.  Both round
+    at 2^-24 in 2 log2(8 N) butterflies a product, below 1e-6 of the largest value; three products
+    and the sums after them: 1e-5."""
+    rng = np.random.default_rng(sum(grid))
+    occ = (rng.random(grid) < 0.8).astype(np.int8)
+    rot = D.mc_rotations(5, 2)
+    cfg = D.BatchConfig(occ=occ, materials=[(1.5, 0.02)], polarizability=model, max_step=2, err_max=1e-9)
+    out = {}
+    with D.Context(grid, 0.3, max_rhs=4) as ctx:
+        for fast in (True, False):
+            ctx.set_kernels(fast)
+            out[fast] = ctx.orientation_solves(cfg, rot)
+    for q in ("cabs", "cext"):
+        np.testing.assert_allclose(out[True][q], out[False][q], rtol=1e-5)
+    M, G = out[True]["mueller"], out[False]["mueller"]
+    assert np.abs(M - G).max() <= 1e-5 * np.abs(G).max()
