@@ -493,54 +493,42 @@ __global__ void first_approx64(F64 f, double d0, double k0, double k1, double k2
     for (int c = 0; c < 3; c++) p[c * f.N + q] = o[c];
 }
 
-// Block sums of (a) the bilinear product sum a b (ldcScalMul, dda_func.cpp:724-755),
-// (b) Re sum a conj(b) (ldScalMulConj, 757-782) and (c) sum over cells of |r| (ldError's
-// numerator, 784-811), over active cells, added to acc[0..1] in FP64.
-__global__ void __launch_bounds__(kT) reduce64(F64 f, int kind, const double2 *a, const double2 *b,
-                                               double *acc)
+// block sums of NV doubles per thread, added to acc[0 .. NV)
+template <int NV>
+__device__ void block_add(double (&v)[NV], double *acc)
 {
-    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < NV; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    __shared__ double sh[NV][kT / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < NV; k++) sh[k][w] = v[k];
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double t = 0.0;
+        for (int u = 0; u < (int)(blockDim.x >> 5); u++) t += sh[threadIdx.x][u];
+        atomicAdd(acc + threadIdx.x, t);
+    }
+}
+
+// Block sums of Re sum a conj(b) (ldScalMulConj, dda_func.cpp:757-782) or, without b, of the sum
+// over cells of |a| (ldError's numerator, 784-811), over active cells, added to acc in FP64.
+__global__ void __launch_bounds__(kT) reduce64(F64 f, const double2 *a, const double2 *b, double *acc)
+{
+    double s[1] = {0.0};
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < f.N; q += (size_t)gridDim.x * blockDim.x) {
         if (!active(f, q)) continue;
-        if (kind == 2) {
-            double t = 0.0;
-            for (int c = 0; c < 3; c++) {
-                const double2 v = a[c * f.N + q];
-                t += v.x * v.x + v.y * v.y;
-            }
-            s0 += sqrt(t);
-        } else {
-            for (int c = 0; c < 3; c++) {
-                const double2 x = a[c * f.N + q], y = b[c * f.N + q];
-                if (kind == 0) {
-                    s0 += x.x * y.x - x.y * y.y;
-                    s1 += x.x * y.y + x.y * y.x;
-                } else {
-                    s0 += x.x * y.x + x.y * y.y;
-                }
-            }
+        double t = 0.0;
+        for (int c = 0; c < 3; c++) {
+            const double2 x = a[c * f.N + q], y = b ? b[c * f.N + q] : x;
+            t += x.x * y.x + x.y * y.y;
         }
+        s[0] += b ? t : sqrt(t);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-    }
-    __shared__ double sh[2][kT / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) {
-        sh[0][w] = s0;
-        sh[1][w] = s1;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t0 = 0.0, t1 = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) {
-            t0 += sh[0][k];
-            t1 += sh[1][k];
-        }
-        atomicAdd(acc, t0);
-        atomicAdd(acc + 1, t1);
-    }
+    block_add<1>(s, acc);
 }
 
 // o = x + c1 y + c2 z on active cells; inactive cells: o = 0 when mask_zero, else unchanged
@@ -671,27 +659,6 @@ __global__ void __launch_bounds__(kT) cabscext64(F64 f, int nmat1, double d0, do
 }
 
 // ---------------------------------------------------------------- mixed precision (COCG)
-// block sums of NV doubles per thread, added to acc[0 .. NV)
-template <int NV>
-__device__ void block_add(double (&v)[NV], double *acc)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < NV; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-    __shared__ double sh[NV][kT / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; k++) sh[k][w] = v[k];
-    __syncthreads();
-    if (threadIdx.x < NV) {
-        double t = 0.0;
-        for (int u = 0; u < (int)(blockDim.x >> 5); u++) t += sh[threadIdx.x][u];
-        atomicAdd(acc + threadIdx.x, t);
-    }
-}
-
 __global__ void to_f32(const double2 *x, float2 *y, size_t n)
 {
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
@@ -709,8 +676,8 @@ __global__ void from_f32_masked(F64 f, const float2 *x, double2 *y)
     }
 }
 
-// out = v - alpha_m conv (- sub) on active cells, 0 elsewhere, in FP64 from the float
-// convolution; acc (may be null): acc[0] += sum over cells of |out| (ldError's numerator)
+// out = v - alpha_m conv - sub on active cells, 0 elsewhere, in FP64 from the float convolution;
+// acc[0] += sum over cells of |out| (ldError's numerator)
 __global__ void __launch_bounds__(kT) mixed_apply(F64 f, const double2 *v, const float2 *conv,
                                                   const double2 *sub, double2 *out, double *acc)
 {
@@ -726,14 +693,13 @@ __global__ void __launch_bounds__(kT) mixed_apply(F64 f, const double2 *v, const
         for (int c = 0; c < 3; c++) {
             const size_t k = c * f.N + q;
             const float2 g = conv[k];
-            double2 o = dsub(v[k], dmul(al, make_double2(g.x, g.y)));
-            if (sub) o = dsub(o, sub[k]);
+            const double2 o = dsub(dsub(v[k], dmul(al, make_double2(g.x, g.y))), sub[k]);
             out[k] = o;
             t += o.x * o.x + o.y * o.y;
         }
         e[0] += sqrt(t);
     }
-    if (acc) block_add<1>(e, acc);
+    block_add<1>(e, acc);
 }
 
 // The Krylov scalars stay on the device: every reduction adds into a set of kSet doubles, the
@@ -1058,27 +1024,20 @@ struct Fp64Run {
         return matvec64(a, ep, src, out, st);
     }
 
-    cudaError_t reduce(int kind, const double2 *a, const double2 *b, double out[2])
+    cudaError_t reduce(const double2 *a, const double2 *b, double &x)
     {
-        cudaError_t e = cudaMemsetAsync(B.scal.acc, 0, 2 * sizeof(double), st);
+        cudaError_t e = cudaMemsetAsync(B.scal.acc, 0, sizeof(double), st);
         if (e) return e;
-        reduce64<<<4 * 148, kT, 0, st>>>(f, kind, a, b, B.scal.acc);
+        reduce64<<<4 * 148, kT, 0, st>>>(f, a, b, B.scal.acc);
         *launches += 1;
-        if ((e = cudaMemcpyAsync(out, B.scal.acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, st))) return e;
+        if ((e = cudaMemcpyAsync(&x, B.scal.acc, sizeof(double), cudaMemcpyDeviceToHost, st))) return e;
         return cudaStreamSynchronize(st);
     }
-    cudaError_t herm(const double2 *a, const double2 *b, double &x)
-    {
-        double o[2];
-        cudaError_t e = reduce(1, a, b, o);
-        x = o[0];
-        return e;
-    }
+    cudaError_t herm(const double2 *a, const double2 *b, double &x) { return reduce(a, b, x); }
     cudaError_t err(const double2 *r, double &x)
     {
-        double o[2];
-        cudaError_t e = reduce(2, r, nullptr, o);
-        x = o[0] / nact;
+        const cudaError_t e = reduce(r, nullptr, x);
+        x /= nact;
         return e;
     }
     cudaError_t lin3(const double2 *x, std::complex<double> c1, const double2 *y, std::complex<double> c2,

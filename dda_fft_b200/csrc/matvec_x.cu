@@ -297,10 +297,8 @@ k2q(MatvecArgs a, const __grid_constant__ CUtensorMap tmap)
     const int e0 = z_order(bz ? 2 * nl - lp : lp, nl, a.zs, z_parity_split(NI)), e1 = z_order(bz ? 2 * nl - lp - 1 : lp + 1, nl, a.zs, z_parity_split(NI));
     const float2 sg = dup2(a.conj ? 1.f : -1.f), ng = dup2(a.conj ? -1.f : 1.f);
     const int k1 = sub;
-    const bool act = sub < R1;
 #pragma unroll 1
     for (int h = 0; h < 2; h++) {
-        if (!act) break;
         P2 X[3][R2];
 #pragma unroll
         for (int c = 0; c < 3; c++) {
@@ -358,8 +356,7 @@ __global__ void __launch_bounds__(Sx<NI>::RM * TL, 512 / (Sx<NI>::RM * TL)) k2f(
     constexpr int R1 = S::R1, R2 = S::R2;
     static_assert(R1 == R2, "square line splits");
     extern __shared__ __align__(128) float2 B[];   // [6][NI][TL]
-    constexpr bool rhs_fast = k2_rhs_fastest(NI);
-    const int js = rhs_fast ? blockIdx.z : blockIdx.x, rhs = rhs_fast ? blockIdx.x : blockIdx.z;
+    const int js = blockIdx.x, rhs = blockIdx.z;
     chain_enter();
     if (a.rhs_active && !a.rhs_active[rhs]) return;
     const int nj = a.L.nj, nl = a.L.nl;
@@ -413,49 +410,42 @@ __global__ void __launch_bounds__(Sx<NI>::RM * TL, 512 / (Sx<NI>::RM * TL)) k2f(
 #pragma unroll 1
     for (int h = 0; h < 2; h++) {
         float2 X[3][R2];
-        const bool act = sub < R1;
         const int k1 = sub;
-        if (act) {
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
+        for (int c = 0; c < 3; c++) {
 #pragma unroll
-                for (int q = 0; q < R2; q++) X[c][q] = Bat(c, h, R2 * k1 + q);
-                dft_reg<R2, false>(X[c]);
-            }
+            for (int q = 0; q < R2; q++) X[c][q] = Bat(c, h, R2 * k1 + q);
+            dft_reg<R2, false>(X[c]);
         }
         __syncthreads();
-        if (act) {
-            {
 #pragma unroll
-                for (int q = 0; q < R2; q++) {
-                    const int kx = 2 * (k1 + R1 * q) + h, mx = kx > NI, ox = mx ? 2 * NI - kx : kx;
-                    const float4 *A = Ayz + (size_t)ox * sxo;
-                    const float4 a01 = __ldg(A), a23 = __ldg(A + sp), a45 = __ldg(A + 2 * sp);
-                    float2 g0 = make_float2(a01.x, a01.y), g1 = make_float2(a01.z, a01.w),
-                           g2 = make_float2(a23.x, a23.y), g3 = make_float2(a23.z, a23.w),
-                           g4 = make_float2(a45.x, a45.y), g5 = make_float2(a45.z, a45.w);
-                    if (mx ^ my) g1 = cscale(g1, -1.f);
-                    if (mx ^ mz) g2 = cscale(g2, -1.f);
-                    if (my ^ mz) g4 = cscale(g4, -1.f);
-                    if (a.conj) {
-                        g0 = cconj(g0); g1 = cconj(g1); g2 = cconj(g2);
-                        g3 = cconj(g3); g4 = cconj(g4); g5 = cconj(g5);
-                    }
-                    const float2 vx = X[0][q], vy = X[1][q], vz = X[2][q];
-                    X[0][q] = cadd(cadd(cmul(g0, vx), cmul(g1, vy)), cmul(g2, vz));
-                    X[1][q] = cadd(cadd(cmul(g1, vx), cmul(g3, vy)), cmul(g4, vz));
-                    X[2][q] = cadd(cadd(cmul(g2, vx), cmul(g4, vy)), cmul(g5, vz));
-                }
-                // inverse step A with the transposed split: lane k1 owns positions k1 + R1 q
+        for (int q = 0; q < R2; q++) {
+            const int kx = 2 * (k1 + R1 * q) + h, mx = kx > NI, ox = mx ? 2 * NI - kx : kx;
+            const float4 *A = Ayz + (size_t)ox * sxo;
+            const float4 a01 = __ldg(A), a23 = __ldg(A + sp), a45 = __ldg(A + 2 * sp);
+            float2 g0 = make_float2(a01.x, a01.y), g1 = make_float2(a01.z, a01.w),
+                   g2 = make_float2(a23.x, a23.y), g3 = make_float2(a23.z, a23.w),
+                   g4 = make_float2(a45.x, a45.y), g5 = make_float2(a45.z, a45.w);
+            if (mx ^ my) g1 = cscale(g1, -1.f);
+            if (mx ^ mz) g2 = cscale(g2, -1.f);
+            if (my ^ mz) g4 = cscale(g4, -1.f);
+            if (a.conj) {
+                g0 = cconj(g0); g1 = cconj(g1); g2 = cconj(g2);
+                g3 = cconj(g3); g4 = cconj(g4); g5 = cconj(g5);
+            }
+            const float2 vx = X[0][q], vy = X[1][q], vz = X[2][q];
+            X[0][q] = cadd(cadd(cmul(g0, vx), cmul(g1, vy)), cmul(g2, vz));
+            X[1][q] = cadd(cadd(cmul(g1, vx), cmul(g3, vy)), cmul(g4, vz));
+            X[2][q] = cadd(cadd(cmul(g2, vx), cmul(g4, vy)), cmul(g5, vz));
+        }
+        // inverse step A with the transposed split: lane k1 owns positions k1 + R1 q
 #pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    dft_reg<R2, true>(X[c]);
+        for (int c = 0; c < 3; c++) {
+            dft_reg<R2, true>(X[c]);
 #pragma unroll
-                    for (int u = 0; u < R2; u++) {
-                        const float2 y = u ? cmul(X[c][u], twid<true>(tw, k1 * u)) : X[c][u];
-                        Bat(c, h, k1 + R1 * u) = y;
-                    }
-                }
+            for (int u = 0; u < R2; u++) {
+                const float2 y = u ? cmul(X[c][u], twid<true>(tw, k1 * u)) : X[c][u];
+                Bat(c, h, k1 + R1 * u) = y;
             }
         }
         __syncthreads();

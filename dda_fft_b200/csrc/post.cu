@@ -903,7 +903,9 @@ void plan_kz_groups(const double *ks, int nrhs, int ndir, bool pairs, int ni, in
     if (elems * sizeof(float2) > ((size_t)1 << 30)) return;   // group sums above 1 GiB: direct
     if (zsum_smem(nl, NR) > 200 * 1024 || xysum_smem(nj, kz_slice_for(ni, nj, NR), NR) > 48 * 1024) return;
     // work: a complex multiply-add per (group, cell) and per (direction, row) against one
-    // per (direction, active cell)
+    // per (direction, active cell).  (ff_zsum does half of the first over mirrored pairs; the line
+    // stays where both forms were measured, so near it the direct form may be taken for longer
+    // than it pays.)
     if (mode == 0 && 2.0 * (G * cells + 2.0 * ndir * ni * nj) > (double)ndir * nact) return;
     P.groups = G;
     P.items = items;

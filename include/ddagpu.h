@@ -267,8 +267,9 @@ int ddagpu_anthrax_rasterize(int device, int i_max, int j_max, int l_max, const 
  * a tensor map of the work buffer; offered where the driver provides the encoder and l_max is
  * at least 8); yz_variant 0 / 1 / 2 = 256, 128 or 256 threads per CTA of the y/z passes.
  * A new context starts with the variants measured fastest at its edges.
- * ddagpu_autotune times every combination (and the generic passes) and keeps the
- * fastest.  No counterpart in the reference. */
+ * ddagpu_autotune times the kernels that the numbers stand for (and the generic passes) and
+ * keeps the fastest; one whose wait for its copies ran out is passed over.  No counterpart in
+ * the reference. */
 int ddagpu_set_fast_variant(ddagpu_ctx *ctx, int x_variant, int yz_variant);
 
 /* Form of the far-field sum (FarField, dda_func.cpp:1576-1625).  When the scattering
