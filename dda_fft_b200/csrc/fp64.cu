@@ -710,18 +710,20 @@ constexpr int kSet = 12;
 // BiCGStab set: rho (0,1), <g,h> (2,3), <w,r> (4,5), <w,w> (6,7), sum |r| (8)
 
 __device__ __forceinline__ double2 set_at(const double *a, int k) { return make_double2(a[k], a[k + 1]); }
-// a / b with b brought to [1, 2) by a power of two: unscaled, its square leaves the doubles' range for
+// a / b with b brought to [1, 4) by a power of two: unscaled, its square leaves the doubles' range for
 // sums below 1e-154 or above 1e154 (a converged residual, right-hand sides in small or large
-// units) while the quotient is an ordinary number.  By zero or infinity part by part: infinite and
-// zero coefficients, as a complex division gives them.
+// units) while the quotient is an ordinary number.  The power is set bit by bit (subnormal sums
+// end between 2^-51 and 2), as ilogb and scalbn took a microsecond of a step.  By zero or infinity
+// part by part: infinite and zero coefficients, as a complex division gives them.
 __device__ __forceinline__ double2 ddiv(double2 a, double2 b)
 {
     const double m = fmax(fabs(b.x), fabs(b.y));
     if (!(m > 0.0) || isinf(m)) return make_double2(a.x / m, a.y / m);
-    const int e = ilogb(m);
-    const double2 c = make_double2(scalbn(b.x, -e), scalbn(b.y, -e));
+    const int e = 2046 - (__double2hiint(m) >> 20);   // biased exponent of 1 / m to a power of two
+    const double w = __hiloint2double((e > 1 ? e : 1) << 20, 0);
+    const double2 c = make_double2(b.x * w, b.y * w);
     const double d = c.x * c.x + c.y * c.y;
-    return make_double2(scalbn((a.x * c.x + a.y * c.y) / d, -e), scalbn((a.y * c.x - a.x * c.y) / d, -e));
+    return make_double2((a.x * c.x + a.y * c.y) / d * w, (a.y * c.x - a.x * c.y) / d * w);
 }
 __device__ __forceinline__ void bil_add(double &re, double &im, double2 a, double2 b)
 {
