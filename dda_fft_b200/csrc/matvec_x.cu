@@ -347,7 +347,7 @@ k2q(MatvecArgs a, const __grid_constant__ CUtensorMap tmap)
 }
 
 // ---- unpacked form, edge 64: a block takes TL neighbouring columns, one complex number per
-// access.  15 M warp instructions per right-hand side against 10.9 M packed ones, but twice the
+// access.  16.4 M warp instructions per right-hand side against 10.9 M packed ones, but twice the
 // warps (16 per SM, 128 registers): 18.4 against 21 us at 24 right-hand sides.
 template <int NI, int TL>
 __global__ void __launch_bounds__(Sx<NI>::RM * TL, 512 / (Sx<NI>::RM * TL)) k2f(MatvecArgs a)

@@ -50,7 +50,8 @@ struct Yz {
     // A warp loads whole rows (forward) where the R2 elements of a lane group are 32-byte runs of the
     // field, eight lines per warp access; with that, without the next rows' prefetch where it
     // spilled (ZS 4) and with at()'s row term k1p takes 321 instead of 398 us (128^3 x 4) and 70
-    // instead of 74 (32 x 128 x 64 x 6).  Longer runs (ML 64) gain nothing from the extra hop.
+    // instead of 74 (32 x 128 x 64 x 6).  (At 128 x 128 the incident-field forms spill still, 20 and 12
+    // bytes a thread.)  Longer runs (ML 64) gain nothing from the extra hop.
     static constexpr bool WIDE = ZS > 1 && ML == 32;
     static constexpr int CW = 8;                            // columns of a lane group: 128-byte runs
     static constexpr int GT = CW * SY::R1;                  // its threads (1, 2 or 4 warps)
