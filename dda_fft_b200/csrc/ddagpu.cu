@@ -1151,7 +1151,7 @@ int ddagpu_set_kernels(ddagpu_ctx *c, int fast)
     if (fast && !matvec_fast_supported(c->L))
         return fail(DDAGPU_EINVAL, "compile-time-sized passes need edges of 4 at least");
     DevGuard dg(c->dev);
-    if (!fast) CK(matvec_prepare(c->L, c->tile_x, c->rows_g));
+    CK(fast ? matvec_fast_prepare(c->L, c->fx, c->fyz, 0) : matvec_prepare(c->L, c->tile_x, c->rows_g));
     c->fast = fast ? 1 : 0;
     return DDAGPU_OK;
 }
